@@ -18,7 +18,7 @@
 // The error stays below one unit in the last place of the line's largest term, as with a
 // chain of FP64 fused multiply-adds, whose rounding errors are of that size too.
 //
-// The stage kernels apply the operators in mirror form (fix_apply_mirror): the solution
+// The stage kernels apply the operators in mirror form (fix_mirror_line): the solution
 // and flux points are symmetric about the cell centre, so the operators satisfy
 // C(NO-1-k, NI-1-j) = sigma C(k, j) (sigma = +1 for the interpolation Lmat, -1 for the
 // derivative Mmat) up to the rounding of their construction (1e-16 to 2e-15 of the
@@ -27,9 +27,9 @@
 // input pairs, U + W and sigma (U - W), so a line takes half the multiply-adds.  The
 // coefficients are those of the operator averaged with its mirror image, each within one
 // unit of 2^-S of both rows, and the error bound above holds for that operator.  The
-// caller keeps the FP64 form for lines with NaN, infinite or huge (above 2^876) inputs,
-// so non-finite states propagate as before.  Zero results are +0; results below the
-// normal range (only from inputs below 2^-960) are flushed to zero.
+// caller keeps the FP64 form for lines with NaN, infinite, huge (above 2^876) or tiny (below
+// 2^-957, not zero) inputs, so non-finite states propagate as before.  Zero results are +0;
+// results below the normal range are flushed to zero.
 #pragma once
 #include <cstdint>
 
@@ -70,6 +70,31 @@ FIX_HD int fix_clz64(uint64_t u) {
   return __clzll((long long)u);
 #else
   return u ? __builtin_clzll(u) : 64;
+#endif
+}
+
+// acc + a b, 32x32->64 signed.  Written as mad.lo.cc / madc.hi because the compiler makes one
+// multiply-add instruction of the pair, and a multiplication and two additions of
+// `acc += (int64_t)a * b` or of mad.wide (counted: 4 against 12 instructions for a chain of
+// four).
+FIX_HD int64_t fix_mad(int a, int b, int64_t acc) {
+#ifdef __CUDA_ARCH__
+  uint32_t lo = (uint32_t)acc, hi = (uint32_t)((uint64_t)acc >> 32);
+  asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.s32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
+  return (int64_t)(((uint64_t)hi << 32) | lo);
+#else
+  return acc + (int64_t)a * b;
+#endif
+}
+
+// v >> d, zero for d > 63
+FIX_HD uint64_t fix_shru(uint64_t v, int d) {
+#ifdef __CUDA_ARCH__
+  uint64_t r;
+  asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(d));  // clamps the amount
+  return r;
+#else
+  return d < 64 ? v >> d : 0;
 #endif
 }
 
@@ -156,45 +181,154 @@ FIX_HD double fix_dot(const int (&h)[NI], const int (&l)[NI], const int* ch, con
   return fix_round(A, B, D, k);
 }
 
-// y = C v for C (NO x NI) in mirror form (fix_mirror_coefs: per row k < (NO+1)/2 the
+// the line's largest magnitude word: the high 31 bits of the largest |x| (0 for a line of
+// zeros and of values below 2^-1042)
+template <int NI>
+FIX_HD uint32_t fix_amax(const double (&v)[NI]) {
+  uint32_t a = 0;
+#pragma unroll
+  for (int j = 0; j < NI; j++) {
+    const uint32_t aj = (uint32_t)(fix_bits(v[j]) >> 32) & 0x7fffffffu;
+    a = aj > a ? aj : a;
+  }
+  return a;
+}
+
+// Does fix_mirror_line take a line whose largest magnitude word is a?  Lines of zeros and
+// those whose largest exponent lies between kFixEmaxMin and kFixEmaxFast: below, results
+// could leave the normal range, above, infinities and NaNs have to propagate.
+constexpr int kFixEmaxMin = 66;
+FIX_HD bool fix_line_ok(uint32_t a) {
+  return a == 0 || a - ((uint32_t)kFixEmaxMin << 20) < ((uint32_t)(kFixEmaxFast + 1 - kFixEmaxMin) << 20);
+}
+
+// V 2^k' (|V| < 2^63) rounded to nearest (ties up in magnitude), k' = k - 1 with k as in
+// fix_round; CHECK: results below the normal range are flushed to zero (otherwise the
+// caller knows that there are none)
+template <bool CHECK>
+FIX_HD double fix_round_v(int64_t V, int k) {
+  const int64_t s = V >> 63;
+  const uint64_t u = (uint64_t)((V ^ s) - s);
+  uint32_t uh = (uint32_t)(u >> 32), ul = (uint32_t)u;
+  int e = k + 1084;  // biased exponent of a value whose leading bit is bit 63, less one
+  if (uh == 0) {     // at most 32 bits are left
+    uh = ul >> 1;
+    ul <<= 31;
+    e -= 31;
+  }
+#ifdef __CUDA_ARCH__
+  const int lz = __clz((int)uh);
+#else
+  const int lz = uh ? __builtin_clz(uh) : 32;
+#endif
+  const uint64_t top = ((((uint64_t)uh << 32) | ul) << (lz - 1)) + 0x200;  // leading bit 62 (lz >= 1)
+  const uint64_t mant = top >> 10;                                         // 2^52 .. 2^53
+  const int E = e - lz;
+  uint32_t h = (uint32_t)(mant >> 32) + ((uint32_t)E << 20);
+  uint32_t l = (uint32_t)mant;
+  if (uh == 0 && ul == 0) h = 0;  // (l is 0 too)
+  if (CHECK && E < 0) h = l = 0;
+  h |= (uint32_t)(s >> 32) & 0x80000000u;
+  return fix_double(((uint64_t)h << 32) | l);
+}
+
+// y = C v for C (NO x NI) in mirror form (fix_mirror_coefs: per row r < (NO+1)/2 the
 // coefficients [P(0..NI/2) | Q(0..NI/2) | R]), scaled by 2^k as fix_dot.  With
-// E_j = X_j + X_{NI-1-j}, O_j = X_j - X_{NI-1-j} (|E|, |O| < 2^58), U = sum P E (+ R X_m for
-// odd NI) and W = sum Q O: y_k = U + W, y_{NO-1-k} = sigma (U - W).  The middle row of an
-// odd NO has only U (sigma = +1) or only W (sigma = -1): the other half is exactly zero.
-// Bounds for NI <= 9 (|P|, |Q|, |R| < 2^59, so |ch| < 2^30): |A| < 9 2^59 = 2^62.2,
-// |B| < 9 1.5 2^59 = 2^62.8, |D| < 9 2^58 = 2^61.2, for sums and differences alike.
-template <int NO, int NI, int SIGMA>
-FIX_HD void fix_apply_mirror(const double (&v)[NI], int emax, const int* ch, const int* cl, int k, double (&y)[NO]) {
+// E_j = X_j + X_{NI-1-j}, O_j = X_j - X_{NI-1-j}, U = sum P E (+ R X_m for odd NI) and
+// W = sum Q O: y_r = U + W, y_{NO-1-r} = sigma (U - W).  The middle row of an odd NO has
+// only U (sigma = +1) or only W (sigma = -1): the other half is exactly zero.
+//
+// What bounds the passes that call this is the number of integer instructions, most of
+// them the alignment of the inputs and the rounding of the outputs, so:
+//  - X = |x| 2^(1080 - emax), 58 bits truncated (5 guard bits): the significand is placed
+//    at the top of 64 bits, with its hidden bit whatever the exponent (an input that has
+//    none is below the line's largest by more than 64 bits and is shifted out), and
+//    shifted right once; the truncation error equals that of rounding with 4 guard bits;
+//  - the limbs of E, O and of the coefficients are h 2^29 + l with |l| <= 2^28 (signed), so
+//    that the products of two low limbs can be left out: at most NI / 4 units of 2^-58 of
+//    the largest term, of either sign, against the one unit, always downwards, that
+//    truncating the sum used to take; three multiply-adds a term instead of four;
+//  - the sum is rounded to a multiple of 2^58 (2^28 in the start value of B).
+// A derivative line of six inputs and five outputs went from about 635 to 350 instructions;
+// 512x512 cells, N = 5 (GB300): E3 1.361 -> 1.150 ms per stage, the step 18.2 -> 17.2 ms.
+// Bounds for NI <= 9 with |P +- Q| < 2^59, |X| < 2^58: |A| < 9 2^59, and the partial sums
+// over U or W alone < 4 2^60 + 2^59; |B| < 9 (2^58 + 2^58) + 2^28: all below 2^63.
+template <int NO, int NI, int SIGMA, bool CHECK>
+FIX_HD void fix_mirror_line(const double (&v)[NI], int emax, const int* ch, const int* cl, int k, double (&y)[NO]) {
   constexpr int NP = NI / 2;
   int64_t X[NI];
-  fix_align_x(v, emax, X);
+  const uint32_t eb = ((uint32_t)emax << 20) | 0xfffffu;
+#pragma unroll
+  for (int j = 0; j < NI; j++) {
+    const uint64_t u = fix_bits(v[j]);
+    const uint32_t a = (uint32_t)(u >> 32) & 0x7fffffffu;
+    const uint32_t d = (eb + (6u << 20) - a) >> 20;  // emax - exponent + 6
+    const uint64_t t = (u << 11) | 0x8000000000000000ull;
+    const int64_t x = (int64_t)fix_shru(t, (int)d);
+    X[j] = (int64_t)u < 0 ? -x : x;
+  }
+  constexpr int64_t kHalfL = (int64_t)1 << (kFixSplit - 1);
+  auto split = [](int64_t x, int& h, int& l) {  // x offset by half a limb
+    h = (int)(x >> kFixSplit);
+    l = (int)(x & ((1 << kFixSplit) - 1)) - (1 << (kFixSplit - 1));
+  };
   int eh[NP > 0 ? NP : 1], el[NP > 0 ? NP : 1], oh[NP > 0 ? NP : 1], ol[NP > 0 ? NP : 1];
 #pragma unroll
   for (int j = 0; j < NP; j++) {
-    fix_split(X[j] + X[NI - 1 - j], eh[j], el[j]);
-    fix_split(X[j] - X[NI - 1 - j], oh[j], ol[j]);
+    split(X[j] + X[NI - 1 - j] + kHalfL, eh[j], el[j]);
+    split(X[j] - X[NI - 1 - j] + kHalfL, oh[j], ol[j]);
   }
   int mh = 0, ml = 0;
-  if (NI & 1) fix_split(X[NP], mh, ml);
+  if (NI & 1) split(X[NP] + kHalfL, mh, ml);
 #pragma unroll
   for (int r = 0; r < (NO + 1) / 2; r++) {
     const int* rh = ch + r * NI;
     const int* rl = cl + r * NI;
     const bool mid = (NO & 1) && r == NO / 2;
-    int64_t Au = 0, Bu = 0, Du = 0, Aw = 0, Bw = 0, Dw = 0;
+    int64_t Au = 0, Bu = kHalfL, Aw = 0, Bw = 0;
     if (!mid || SIGMA > 0) {
 #pragma unroll
-      for (int j = 0; j < NP; j++) fix_mac(eh[j], el[j], rh[j], rl[j], Au, Bu, Du);
-      if (NI & 1) fix_mac(mh, ml, rh[2 * NP], rl[2 * NP], Au, Bu, Du);
+      for (int j = 0; j < NP; j++) {
+        Au = fix_mad(eh[j], rh[j], Au);
+        Bu = fix_mad(eh[j], rl[j], Bu);
+        Bu = fix_mad(el[j], rh[j], Bu);
+      }
+      if (NI & 1) {
+        Au = fix_mad(mh, rh[2 * NP], Au);
+        Bu = fix_mad(mh, rl[2 * NP], Bu);
+        Bu = fix_mad(ml, rh[2 * NP], Bu);
+      }
     }
     if (!mid || SIGMA < 0) {
 #pragma unroll
-      for (int j = 0; j < NP; j++) fix_mac(oh[j], ol[j], rh[NP + j], rl[NP + j], Aw, Bw, Dw);
+      for (int j = 0; j < NP; j++) {
+        Aw = fix_mad(oh[j], rh[NP + j], Aw);
+        Bw = fix_mad(oh[j], rl[NP + j], Bw);
+        Bw = fix_mad(ol[j], rh[NP + j], Bw);
+      }
     }
-    y[r] = fix_round(Au + Aw, Bu + Bw, Du + Dw, k);
-    if (!mid)
-      y[NO - 1 - r] = SIGMA > 0 ? fix_round(Au - Aw, Bu - Bw, Du - Dw, k) : fix_round(Aw - Au, Bw - Bu, Dw - Du, k);
+    y[r] = fix_round_v<CHECK>(Au + Aw + ((Bu + Bw) >> kFixSplit), k);
+    if (!mid) {
+      const int64_t V = Au - Aw + ((Bu - Bw) >> kFixSplit);
+      y[NO - 1 - r] = fix_round_v<CHECK>(SIGMA > 0 ? V : -V, k);
+    }
   }
+}
+
+// the same for any finite line with emax <= kFixEmaxFast: lines below kFixEmaxMin are scaled
+// up by 2^200 (exact) and their results back
+template <int NO, int NI, int SIGMA>
+FIX_HD void fix_apply_mirror(const double (&v)[NI], int emax, const int* ch, const int* cl, int k, double (&y)[NO]) {
+  if (emax >= kFixEmaxMin) {
+    fix_mirror_line<NO, NI, SIGMA, true>(v, emax, ch, cl, k, y);
+    return;
+  }
+  double w[NI];
+#pragma unroll
+  for (int j = 0; j < NI; j++) w[j] = v[j] * 0x1p200;
+  const int ew = fix_emax(w);
+  const int em = ew > kFixEmaxMin ? ew : kFixEmaxMin;  // (a line of zeros)
+  fix_mirror_line<NO, NI, SIGMA, true>(w, em, ch, cl, k - emax + em - 200, y);
 }
 
 // integer form of coefficients (host side): c = round(C 2^S), S the largest shift that
@@ -223,6 +357,13 @@ inline void fix_split_coef(double C, int S, int* ch, int* cl) {
   *cl = (int)(c & ((1 << kFixSplit) - 1));
 }
 
+// c = ch 2^29 + cl with -2^28 <= cl < 2^28
+inline void fix_split_signed(int64_t c, int* ch, int* cl) {
+  const int64_t half = (int64_t)1 << (kFixSplit - 1);
+  *ch = (int)((c + half) >> kFixSplit);
+  *cl = (int)((c + half) & ((1 << kFixSplit) - 1)) - (int)half;
+}
+
 // the mirror form of C (NO x NI, row-major C[k NI + j], C(NO-1-k, NI-1-j) = sigma C(k, j)
 // up to rounding) for fix_apply_mirror: for each row k < (NO+1)/2, k' = NO-1-k, and input
 // pair j < NI/2, j' = NI-1-j, from the integers c = round(C 2^S),
@@ -241,15 +382,12 @@ inline void fix_mirror_coefs(const double* C, int NO, int NI, int sigma, int S, 
       const int jj = NI - 1 - j;
       const int64_t p = (c(k, j) + c(k, jj) + sigma * (c(kk, jj) + c(kk, j)) + 2) >> 2;
       const int64_t q = (c(k, j) - c(k, jj) + sigma * (c(kk, jj) - c(kk, j)) + 2) >> 2;
-      ch[k * NI + j] = (int)(p >> kFixSplit);
-      cl[k * NI + j] = (int)(p & ((1 << kFixSplit) - 1));
-      ch[k * NI + NP + j] = (int)(q >> kFixSplit);
-      cl[k * NI + NP + j] = (int)(q & ((1 << kFixSplit) - 1));
+      fix_split_signed(p, &ch[k * NI + j], &cl[k * NI + j]);
+      fix_split_signed(q, &ch[k * NI + NP + j], &cl[k * NI + NP + j]);
     }
     if (NI & 1) {
       const int64_t r = (c(k, NP) + sigma * c(kk, NP) + 1) >> 1;
-      ch[k * NI + 2 * NP] = (int)(r >> kFixSplit);
-      cl[k * NI + 2 * NP] = (int)(r & ((1 << kFixSplit) - 1));
+      fix_split_signed(r, &ch[k * NI + 2 * NP], &cl[k * NI + 2 * NP]);
     }
   }
 }

@@ -201,13 +201,14 @@ __device__ __forceinline__ int interior_fp(int i) {
 
 // interpolation along one line from the N solution values to the N+1 flux points,
 // y_f = sum_j L(f,j) v_j: the integer form (fixdot.cuh), or FP64 for a line with
-// non-finite or huge values, where the mirror symmetry of the points halves the
+// non-finite, huge or tiny values, where the mirror symmetry of the points halves the
 // multiplications (see OpsN::CE)
 template <int N, class O>
 __device__ __forceinline__ void interp_line(const double (&v)[N], double (&y)[N + 1]) {
-  const int emax = fix_emax(v);
-  if (emax <= kFixEmaxFast) {
-    fix_apply_mirror<N + 1, N, 1>(v, emax, O::ops().LH, O::ops().LL, emax - 1017 - kFixG - O::ops().LS, y);
+  const uint32_t am = fix_amax(v);
+  if (fix_line_ok(am)) {
+    const int emax = max((int)(am >> 20), kFixEmaxMin);
+    fix_mirror_line<N + 1, N, 1, false>(v, emax, O::ops().LH, O::ops().LL, emax - 1017 - kFixG - O::ops().LS, y);
     return;
   }
   double ev[N / 2 > 0 ? N / 2 : 1], od[N / 2 > 0 ? N / 2 : 1];
@@ -231,16 +232,17 @@ __device__ __forceinline__ void interp_line(const double (&v)[N], double (&y)[N 
 }
 
 // the derivative along one line, y_i = sum_r M(r,i) x_r (i < N) from the N+1 flux values
-// x_r = x[r*xs]: the integer form (fixdot.cuh), or FP64 for a line with non-finite or
-// huge values
+// x_r = x[r*xs]: the integer form (fixdot.cuh), or FP64 for a line with non-finite,
+// huge or tiny values
 template <int N, class O>
 __device__ __forceinline__ void deriv_line(const double* x, int xs, double (&y)[N]) {
   double v[N + 1];
 #pragma unroll
   for (int r = 0; r <= N; r++) v[r] = x[r * xs];
-  const int emax = fix_emax(v);
-  if (emax <= kFixEmaxFast) {
-    fix_apply_mirror<N, N + 1, -1>(v, emax, O::ops().MH, O::ops().ML, emax - 1017 - kFixG - O::ops().MS, y);
+  const uint32_t am = fix_amax(v);
+  if (fix_line_ok(am)) {
+    const int emax = max((int)(am >> 20), kFixEmaxMin);
+    fix_mirror_line<N, N + 1, -1, false>(v, emax, O::ops().MH, O::ops().ML, emax - 1017 - kFixG - O::ops().MS, y);
   } else {
 #pragma unroll
     for (int i = 0; i < N; i++) {
@@ -655,7 +657,7 @@ __device__ __forceinline__ void e2_chunk(const SolveDev& s, int c0, int chunk, i
 }
 
 template <int N>
-__global__ void __launch_bounds__(512) k_e2(SolveDev s, int epb, int chunk) {
+__global__ void __launch_bounds__(512, 2) k_e2(SolveDev s, int epb, int chunk) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
   e2_chunk<N, OpsTU>(s, blockIdx.x * chunk, chunk, epb, sm);
@@ -858,7 +860,7 @@ __device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int 
 }
 
 template <int N>
-__global__ void __launch_bounds__(512) k_e3(SolveDev s, RKStage rk, int epb, int update, int c0, int c1) {
+__global__ void __launch_bounds__(512, 2) k_e3(SolveDev s, RKStage rk, int epb, int update, int c0, int c1) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
   const int e0 = c0 + blockIdx.x * epb;
