@@ -105,11 +105,12 @@ __global__ void __launch_bounds__(512, 2) kg_e1(BatchDev b, int sensor_on) {
 }
 
 template <int N>
-__global__ void __launch_bounds__(256) kg_f1(BatchDev b) {
+__global__ void __launch_bounds__(kF1Threads, 2) kg_f1(BatchDev b) {
+  extern __shared__ __align__(16) double sm[];
   pdl_wait();
   for_tiles(b, gidx(PF1, N), b.ftiles, [&](const int4& T, const SolveDev& s) {
-    unsigned long long evb = 0ull;
-    if ((int)threadIdx.x < T.z) evb = f1_point<N>(s, T.y + threadIdx.x);
+    const unsigned long long evb = f1_points<N>(s, T.y + (int)(threadIdx.x & ~31u), (int)blockDim.x, T.y + T.z,
+                                                reinterpret_cast<F1Warp*>(sm), [](int i) { return i; });
     block_max_ull(evb, s.eig);
   });
 }
@@ -180,6 +181,7 @@ template <int N>
 static void pass_shapes(int nsm, const int (&epb)[4], const int (&threads)[4], PassShape (&sh)[kPasses]) {
   const int lim = 200 * 1024;
   cudaFuncSetAttribute(kg_e1<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(kg_f1<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_e2<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_e3<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_ct<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
@@ -198,7 +200,7 @@ static void pass_shapes(int nsm, const int (&epb)[4], const int (&threads)[4], P
     p.grid = nsm * occ;
   };
   fill(sh[PE1], (const void*)kg_e1<N>, threads[0], epb[0], cell_smem_bytes(N, epb[0], 0));
-  fill(sh[PF1], (const void*)kg_f1<N>, 256, 0, 0);
+  fill(sh[PF1], (const void*)kg_f1<N>, kF1Threads, 0, f1_smem(kF1Threads));
   fill(sh[PE2], (const void*)kg_e2<N>, threads[1], epb[1], cell_smem_bytes(N, epb[1], 1));
   fill(sh[PE3], (const void*)kg_e3<N>, threads[2], epb[2], cell_smem_bytes(N, epb[2], 2));
   fill(sh[PCT], (const void*)kg_ct<N>, threads[3], epb[3], cell_smem_bytes(N, epb[3], 3));
@@ -209,7 +211,7 @@ template <int N>
 static void launch_pass(const BatchDev& a, int pass, const PassShape& p, cudaStream_t st, int arg) {
   switch (pass) {
     case PE1: launch_pdl(kg_e1<N>, p.grid, p.threads, p.smem, st, a, arg); break;
-    case PF1: launch_pdl(kg_f1<N>, p.grid, p.threads, 0, st, a); break;
+    case PF1: launch_pdl(kg_f1<N>, p.grid, p.threads, p.smem, st, a); break;
     case PE2: launch_pdl(kg_e2<N>, p.grid, p.threads, p.smem, st, a, p.epb); break;
     case PE3: launch_pdl(kg_e3<N>, p.grid, p.threads, p.smem, st, a, arg); break;
     case PCT: launch_pdl(kg_ct<N>, p.grid, p.threads, p.smem, st, a, arg); break;
@@ -289,7 +291,8 @@ struct ChorusBatch {
   int ctiles = 0, ftiles = 0;
 };
 
-static constexpr int kFaceTile = 256;  // face points per tile (one per thread)
+static constexpr int kFaceTile = 256;   // face points per tile (one per thread)
+static constexpr int kFluxTile = 4 * kF1Threads;  // of the flux pass, whose warps copy ahead
 
 static int batch_alloc(ChorusBatch* b, int cap_solves, int cap_ctiles, int cap_ftiles) {
   auto fr = [](void* p) { if (p) cudaFree(p); };
@@ -351,7 +354,7 @@ static int batch_rebuild(ChorusBatch* b) {
       for (int a = 0; a < n; a += step) grp[gidx(pass, sl.N)].push_back(make_int4(i, a, std::min(step, n - a), 0));
     };
     cut(PE1, sl.NC, o.epb[0]);
-    cut(PF1, sl.nfp_faces, kFaceTile);
+    cut(PF1, sl.nfp_faces, kFluxTile);
     long long chunk = order_cells[sl.N] / (16LL * b->nsm);
     chunk = std::max<long long>(o.epb[1], std::min<long long>(chunk, o.threads[1]));
     chunk -= chunk % o.epb[1];

@@ -122,6 +122,7 @@ struct Dispatch {
   void (*f1)(const SolveDev&, cudaStream_t, int, int, int, int);
   void (*e2)(const SolveDev&, const Launch&, cudaStream_t);
   void (*f2)(const SolveDev&, cudaStream_t);
+  void (*qavg)(const SolveDev&, cudaStream_t);
   void (*e3)(const SolveDev&, const RKStage&, const Launch&, cudaStream_t, int, int);
   void (*ct)(const SolveDev&, const Launch&, cudaStream_t, int, int, int);
   void (*nqsp)(const SolveDev&, int, int, cudaStream_t);
@@ -129,7 +130,7 @@ struct Dispatch {
   void (*diag)(const SolveDev&, const Launch&, cudaStream_t, int);
 };
 #define DISPATCH(n) \
-  Dispatch{launch_e1<n>, launch_e1_nosensor_n##n, launch_f1<n>, launch_e2<n>, launch_f2<n>, launch_e3<n>, launch_ct<n>, launch_nqsp<n>, launch_divb<n>, \
+  Dispatch{launch_e1<n>, launch_e1_nosensor_n##n, launch_f1<n>, launch_e2<n>, launch_f2<n>, launch_qavg<n>, launch_e3<n>, launch_ct<n>, launch_nqsp<n>, launch_divb<n>, \
            launch_diag<n>}
 static const Dispatch* dispatch_for(int N) {
   static const Dispatch d[kMaxN + 1] = {Dispatch{}, Dispatch{}, DISPATCH(2), DISPATCH(3), DISPATCH(4),
@@ -502,6 +503,7 @@ int chorus_gpu_bind(const ChorusDims* dims, const int32_t* IF2C, const int32_t* 
   s.nface1 = c->nface1;
   s.artiv = params->ARTIV == 1;
   s.gam = params->gam;
+  s.gas = ix_gas(params->gam);
   s.mu = params->mu;
   s.eta0 = params->eta0;
   s.B0x = params->B0x;
@@ -1012,6 +1014,7 @@ int nablaqsp_gpu(ChorusCtx* c, const int32_t* v_sta, const int32_t* v_end) {
   if (*v_sta < 1 || *v_end > 9 || *v_sta > *v_end) return set_err(CHORUS_EINVAL, "variable range %d..%d", *v_sta, *v_end);
   if (ctx_device(c)) return CHORUS_ECUDA;
   if (*v_end == 9) fill_qvf9(c);  // nablaQsp(9,9) reads the A_z traces
+  c->D->qavg(c->sd, c->st);       // and every variable the face averages
   c->D->nqsp(c->sd, *v_sta - 1, *v_end - 1, c->st);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c->st));
@@ -1249,7 +1252,10 @@ int chorus_gpu_download_array(ChorusCtx* c, const char* name, double* out, int64
       // the stage averages the grad Q traces where it reads them: store the averages
       // (idempotent) so that the arrays equal the reference's nablaQvfi / nablaQvfj
       if (x.p == s.nQvf) c->D->f2(s, c->st);
-      if (x.p == s.Qvf) fill_qvf9(c);
+      if (x.p == s.Qvf) {
+        fill_qvf9(c);
+        c->D->qavg(s, c->st);
+      }
       const size_t per = (size_t)NF1 * x.w;
       if ((size_t)count != per * NC) return set_err(CHORUS_EINVAL, "%s has %zu elements", name, per * NC);
       int rc = pull(x.p, (size_t)NC * NFP * x.w, h);

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "../../include/chorus_gpu.h"
+#include "intflux.cuh"
 
 namespace chorus {
 
@@ -52,7 +53,8 @@ void initial_point(int problem, double gam, double x, double y, const double* B,
 // Device-side view of one solve.  Element-blocked layouts (e = cell, 0-based):
 //   Q, Qk0..   [e][js][is][9]              (the reference's Q(9,N,N,NC))
 //   resid      [e][js][is][9]
-//   Qvf        [e][fp][9]    fp = family-1 points (jfp*(N+1)+ifp), then family-2
+//   Qvf        [e][fp][9]    (traces on faces: the cell's own, averaged where they are read)
+//                            fp = family-1 points (jfp*(N+1)+ifp), then family-2
 //                            points ((N+1)N + jfp*N+ifp): one block per cell
 //   Fc         [e][fp][8]    inviscid contravariant flux (F1 / G2)
 //   Azf        [e][fp]       A_z at the flux points (upwinded on faces after a stage,
@@ -112,6 +114,7 @@ struct SolveDev {
   double* diag;                 // per-cell diagnostic partial sums [e][2]
   const int* plot_flag;         // nonzero: the last stage records Se6 (read by E1 at run time)
   double* nQs9;                 // [e][sp][2] grad A_z of variable 9 (nablaQs(9,:,...)), kept apart from nQs
+  IxGas gas;                    // gamma for the integer fluxes
   void* pad3;                   // keeps the size a multiple of 16 bytes
 };
 
@@ -147,6 +150,7 @@ template <int N> void launch_e1(const SolveDev& s, const Launch& L, cudaStream_t
 template <int N> void launch_f1(const SolveDev& s, cudaStream_t st, int a2 = 0, int b2 = -1, int a1 = 0, int b1 = -1);
 template <int N> void launch_e2(const SolveDev& s, const Launch& L, cudaStream_t st);
 template <int N> void launch_f2(const SolveDev& s, cudaStream_t st);
+template <int N> void launch_qavg(const SolveDev& s, cudaStream_t st);
 template <int N> void launch_e3(const SolveDev& s, const RKStage& rk, const Launch& L, cudaStream_t st, int c0 = 0,
                                 int c1 = -1);
 // modes 0 and 2: cells [c0, c1); mode 1 (the face average): two-sided faces [c0, c1)

@@ -1,0 +1,418 @@
+// intflux.cuh -- the ideal-MHD point fluxes in integer arithmetic.
+//
+// GB300 executes FP64 at 2 lane-operations per clock per SM (a warp instruction occupies
+// its scheduler's FP64 unit for 64 clocks), the integer pipes take 64 each.  The nonlinear
+// fluxes are products and sums of few variables, so they are evaluated as block fixed-point
+// numbers: a value is v 2^e with a 64-bit integer v and an exponent e that a group of
+// quantities shares, products keep the upper part of the 128-bit product of two such
+// integers, sums align to the larger exponent, and each result is rounded once into a
+// double.
+//
+//   * Groups: the x and y components of the momentum (of both sides of a face), their z
+//     components, the same for B, the energies, the densities.  The z components have
+//     exponents of their own because they can be small and decoupled from the plane.
+//   * A product takes the operands as limbs v = h 2^31 + l (0 <= l < 2^31):
+//     (a b) >> 62 = ha hb + ((ha lb + la hb) >> 31) in three 32x32->64 multiply-adds; the
+//     product of the low limbs is below one unit and left out.
+//   * Values keep 57 to 61 significant bits relative to the largest term of their sum, so
+//     the errors before the final rounding stay below those of the FP64 chain, which
+//     rounds every intermediate to 53 bits.
+//
+// The integer form takes finite states with a normal positive density and exponents within
+// a wide window (2^-200 .. 2^200; zero and smaller values of momentum and B as well); everything else (infinities, NaNs, zero or negative
+// density, a density ratio above 8 across a face, a negative discriminant) is left to the
+// FP64 form, whose results on such states the caller keeps.
+#pragma once
+#include <cstdint>
+
+#include "fixdot.cuh"
+
+namespace chorus {
+
+struct Limbs {
+  int h, l;
+};
+
+FIX_HD Limbs ix_limbs(int64_t v) { return Limbs{(int)(v >> 31), (int)(v & 0x7fffffff)}; }
+
+// v >> d for d >= 0, the sign for d > 63
+FIX_HD int64_t ix_shr(int64_t v, int d) {
+#ifdef __CUDA_ARCH__
+  int64_t r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(d));  // clamps the amount
+  return r;
+#else
+  return v >> (d < 63 ? d : 63);
+#endif
+}
+FIX_HD int64_t ix_shl(int64_t v, int n) { return (int64_t)((uint64_t)v << n); }
+
+// (a b) >> 62
+FIX_HD int64_t ix_mul(Limbs a, Limbs b) {
+  const int64_t t = fix_mad(a.l, b.h, fix_mad(a.h, b.l, 0));
+  return fix_mad(a.h, b.h, t >> 31);
+}
+FIX_HD int64_t ix_mul(int64_t a, Limbs b) { return ix_mul(ix_limbs(a), b); }
+
+// a sum of products, >> 62 at the end
+struct IxSum {
+  int64_t A = 0, T = 0;
+  FIX_HD void add(Limbs a, Limbs b) {
+    T = fix_mad(a.h, b.l, T);
+    T = fix_mad(a.l, b.h, T);
+    A = fix_mad(a.h, b.h, A);
+  }
+  FIX_HD void square(Limbs a) {  // half of the cross terms: value() with shift 30
+    T = fix_mad(a.h, a.l, T);
+    A = fix_mad(a.h, a.h, A);
+  }
+  FIX_HD int64_t value() const { return A + (T >> 31); }
+  FIX_HD int64_t value2() const { return ix_shl(A, 1) + (T >> 30); }  // >> 61
+  FIX_HD int64_t value4() const { return ix_shl(A, 2) + (T >> 29); }  // >> 60
+  FIX_HD int64_t value4_squares() const { return ix_shl(A, 2) + (T >> 28); }
+};
+
+FIX_HD uint32_t ix_abs_word(double x) { return (uint32_t)(fix_bits(x) >> 32) & 0x7fffffffu; }
+FIX_HD uint32_t ix_max(uint32_t a, uint32_t b) { return a > b ? a : b; }
+FIX_HD int ix_max(int a, int b) { return a > b ? a : b; }
+
+// x as an integer aligned to the exponent of the magnitude word m >= that of x: a value of
+// that exponent has its leading bit at bit 63 - SH, i.e. v = x 2^(63 - SH + 1023 - (m >> 20))
+// truncated (a zero, which has no hidden bit, is shifted out: m is that of a group that
+// has a nonzero value, above 2^-900, or the group is all zero and not used)
+template <int SH>
+FIX_HD int64_t ix_align(double x, uint32_t m) {
+  const uint64_t u = fix_bits(x);
+  const uint32_t a = (uint32_t)(u >> 32) & 0x7fffffffu;
+  const int d = (int)(((m | 0xfffffu) + ((uint32_t)SH << 20) - a) >> 20);
+  const int64_t v = (int64_t)fix_shru((u << 11) | 0x8000000000000000ull, d);
+  return (int64_t)u < 0 ? -v : v;
+}
+// the exponent e of v 2^e for ix_align<SH>
+template <int SH>
+FIX_HD int ix_exp(uint32_t m) {
+  return (int)(m >> 20) - 1023 - (63 - SH);
+}
+
+// v 2^e as a double, rounded to nearest; results below the normal range are flushed to zero
+FIX_HD double ix_double(int64_t v, int e) { return fix_cvt_v<true>(v, e + 1); }
+
+// 2^122 / d for d in [2^61, 2^62): in (2^60, 2^61], within a few units.  The hardware
+// approximation r0 (relative error below 2^-19.9) refined by 1/D = r0 (1 + e + e^2 + ...),
+// e = 1 - D r0, to e^3 < 2^-59.
+FIX_HD int64_t ix_rcp(int64_t d) {
+  const uint32_t hi = (uint32_t)(d >> 41) & 0xfffffu;  // the 20 bits below the leading one
+#ifdef __CUDA_ARCH__
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(__hiloint2double((int)(hi | 0x3ff00000u), (int)((uint32_t)(d >> 9)))));
+  const int r0 = (int)(((uint32_t)__double2hiint(r) - (1021u << 20)) << 9);  // 2^30 / D
+#else
+  const int r0 = (int)((uint32_t)(1073741824.0 / (1.0 + hi * 0x1p-20 + 0x1p-21)) & ~511u);
+#endif
+  const Limbs D = ix_limbs(d);  // D 2^61
+  const int64_t P = fix_mad(D.h, r0, fix_mad(D.l, r0, 0) >> 31);  // D r0, 60 fraction bits
+  const int64_t e = ((int64_t)1 << 60) - P;                           // |e| < 2^40.2
+  const int eh = (int)(e >> 10);
+  const int64_t s = e + (fix_mad(eh, eh, 0) >> 40);  // e + e^2
+  const int sh = (int)(s >> 10), sl = (int)(s & 1023);
+  return ((int64_t)r0 << 31) + (fix_mad(r0, sh, fix_mad(r0, sl, 0) >> 10) >> 19);
+}
+
+// sqrt(v 2^e) for v > 0 as s 2^es, s in [2^60, 2^61]: y0 = 1/sqrt by the hardware
+// approximation (relative error below 2^-22), a = x y0, f = 1 - x y0^2,
+// sqrt x = a (1 - f)^(-1/2) = a (1 + f/2 + 3 f^2 / 8 + ...), the cubic term is below 2^-64
+FIX_HD int64_t ix_sqrt(int64_t v, int e, int& es) {
+#ifdef __CUDA_ARCH__
+  int lz = __clzll(v);
+#else
+  int lz = __builtin_clzll((uint64_t)v);
+#endif
+  // x = v << n in [2^60, 2^62) with e - n even
+  int n = lz - 2;
+  n -= (n ^ e) & 1;
+  int64_t x = n >= 0 ? (int64_t)((uint64_t)v << n) : v >> 1;
+  const int er = e - n;  // even: v 2^e = x 2^er
+  // X = x 2^-62 in [1/4, 1): y0 ~ X^-1/2 in (1, 2], 29 fraction bits
+  const float xf = (float)(uint32_t)(x >> 30);  // 2^32 X
+#ifdef __CUDA_ARCH__
+  float yf;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yf) : "f"(xf));
+#else
+  const float yf = 1.0f / __builtin_sqrtf(xf);
+#endif
+  const int y0 = (int)(yf * 0x1p45f);  // 2^16 2^29 / sqrt(2^32 X)
+  const Limbs L = ix_limbs(x);
+  const int64_t a = fix_mad(L.h, y0, fix_mad(L.l, y0, 0) >> 31);  // X y0: 60 fraction bits (62 + 29 - 31)
+  const Limbs La = ix_limbs(a);
+  const int64_t b = fix_mad(La.h, y0, fix_mad(La.l, y0, 0) >> 31);  // X y0^2: 58 fraction bits
+  const int64_t f = ((int64_t)1 << 58) - b;                               // |f| < 2^-20: below 2^38
+  const int fh = (int)(f >> 8);                                            // 50 fraction bits
+  const int64_t c = (f >> 1) + ((3 * (fix_mad(fh, fh, 0) >> 20)) >> 25);  // f/2 + 3 f^2/8, 58 fraction bits
+  const int c1 = (int)(c >> 7), c0 = (int)(c & 127);                       // 51 and 58 fraction bits
+  es = er / 2 + 31 - 61;
+  // 2 a (1 + c), a = h 2^-29 + l 2^-60
+  return a + a + (fix_mad(La.h, c1, (fix_mad(La.l, c1, 0) >> 31) + (fix_mad(La.h, c0, 0) >> 7)) >> 19);
+}
+
+// v >> d, or v << -d (where the caller knows that it fits)
+FIX_HD int64_t ix_shift(int64_t v, int d) { return d >= 0 ? ix_shr(v, d) : ix_shl(v, -d); }
+
+// leading zeros of |v| among the upper 32 bits, less `keep`: a left shift by that many bits
+// (at least 0) leaves |v| < 2^(63 - keep)
+FIX_HD int ix_room(int64_t v, int keep) {
+  const int hi = (int)(v >> 32);
+  const uint32_t a = (uint32_t)(hi ^ (hi >> 31));
+#ifdef __CUDA_ARCH__
+  return ix_max(__clz((int)a) - keep, 0);
+#else
+  return ix_max((a ? __builtin_clz(a) : 32) - keep, 0);
+#endif
+}
+
+// constants of a solve, prepared once (host or device): half of gamma - 1, gamma, as limbs
+// of normalised integers in [2^60, 2^61) with their exponents
+struct IxGas {
+  Limbs g, gam;
+  int eg, egam;
+  int eh, pad;  // E + p + B^2/2 <= (1 + gamma) E, as p >= 0 and B^2/2 <= E: below 2^(eh + 0.7) E
+};
+FIX_HD IxGas ix_gas(double gamma) {
+  IxGas c;
+  const double gm = 0.5 * (gamma - 1.0);
+  c.g = ix_limbs(ix_align<3>(gm, ix_abs_word(gm)));
+  c.eg = ix_exp<3>(ix_abs_word(gm));
+  c.gam = ix_limbs(ix_align<3>(gamma, ix_abs_word(gamma)));
+  c.egam = ix_exp<3>(ix_abs_word(gamma));
+  c.pad = 0;
+  for (c.eh = 1; c.eh < 60 && 1.0 + gamma > 1.62 * (double)(1LL << c.eh); c.eh++) {
+  }
+  return c;
+}
+
+constexpr uint32_t kIxLow = 823u << 20, kIxHigh = 1223u << 20;  // 2^-200 .. 2^200
+
+// a product as an increment of a sum: (a b) >> 61
+FIX_HD int64_t ix_prod(Limbs a, Limbs b) {
+  IxSum p;
+  p.add(a, b);
+  return p.value2();
+}
+
+// Rusanov flux along the unit normal (ux, uy) times `scale` (rusanov_core): Fh = scale
+// (Fl + Fr - eigv (qr - ql)).  q(side, k) reads variable k of the left (0) or right (1)
+// state, out(j, a, b) takes components 2 j and 2 j + 1.  Returns false, without output, where
+// the integer form does not apply.
+//
+// The two sides stream through sums (of the momentum flux, of the magnetic tension, ...) that
+// align when both are in, so that no component of the states lives longer than its side.
+// Bounds, in the comments: [b] means a magnitude below 2^b.
+template <class Q, class Out>
+FIX_HD bool rusanov_int(Q&& q, double ux, double uy, const IxGas& gas, double scale, double& eigv, Out&& out) {
+  // ---- exponents of the groups, range of the state
+  auto word = [&](int k) { return ix_max(ix_abs_word(q(0, k)), ix_abs_word(q(1, k))); };
+  const uint32_t zero = 66u << 20;  // a group of zeros: zeros are shifted out at this exponent
+  const uint32_t me = word(4), mr = word(0), ms = ix_abs_word(scale);
+  const uint32_t mm = ix_max(zero, ix_max(word(1), word(2))), mz = ix_max(zero, word(3));
+  const uint32_t mb = ix_max(zero, ix_max(word(5), word(6))), mw = ix_max(zero, word(7));
+  const uint32_t rl = (uint32_t)(fix_bits(q(0, 0)) >> 32), rr = (uint32_t)(fix_bits(q(1, 0)) >> 32);  // sign set: huge
+  const uint32_t rmin = rl < rr ? rl : rr, rmax = rl < rr ? rr : rl;
+  if (ix_max(ix_max(ix_max(rmax, me), ix_max(mm, mz)), ix_max(ix_max(mb, mw), ms)) >= kIxHigh || rmin < kIxLow ||
+      me < kIxLow || ms < kIxLow || rmax - rmin >= (3u << 20))
+    return false;
+  const int em = ix_exp<4>(mm), emz = ix_exp<4>(mz), eB = ix_exp<4>(mb), eBz = ix_exp<4>(mw), eE = ix_exp<3>(me);
+  const bool hasz = ix_max(mz, mw) != zero;
+  const Limbs nx = ix_limbs(ix_align<3>(ux, 1023u << 20)), ny = ix_limbs(ix_align<3>(uy, 1023u << 20));  // [60], 2^-60
+  // ---- densities, mass fluxes, normal velocities
+  Limbs ri[2], V[2], mx[2], my[2];
+  const int e_ri = -122 - ix_exp<2>(rmin);  // of both reciprocals
+  int64_t Vv[2], F0 = 0;
+#pragma unroll
+  for (int s = 0; s < 2; s++) {
+    const double rho = q(s, 0);
+    const uint32_t r = ix_abs_word(rho);
+    ri[s] = ix_limbs(ix_rcp(ix_align<2>(rho, r)) >> ((r >> 20) - (rmin >> 20)));  // [61]
+    mx[s] = ix_limbs(ix_align<4>(q(s, 1), mm));  // [60]
+    my[s] = ix_limbs(ix_align<4>(q(s, 2), mm));
+    IxSum f;
+    f.add(mx[s], nx); f.add(my[s], ny);
+    const int64_t f0 = f.value4();  // [60.5], em
+    F0 += f0;
+    Vv[s] = ix_mul(f0, ri[s]);
+  }
+  const int nV = ix_room((Vv[0] ^ (Vv[0] >> 63)) | (Vv[1] ^ (Vv[1] >> 63)), 3), eV = em + e_ri + 62 - nV;
+  Vv[0] = ix_shl(Vv[0], nV);  // [60]: slow flows keep their bits
+  Vv[1] = ix_shl(Vv[1], nV);
+  V[0] = ix_limbs(Vv[0]);
+  V[1] = ix_limbs(Vv[1]);
+  // ---- the sums over the sides.  z squares and products align with those of the plane.
+  int dkx = 0, dkz = 0, dbx = 0, dbz = 0, dcx = 0, dcz = 0;
+  if (hasz) {
+    const int km = ix_max(em, emz), kb = ix_max(eB, eBz), kc = ix_max(em + eB, emz + eBz);
+    dkx = 2 * (km - em); dkz = 2 * (km - emz);
+    dbx = 2 * (kb - eB); dbz = 2 * (kb - eBz);
+    dcx = kc - em - eB; dcz = kc - emz - eBz;
+  }
+  const int ek = 2 * em + dkx + 60 + e_ri + 62, eB2 = 2 * eB + dbx + 60, emB = em + eB + dcx + 60;
+  const int KS = ix_max(ix_max(eE + 1, ek), eB2);
+  const int ep = KS + gas.eg + 62, ept = ix_max(ep, eB2 - 1), eEp = eE + gas.eh;
+  const int ebn = eB + e_ri + 62;
+  int64_t aVx = 0, aVy = 0, aBx = 0, aBy = 0, aVz = 0, aBz = 0, cVz = 0, cnz = 0, bE = 0;
+  int64_t W = 0, aE = 0, ps = 0, P = 0, bns = 0, sbX = 0, sbY = 0, sbZ = 0;
+  bool ok = true;
+#pragma unroll
+  for (int s = 0; s < 2; s++) {
+    const int64_t vbx = ix_align<4>(q(s, 5), mb), vby = ix_align<4>(q(s, 6), mb);
+    sbX += vbx;
+    sbY += vby;
+    const Limbs bx = ix_limbs(vbx), by = ix_limbs(vby);
+    aVx += ix_prod(mx[s], V[s]);
+    aVy += ix_prod(my[s], V[s]);
+    IxSum b, k2, b2, mB, w;
+    b.add(bx, nx); b.add(by, ny);
+    const int64_t bn = b.value4();  // [60.5], eB
+    bns += bn;
+    const Limbs Bn = ix_limbs(bn), bnl = ix_limbs(ix_mul(bn, ri[s]));  // bnl [59.5], ebn
+    aBx += ix_prod(bx, Bn);
+    aBy += ix_prod(by, Bn);
+    k2.square(mx[s]); k2.square(my[s]);
+    b2.square(bx); b2.square(by);
+    mB.add(mx[s], bx); mB.add(my[s], by);
+    int64_t kv = k2.value4_squares(), bv = b2.value4_squares(), mBv = mB.value4();  // [61]
+    w.add(my[s], bx); w.add(mx[s], ix_limbs(-vby));
+    W += ix_mul(w.value4(), ri[s]);  // v Bx - u By, [60] a side
+    if (hasz) {
+      const int64_t vz = ix_align<4>(q(s, 3), mz), vw = ix_align<4>(q(s, 7), mw);
+      sbZ += vw;
+      const Limbs mzl = ix_limbs(vz), bzl = ix_limbs(vw);
+      IxSum kz, bz, mbz;
+      kz.square(mzl); bz.square(bzl); mbz.add(mzl, bzl);
+      kv = ix_shr(kv, dkx) + ix_shr(kz.value4_squares(), dkz);  // [61.6]
+      bv = ix_shr(bv, dbx) + ix_shr(bz.value4_squares(), dbz);
+      mBv = ix_shr(mBv, dcx) + ix_shr(mbz.value4(), dcz);
+      aVz += ix_prod(mzl, V[s]);
+      aBz += ix_prod(bzl, Bn);
+      cVz += ix_prod(bzl, V[s]);
+      cnz += ix_prod(mzl, bnl);
+    }
+    bE += ix_prod(ix_limbs(mBv), bnl);
+    const int64_t E = ix_align<3>(q(s, 4), me);  // [61]
+    const int64_t S = ix_shr(E, KS - eE - 1) - ix_shr(ix_mul(kv, ri[s]), KS - ek) - ix_shr(bv, KS - eB2);
+    ok = ok && S >= 0;  // 2 p / (gamma - 1); then [61]
+    const int64_t p = ix_mul(S, gas.g);
+    P += p;
+    const int64_t pt = ix_shr(p, ept - ep) + ix_shr(bv, ept - eB2 + 1);  // [62]
+    ps += pt >> 2;
+    aE += ix_prod(ix_limbs(ix_shr(E, gas.eh) + ix_shift(pt, eEp - ept)), V[s]);  // [61.7] [60]
+  }
+  // ---- wave speed: with P = gamma (pl + pr), T = P + 2 |B|^2, N = 2 bn^2 (B averaged) and
+  // rs = rho_l + rho_r, cf^2 = (T + sqrt(T^2 - 4 P N)) / (2 rs)
+  P = ix_mul(P, gas.gam);
+  if (!ok || P <= 0) return false;
+  int64_t eign;  // -eigv
+  int ee;
+  {
+    const int nP = ix_room(P, 3);  // (a pressure far below the energy has few bits)
+    P = ix_shl(P, nP);
+    const int eP = ep + gas.egam + 62 - nP;
+    IxSum b2;
+    b2.square(ix_limbs(sbX >> 1));
+    b2.square(ix_limbs(sbY >> 1));
+    int64_t D = b2.value4_squares();
+    if (hasz) {
+      IxSum z;
+      z.square(ix_limbs(sbZ >> 1));
+      D = ix_shr(D, dbx) + ix_shr(z.value4_squares(), dbz);
+    }
+    const Limbs bn = ix_limbs(bns);  // twice the average
+    const int K = ix_max(eP, eB2 + 1) + 1;
+    const int64_t Pk = ix_shr(P, K - eP), Nk = ix_shr(ix_mul(bn, bn), K - (2 * eB + 61));
+    const int64_t T = Pk + ix_shr(D, K - eB2 - 1);  // [61.5]
+    const Limbs Tl = ix_limbs(T);
+    const int64_t disc = ix_mul(Tl, Tl) - ix_mul(ix_shl(Pk, 1), ix_limbs(ix_shl(Nk, 1)));
+    if (disc < 0) return false;
+    int64_t U = T >> 1;  // K + 1
+    if (disc > 0) {
+      int es;
+      const int64_t sq = ix_sqrt(disc, 2 * K + 62, es);
+      U += ix_shr(sq, K + 1 - es);
+    }
+    const int64_t rs = ix_align<3>(q(0, 0), mr) + ix_align<3>(q(1, 0), mr);  // 2^60 < rs < 2^62
+    const int up = rs < ((int64_t)1 << 61) ? 1 : 0;
+    const int64_t irs = ix_rcp(ix_shl(rs, up));
+    int ec;
+    const int64_t cf = ix_sqrt(ix_mul(U, ix_limbs(irs)), K - 122 - ix_exp<3>(mr) + up + 62, ec);
+    const int64_t va = Vv[0] + Vv[1];
+    ee = ix_max(eV, ec) + 1;
+    eign = -(ix_shr(va < 0 ? -va : va, ee - eV + 1) + ix_shr(cf, ee - ec));  // [60.6]
+    eigv = ix_double(-eign, ee);
+  }
+  const Limbs eig = ix_limbs(eign), sc = ix_limbs(ix_align<3>(scale, ms));
+  const int esc = ix_exp<3>(ms) + 62;
+  auto scaled = [&](int64_t v, int e) { return ix_double(ix_mul(v, sc), e + esc); };
+  // - eigv (qr - ql) of variable k: one FP64 subtraction (the pipe has room), so that small
+  // differences keep their bits; [60.6] at exponent ed
+  auto jump = [&](int k, int& ed) {
+    const double d = q(1, k) - q(0, k);
+    const uint32_t m = ix_max(zero, ix_abs_word(d));
+    ed = ix_exp<3>(m) + ee + 61;
+    return ix_prod(ix_limbs(ix_align<3>(d, m)), eig);
+  };
+  int ed;
+  double f0, f1;
+  // ---- mass
+  {
+    const int64_t d = jump(0, ed);
+    const int K = ix_max(em, ed) + 1;
+    f0 = scaled(ix_shr(F0, K - em) + ix_shr(d, K - ed), K);
+  }
+  // ---- momentum
+  {
+    const int np = ix_room(ps, 2), epts = ept + 2 - np;
+    const Limbs pt = ix_limbs(ix_shl(ps, np));  // [61]
+    const int ea = em + eV + 61, eb = 2 * eB + 61;
+    auto component = [&](int k, int64_t aV, int64_t aB, Limbs nn) {
+      IxSum p;
+      p.add(pt, nn);
+      const int64_t d = jump(k, ed);
+      const int K = ix_max(ix_max(ea, eb), ix_max(epts, ed)) + 1;
+      return scaled(ix_shr(aV, K - ea) - ix_shr(aB, K - eb) + ix_shr(p.value4(), K - epts) + ix_shr(d, K - ed), K);
+    };
+    f1 = component(1, aVx, aBx, nx);
+    out(0, f0, f1);
+    f0 = component(2, aVy, aBy, ny);
+  }
+  f1 = 0.0;
+  if (hasz) {
+    const int64_t d = jump(3, ed);
+    const int ea = emz + eV + 61, eb = eBz + eB + 61, K = ix_max(ix_max(ea, eb), ed) + 1;
+    f1 = scaled(ix_shr(aVz, K - ea) - ix_shr(aBz, K - eb) + ix_shr(d, K - ed), K);
+  }
+  out(1, f0, f1);
+  // ---- energy
+  {
+    const int64_t d = jump(4, ed);
+    const int ea = eEp + eV + 61, eb = emB + ebn + 61, K = ix_max(ix_max(ea, eb), ed) + 1;
+    f0 = scaled(ix_shr(aE, K - ea) - ix_shr(bE, K - eb) + ix_shr(d, K - ed), K);
+  }
+  // ---- induction: (v Bx - u By) (uy, -ux) in the plane
+  {
+    const int eW = em + eB + 60 + e_ri + 62 + 1;  // of W n >> 61
+    int64_t d = jump(5, ed);
+    int K = ix_max(eW, ed) + 1;
+    f1 = scaled(ix_shr(ix_prod(ix_limbs(W), ny), K - eW) + ix_shr(d, K - ed), K);
+    out(2, f0, f1);
+    d = jump(6, ed);
+    K = ix_max(eW, ed) + 1;
+    f0 = scaled(ix_shr(ix_prod(ix_limbs(-W), nx), K - eW) + ix_shr(d, K - ed), K);
+  }
+  f1 = 0.0;
+  if (hasz) {
+    const int64_t d = jump(7, ed);
+    const int ea = eBz + eV + 61, eb = emz + ebn + 61, K = ix_max(ix_max(ea, eb), ed) + 1;
+    f1 = scaled(ix_shr(cVz, K - ea) - ix_shr(cnz, K - eb) + ix_shr(d, K - ed), K);
+  }
+  out(3, f0, f1);
+  return true;
+}
+
+}  // namespace chorus

@@ -28,6 +28,7 @@
 
 #include "chorus_internal.h"
 #include "fixdot.cuh"
+#include "intflux.cuh"
 #include "physics.cuh"
 
 namespace chorus {
@@ -438,83 +439,211 @@ __device__ __forceinline__ int active_cells(const SolveDev& s, int e0, int cnt, 
 // ---------------------------------------------------------------------------
 // F1: Rusanov flux on every face point (interfaceflux / CYCLOCFLUX / BCFLUX)
 // ---------------------------------------------------------------------------
-// one face point t of the solve's two-sided (t < nface2*N) then FREE face points;
-// returns the bit pattern of its wave speed for the block max
-template <int N>
-__device__ __forceinline__ unsigned long long f1_point(const SolveDev& s, int t) {
+// the FP64 form of a face point's flux, for the states that the integer form leaves out:
+// a call, so that it takes no registers from the points that do not need it
+static __device__ __noinline__ double rusanov_fp64(const double* pl, const double* pr, const FaceNorm* fn, double gam,
+                                            double* Fh) {
+  double ql[9], qr[9], vnl, ev;
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    ql[k] = pl[k];
+    qr[k] = pr[k];
+  }
+  rusanov_core(ql, qr, fn->ux, fn->uy, gam, fn->msl, Fh, vnl, ev);
+  return ev;
+}
+
+// asynchronous copies into shared memory
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// shared memory of one warp of the face pass, for 32 points: two buffers of their traces
+// (left and right) and face normals, their flux records, the places of the traces, and the
+// face records of three rounds
+struct F1Warp {
+  double q[2][2][32 * 9];  // [buffer][side][point][variable]
+  double2 fn[2][32][2];    // [buffer][point] FaceNorm
+  double F[32 * 9];        // [point][component], a stride of 9 against bank conflicts
+  long long g[2][2][32];   // [buffer][side][point] flux-point index; right: -1 on a FREE face
+  int4 rec[3][32];
+};
+constexpr int kF1Threads = 160;
+constexpr size_t f1_smem(int threads) { return (size_t)(threads / 32) * sizeof(F1Warp); }
+
+// Face points first .. first + 31, then on by step, ... < n of a warp (first and step are the
+// warp's, the same for its lanes); map(i) is the point's number among the solve's two-sided
+// (t < nface2*N) then FREE face points.  Returns the bit pattern of the lane's largest wave
+// speed.
+//
+// A point is one lane's work, some 1900 integer instructions at about 150 registers, so ten
+// warps share an SM: too few to hide the two dependent loads (face record, traces) behind
+// other warps.  The warp therefore copies the next 32 points' traces and the face records of
+// the 32 after them while it computes a round.  The 72-byte traces and 64-byte flux records
+// are moved by the warp together, consecutive lanes taking consecutive words of a record:
+// one lane per record would touch every 32-byte sector of the L2 four times.
+// 512x512 cells, N = 5 (GB300): 0.867 ms a stage in FP64 (80% of that pipe), 0.62 ms in integer
+// form with one thread's own loads and the averaged traces stored, 0.36 ms in this form, of
+// which the 5.1 kB per cell that it moves take 0.2 ms at the copy rate.  Ten warps at 168
+// registers: at 128 registers (16 warps) the spills go past an L1 that the traces fill, 0.73 ms.
+template <int N, class Map>
+__device__ __forceinline__ unsigned long long f1_points(const SolveDev& s, int first, int step, int n, F1Warp* warps, Map&& map) {
   constexpr int NFP = D<N>::NFP;
-  const int n2 = s.nface2 * N, n1 = s.nface1 * N;
+  const int n2 = s.nface2 * N, lane = threadIdx.x & 31;
+  F1Warp& w = warps[threadIdx.x >> 5];
+  auto fetch_rec = [&](int i, int slot) {
+    if (i >= n) return;
+    const int t = map(i);
+    if (t < n2) cp_async16(&w.rec[slot][lane], s.face2 + t / N);
+    else cp_async8(&w.rec[slot][lane], s.face1 + (t - n2) / N);
+  };
+  auto normal = [&](int t) { return t < n2 ? s.fn2 + t : s.fn1 + (t - n2); };
+  // the round whose lane has point i: where its traces are, and their copies
+  auto fetch_data = [&](int i, int slot, int buf) {
+    long long gl = -1, gr = -1;
+    if (i < n) {
+      const int t = map(i);
+      const int4 fc = w.rec[slot][lane];
+      const int nfp = t < n2 ? t % N : (t - n2) % N;
+      gl = (long long)fc.x * NFP + face_fp<N>(fc.y, nfp);
+      if (t < n2) gr = (long long)fc.z * NFP + face_fp<N>(fc.w, N - 1 - nfp);
+      const double2* pn = reinterpret_cast<const double2*>(normal(t));
+      cp_async16(&w.fn[buf][lane][0], pn);
+      cp_async16(&w.fn[buf][lane][1], pn + 1);
+    }
+    w.g[buf][0][lane] = gl;
+    w.g[buf][1][lane] = gr;
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+      const int j = r * 32 + lane, p = j / 9, k = j - 9 * p;
+      const long long pl = w.g[buf][0][p], pr = w.g[buf][1][p];
+      if (pl >= 0) {
+        cp_async8(&w.q[buf][0][j], s.Qvf + pl * 9 + k);
+        cp_async8(&w.q[buf][1][j], s.Qvf + (pr >= 0 ? pr : pl) * 9 + k);  // a FREE face has its own state on both sides
+      }
+    }
+  };
+  fetch_rec(first + lane, 0);
+  fetch_rec(first + step + lane, 1);
+  cp_async_commit();
+  pdl_wait();  // (the face records do not depend on the pass before)
+  cp_async_wait();
+  fetch_data(first + lane, 0, 0);
+  cp_async_commit();
   unsigned long long evb = 0ull;
-  if (t < n2 + n1) {
-    const bool two = t < n2;
-    const int tt = two ? t : t - n2;
-    const int f = tt / N, nfp = tt - f * N;
-    size_t gl, gr = 0;
-    FaceNorm fn;
-    if (two) {
-      const int4 fc = s.face2[f];
-      gl = (size_t)fc.x * NFP + face_fp<N>(fc.y, nfp);
-      gr = (size_t)fc.z * NFP + face_fp<N>(fc.w, N - 1 - nfp);
-      fn = s.fn2[tt];
-    } else {
-      const int2 fc = s.face1[f];
-      gl = (size_t)fc.x * NFP + face_fp<N>(fc.y, nfp);
-      fn = s.fn1[tt];
-    }
-    double ql[9], qr[9];
-    const double* pl = s.Qvf + gl * 9;
+  int buf = 0, slot = 0;
+#pragma unroll 1
+  for (int i0 = first; i0 < n; i0 += step) {
+    const int next = slot == 2 ? 0 : slot + 1, i = i0 + lane;
+    cp_async_wait();  // this round's traces, the next round's records
+    __syncwarp();
+    fetch_data(i + step, next, buf ^ 1);
+    fetch_rec(i + 2 * step, next == 2 ? 0 : next + 1);
+    cp_async_commit();
+    if (i < n) {
+      const int t = map(i);
+      const long long gl = w.g[buf][0][lane], gr = w.g[buf][1][lane];
+      const double2 nrm = w.fn[buf][lane][0];
+      // (the states are read from shared memory where they are used, not kept)
+      const volatile double* ql = w.q[buf][0] + 9 * lane;
+      const volatile double* qr = w.q[buf][1] + 9 * lane;
+      double* F = w.F + 9 * lane;
+      auto put = [&](int j, double a, double b) {
+        F[2 * j] = a;
+        F[2 * j + 1] = b;
+      };
+      double ev;
+      if (!rusanov_int([&](int side, int k) { return side ? qr[k] : ql[k]; }, nrm.x, nrm.y, s.gas, w.fn[buf][lane][1].x, ev, put)) {
+        double Fd[8];
+        ev = rusanov_fp64(w.q[buf][0] + 9 * lane, w.q[buf][1] + 9 * lane, normal(t), s.gam, Fd);
 #pragma unroll
-    for (int k = 0; k < 9; k++) ql[k] = pl[k];
-    if (two) {
-      const double* pr = s.Qvf + gr * 9;
-#pragma unroll
-      for (int k = 0; k < 9; k++) qr[k] = pr[k];
-    } else {
-#pragma unroll
-      for (int k = 0; k < 9; k++) qr[k] = ql[k];
-    }
-    double Fh[8], vnl, ev;
-    rusanov_core(ql, qr, fn.ux, fn.uy, s.gam, fn.msl, Fh, vnl, ev);
-    evb = ev_bits(ev, s.err);
-    const double az = vnl > 0.0 ? ql[8] : qr[8];
-    double2* fl = reinterpret_cast<double2*>(s.Fc + gl * 8);  // 64-byte flux records
-#pragma unroll
-    for (int k = 0; k < 4; k++) fl[k] = make_double2(Fh[2 * k], Fh[2 * k + 1]);
-    s.Azf[gl] = az;
-    if (two && s.skip && nfp == 0) {
-      const int4 fc = s.face2[f];
-      if (s.act[fc.x] | s.act[fc.z]) {
-        s.nv[fc.x] = 1;
-        s.nv[fc.z] = 1;
+        for (int j = 0; j < 4; j++) put(j, Fd[2 * j], Fd[2 * j + 1]);
+      }
+      const unsigned long long e = ev_bits(ev, s.err);
+      evb = e > evb ? e : evb;
+      // A_z from the upwind side (getrusanov.f90:99-103); the sign of u.n is that of m.n
+      const double az = fma(ql[1], nrm.x, ql[2] * nrm.y) > 0.0 ? ql[8] : qr[8];
+      s.Azf[gl] = az;
+      if (gr >= 0) {
+        s.Azf[gr] = az;
+        if (s.skip && t % N == 0) {
+          const int4 fc = w.rec[slot][lane];
+          if (s.act[fc.x] | s.act[fc.z]) {
+            s.nv[fc.x] = 1;
+            s.nv[fc.z] = 1;
+          }
+        }
       }
     }
-    if (two) {
-      double2* fr = reinterpret_cast<double2*>(s.Fc + gr * 8);
+    __syncwarp();
+    // the flux records, four lanes to a record
 #pragma unroll
-      for (int k = 0; k < 4; k++) fr[k] = make_double2(times_sign(Fh[2 * k], fn.ss), times_sign(Fh[2 * k + 1], fn.ss));
-      s.Azf[gr] = az;
-      double* al = s.Qvf + gl * 9;
-      double* ar = s.Qvf + gr * 9;
-#pragma unroll
-      for (int k = 0; k < 9; k++) {
-        const double a = half(ql[k] + qr[k]);
-        al[k] = a;
-        ar[k] = a;
+    for (int r = 0; r < 4; r++) {
+      const int p = r * 8 + (lane >> 2), j = lane & 3;
+      const long long pl = w.g[buf][0][p], pr = w.g[buf][1][p];
+      if (pl < 0) continue;
+      const double a = w.F[9 * p + 2 * j], b = w.F[9 * p + 2 * j + 1];
+      reinterpret_cast<double2*>(s.Fc + pl * 8)[j] = make_double2(a, b);
+      if (pr >= 0) {
+        const double ss = w.fn[buf][p][1].y;
+        reinterpret_cast<double2*>(s.Fc + pr * 8)[j] = make_double2(times_sign(a, ss), times_sign(b, ss));
       }
     }
+    __syncwarp();
+    buf ^= 1;
+    slot = next;
   }
   return evb;
 }
 
 // face points [t2, t2 + n2) of the two-sided list, then [t1, t1 + n - n2) of the FREE list
-// (f1_point numbering: the FREE faces follow the two-sided ones)
+// (f1_points numbering: the FREE faces follow the two-sided ones)
 template <int N>
-__global__ void __launch_bounds__(256, 3) k_f1(SolveDev s, int t2, int n2, int t1, int n) {
-  pdl_wait();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned long long evb = 0ull;
-  if (i < n) evb = f1_point<N>(s, i < n2 ? t2 + i : t1 + (i - n2));
+__global__ void __launch_bounds__(kF1Threads, 2) k_f1(SolveDev s, int t2, int n2, int t1, int n) {
+  extern __shared__ __align__(16) double sm[];
+  const int nw = blockDim.x >> 5;
+  const unsigned long long evb = f1_points<N>(s, (blockIdx.x * nw + (threadIdx.x >> 5)) * 32, gridDim.x * nw * 32, n,
+                                              reinterpret_cast<F1Warp*>(sm),
+                                              [&](int i) { return i < n2 ? t2 + i : t1 + (i - n2); });
   block_max_ull(evb, s.eig);
+}
+
+// the traces of the two-sided faces replaced by their mean (interfaceflux /
+// CYCLOCFLUX, interfaceflux_all.f90:79-91).  A stage takes the mean where it reads the traces
+// (E2, E3: few cells as a rule); this pass makes the stored traces equal to the reference's
+// Qvfi/Qvfj where they are downloaded or differentiated.  (A second run changes nothing.)
+template <int N>
+__global__ void __launch_bounds__(256) k_qavg(SolveDev s) {
+  constexpr int NFP = D<N>::NFP;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= s.nface2 * N) return;
+  const int f = t / N, nfp = t - f * N;
+  const int4 fc = s.face2[f];
+  double* a = s.Qvf + ((size_t)fc.x * NFP + face_fp<N>(fc.y, nfp)) * 9;
+  double* b = s.Qvf + ((size_t)fc.z * NFP + face_fp<N>(fc.w, N - 1 - nfp)) * 9;
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const double v = half(a[k] + b[k]);
+    a[k] = v;
+    b[k] = v;
+  }
+}
+
+// the flux point across the face from point fp of cell c: its index among all flux points, or
+// -1 for an interior point and on a FREE face
+template <int N>
+__device__ __forceinline__ long long across(const SolveDev& s, int c, int fp) {
+  int nfp = 0;
+  const int lf = fp_face<N>(fp, nfp);
+  const int o = lf ? (&s.nbr[c].x)[lf - 1] : -1;
+  if (o < 0) return -1;
+  return (long long)o * D<N>::NFP + face_fp<N>((&s.nbrlf[c].x)[lf - 1], N - 1 - nfp);
 }
 
 // ---------------------------------------------------------------------------
@@ -554,7 +683,8 @@ __device__ __forceinline__ void e2_cells(const SolveDev& s, const int* cells, in
   for (int i = threadIdx.x; i < n * NFP * 8; i += blockDim.x) {
     const int le = i / (NFP * 8), r = i - le * (NFP * 8), fp = r >> 3, k = r & 7;
     const size_t g = (size_t)cells[le] * NFP + fp;
-    const double q = s.Qvf[g * 9 + k];
+    const long long o = across<N>(s, cells[le], fp);  // face traces enter as the mean of both sides
+    const double own = s.Qvf[g * 9 + k], q = o >= 0 ? half(own + s.Qvf[o * 9 + k]) : own;
     sP[(le * NFP + fp) * 16 + k] = q * s.met[2 * g];
     sP[(le * NFP + fp) * 16 + 8 + k] = q * s.met[2 * g + 1];
   }
@@ -741,30 +871,28 @@ __device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int 
       double q[9], gq[18], Fv[8];
       const double* pq = s.Qvf + g * 9;
       const double* pg = s.nQvf + g * 18;
-#pragma unroll
-      for (int k = 0; k < 8; k++) q[k] = pq[k];
-      q[8] = 0.0;
-      // on a two-sided face the trace of grad Q is the mean of both sides'
-      // (interfaceVISflux / CYCLOCVISFLUX, interfaceflux_all.f90:118-199,
-      // cyclocflux_all.f90:118-208); a FREE face keeps its own (BCVISFLUX)
-      int nfp = 0;
-      const int lf = fp_face<N>(fp, nfp);
-      const int o = lf ? (&s.nbr[c].x)[lf - 1] : -1;
+      // on a two-sided face the traces of Q and of grad Q are the means of both sides'
+      // (interfaceflux_all.f90:79-91, 118-199, cyclocflux_all.f90:118-208); a FREE face keeps
+      // its own (BCVISFLUX)
+      const long long o = across<N>(s, c, fp);
       if (o >= 0) {
-        const int olf = (&s.nbrlf[c].x)[lf - 1];
-        const double* po = s.nQvf + ((size_t)o * NFP + face_fp<N>(olf, N - 1 - nfp)) * 18;
+        const double* qo = s.Qvf + o * 9;
+        const double* po = s.nQvf + o * 18;
 #pragma unroll
         for (int k = 0; k < 8; k++) {
+          q[k] = half(pq[k] + qo[k]);
           gq[k] = half(pg[k] + po[k]);
           gq[9 + k] = half(pg[9 + k] + po[9 + k]);
         }
       } else {
 #pragma unroll
         for (int k = 0; k < 8; k++) {
+          q[k] = pq[k];
           gq[k] = pg[k];
           gq[9 + k] = pg[9 + k];
         }
       }
+      q[8] = 0.0;
       gq[8] = 0.0;
       gq[17] = 0.0;
       vflux_contra(q, gq, mut, s.eta0, s.gam, s.met[2 * g], s.met[2 * g + 1], Fv);

@@ -1,5 +1,7 @@
 // kernels_inst.cuh -- explicit instantiation of the stage kernels for N = CHORUS_N.
 // Each translation unit holds its own constant-memory copy of the N-point operators.
+#include <algorithm>
+
 #include "kernels.cuh"
 
 #ifndef CHORUS_N
@@ -28,6 +30,18 @@ inline int grid_cells(int nc, int epb) { return (nc + epb - 1) / epb; }
 // eight CTAs per SM (small meshes), so that the points spread over every SM
 inline int face_threads(int n) { return n >= 152 * 8 * 256 ? 256 : 64; }
 
+// SMs of the current device, looked up once
+int sm_count() {
+  static int nsm_of[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return 152;
+  if (!nsm_of[dev] && (cudaDeviceGetAttribute(&nsm_of[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+                       nsm_of[dev] <= 0))
+    nsm_of[dev] = 152;
+  return nsm_of[dev];
+}
+
 void set_smem_limits() {
   static bool done[64] = {false};
   int dev = 0;
@@ -36,6 +50,7 @@ void set_smem_limits() {
   const int lim = 200 * 1024;
   cudaFuncSetAttribute(k_e1<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_e2<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(k_f1<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_e3<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_ct_elem<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_diag_interp<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
@@ -63,27 +78,27 @@ void launch_f1<kN>(const SolveDev& s, cudaStream_t st, int a2, int b2, int a1, i
   if (b2 < 0) b2 = s.nface2;
   if (b1 < 0) b1 = s.nface1;
   const int n2 = (b2 - a2) * kN, n = n2 + (b1 - a1) * kN;
+  // two resident CTAs of 256 threads per SM walk the points; fewer points than that go one
+  // to a thread, in CTAs of 64 so that they spread over every SM
+  const int thr = n >= 2 * kF1Threads * sm_count() ? kF1Threads : 64;
+  const int grid = std::min((n + thr - 1) / thr, thr == kF1Threads ? 2 * sm_count() : n);
   if (n > 0)
-    launch_pdl(k_f1<kN>, (n + face_threads(n) - 1) / face_threads(n), face_threads(n), 0, st, s, a2 * kN, n2,
-               (s.nface2 + a1) * kN, n);
+    launch_pdl(k_f1<kN>, grid, thr, f1_smem(thr), st, s, a2 * kN, n2, (s.nface2 + a1) * kN, n);
 }
 template <>
 void launch_e2<kN>(const SolveDev& s, const Launch& L, cudaStream_t st) {
   // chunks of up to one cell per thread, but small enough for about 16 CTAs per SM
-  static int nsm_of[64];  // SM count per device, looked up once
-  int dev = 0, nsm = 152;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64) {
-    if (!nsm_of[dev] && (cudaDeviceGetAttribute(&nsm_of[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-                         nsm_of[dev] <= 0))
-      nsm_of[dev] = 152;
-    nsm = nsm_of[dev];
-  }
+  const int nsm = sm_count();
   int chunk = s.NC / (16 * nsm);
   chunk = chunk < L.epb ? L.epb : (chunk > L.threads ? L.threads : chunk);
   chunk -= chunk % L.epb;
   if (!s.skip) chunk = L.epb;  // every cell needs its gradients: one group per CTA
   launch_pdl(k_e2<kN>, grid_cells(s.NC, chunk), L.threads, smem_e2(L.epb), st, s, L.epb, chunk);
+}
+template <>
+void launch_qavg<kN>(const SolveDev& s, cudaStream_t st) {
+  const int n = s.nface2 * kN;
+  if (n > 0) k_qavg<kN><<<(n + face_threads(n) - 1) / face_threads(n), face_threads(n), 0, st>>>(s);
 }
 template <>
 void launch_f2<kN>(const SolveDev& s, cudaStream_t st) {

@@ -29,14 +29,18 @@ __host__ __device__ __forceinline__ double rcp_pos(double x) {
 #endif
 }
 
-// x/2 without an FP64 instruction: decrement the exponent field (exact for normal
-// numbers, the same value as 0.5*x); zeros, subnormals, infinities and NaNs take the
-// multiply.  0.5*a + 0.5*b == half(a + b) bit for bit for normal operands.
+// x/2 without an FP64 instruction (a multiplication for the rare values would be predicated
+// and take its time for all): the exponent field less one for normal results; zeros and
+// results below the normal range shift the significand, rounded to nearest even as the
+// multiplication does; infinities and NaNs stay.  0.5*a + 0.5*b == half(a + b) bit for bit for
+// normal operands.
 __host__ __device__ __forceinline__ double half(double x) {
 #ifdef __CUDA_ARCH__
-  const long long b = __double_as_longlong(x);
-  const int ex = (int)((b >> 52) & 0x7FF);
-  return (ex > 1 && ex < 0x7FF) ? __longlong_as_double(b - (1LL << 52)) : 0.5 * x;
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x), m = b & 0x7fffffffffffffffULL;
+  const int ex = (int)(m >> 52);
+  const unsigned long long tiny = (m >> 1) + (m & (m >> 1) & 1);
+  const unsigned long long r = ex > 1 ? (ex < 0x7FF ? m - (1ULL << 52) : m) : tiny;
+  return __longlong_as_double((long long)(r | (b & 0x8000000000000000ULL)));
 #else
   return 0.5 * x;
 #endif
