@@ -134,7 +134,8 @@ __global__ void __launch_bounds__(512, 2) kg_e3(BatchDev b, int stage) {
   for_tiles(b, gidx(PE3, N), b.ctiles, [&](const int4& T, const SolveDev& s) {
     if (threadIdx.x == 0) srk = b.rk[stage * b.cap + T.x];
     __syncthreads();
-    e3_body<N, OpsAll<N>>(s, T.y, T.z, T.z, srk, 1, sm);
+    if (e3_pre(srk, 1)) e3_body<N, OpsAll<N>, true>(s, T.y, T.z, T.z, srk, 1, sm);
+    else e3_body<N, OpsAll<N>, false>(s, T.y, T.z, T.z, srk, 1, sm);
   });
 }
 
@@ -162,7 +163,7 @@ size_t cell_smem_bytes(int N, int epb, int pass) {
   switch (pass) {
     case 0: d = (size_t)epb * (NS * 9 + 2 * NS + NFP * 9) + N * N; break;
     case 1: d = (size_t)epb * (NFP * 16 + NS * 17); break;
-    case 2: d = (size_t)epb * (NFP * 8 + NS * (1 + 9 + 1 + 2) + NFP * 2); break;
+    case 2: return e3_smem(N, epb);
     default: d = (size_t)epb * (NFP * 2 + NS * 2); break;
   }
   return sizeof(double) * d;

@@ -81,6 +81,16 @@ static void make_ops(int N, const double* Lmat, const double* Mmat, const double
   fix_mirror_coefs(Lrow, N + 1, N, 1, o.LS, o.LH, o.LL);
   o.MS = fix_shift_for(Mmat, (N + 1) * N);
   fix_mirror_coefs(Mmat, N, N + 1, -1, o.MS, o.MH, o.ML);
+  // |sum| <= sum over the row of |c| for inputs below 2^58: two of them shifted by MV add up to
+  // less than 2^62
+  double row = 0.0;
+  for (int i = 0; i < N; i++) {
+    double a = 0.0;
+    for (int r = 0; r <= N; r++) a += std::fabs(Mmat[r + (N + 1) * i]);
+    row = std::max(row, a);
+  }
+  for (o.MV = 0; std::ldexp(row, o.MS - o.MV) > 0x1.f0p60; o.MV++) {
+  }
   // AV smoothing A = Hlow * H: project N points onto the N-1 low-order points
   // (hhval at Xs_low, AV.f90:19-35) and evaluate back (hhval_low at Xs, :41-58)
   double xsl[kMaxN], xfl[kMaxN + 1];
@@ -141,14 +151,13 @@ static const Dispatch* dispatch_for(int N) {
 // default launch shapes per N (cells per CTA, threads per CTA)
 Launch default_launch(int N, int which) {
   // which: 0 = E1, 1 = E2, 2 = E3, 3 = CT; cells per CTA and threads per CTA as the
-  // autotuner picked them on GB300 for N = 3..6 (for N = 6 the shapes of an earlier tuning,
-  // which the batched form runs faster); the CT passes take about 128/(2N) cells
-  // so that their (cell, line) loop fills the 128 threads
-  static const int epb[kMaxN + 1][4] = {{0}, {0}, {16, 16, 16, 32}, {16, 4, 2, 21}, {4, 4, 4, 16},
-                                        {4, 2, 5, 12}, {3, 2, 2, 10}, {2, 2, 2, 9}, {2, 2, 2, 8}};
-  static const int thr[kMaxN + 1][4] = {{0}, {0}, {128, 128, 128, 128}, {224, 128, 32, 128}, {128, 128, 96, 128},
-                                        {128, 128, 160, 128}, {96, 192, 128, 128}, {128, 128, 128, 128},
-                                        {128, 128, 128, 128}};
+  // autotuner's sweep picked them on GB300 (2 M solution points); the CT passes take about
+  // 128/(2N) cells so that their (cell, line) loop fills the 128 threads
+  static const int epb[kMaxN + 1][4] = {{0}, {0}, {16, 6, 16, 32}, {16, 4, 8, 21}, {4, 4, 6, 16},
+                                        {4, 2, 5, 12}, {3, 2, 3, 10}, {2, 1, 3, 9}, {2, 1, 2, 8}};
+  static const int thr[kMaxN + 1][4] = {{0}, {0}, {128, 96, 96, 128}, {224, 128, 96, 128}, {128, 128, 128, 128},
+                                        {128, 128, 128, 128}, {96, 192, 128, 128}, {128, 128, 224, 128},
+                                        {128, 128, 160, 128}};
   return Launch{epb[N][which], thr[N][which]};
 }
 

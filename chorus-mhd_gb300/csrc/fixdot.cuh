@@ -269,8 +269,11 @@ FIX_HD double fix_cvt_v(int64_t V, int k) {
 // 512x512 cells, N = 5 (GB300): E3 1.361 -> 1.150 ms per stage, the step 18.2 -> 17.2 ms.
 // Bounds for NI <= 9 with |P +- Q| < 2^59, |X| < 2^58: |A| < 9 2^59, and the partial sums
 // over U or W alone < 4 2^60 + 2^59; |B| < 9 (2^58 + 2^58) + 2^28: all below 2^63.
-template <int NO, int NI, int SIGMA, bool CHECK>
-FIX_HD void fix_mirror_line(const double (&v)[NI], int emax, const int* ch, const int* cl, int k, double (&y)[NO]) {
+//
+// fix_mirror_sums hands out the sums V of the rows as they are formed, put(row, V): y =
+// V 2^(k-1) with k as in fix_dot, |V| at most the row's sum of |c|, below 2^62.2.
+template <int NO, int NI, int SIGMA, class Put>
+FIX_HD void fix_mirror_sums(const double (&v)[NI], int emax, const int* ch, const int* cl, Put&& put) {
   constexpr int NP = NI / 2;
   int64_t X[NI];
   const uint32_t eb = ((uint32_t)emax << 20) | 0xfffffu;
@@ -323,12 +326,17 @@ FIX_HD void fix_mirror_line(const double (&v)[NI], int emax, const int* ch, cons
         Bw = fix_mad(ol[j], rh[NP + j], Bw);
       }
     }
-    y[r] = fix_round_v<CHECK>(Au + Aw + ((Bu + Bw) >> kFixSplit), k);
+    put(r, Au + Aw + ((Bu + Bw) >> kFixSplit));
     if (!mid) {
       const int64_t V = Au - Aw + ((Bu - Bw) >> kFixSplit);
-      y[NO - 1 - r] = fix_round_v<CHECK>(SIGMA > 0 ? V : -V, k);
+      put(NO - 1 - r, SIGMA > 0 ? V : -V);
     }
   }
+}
+
+template <int NO, int NI, int SIGMA, bool CHECK>
+FIX_HD void fix_mirror_line(const double (&v)[NI], int emax, const int* ch, const int* cl, int k, double (&y)[NO]) {
+  fix_mirror_sums<NO, NI, SIGMA>(v, emax, ch, cl, [&](int r, int64_t V) { y[r] = fix_round_v<CHECK>(V, k); });
 }
 
 // the same for any finite line with emax <= kFixEmaxFast: lines below kFixEmaxMin are scaled

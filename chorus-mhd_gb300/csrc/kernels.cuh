@@ -85,6 +85,7 @@ struct OpsN {
   int MH[(kMaxN + 1) * kMaxN];
   int ML[(kMaxN + 1) * kMaxN];
   int MS;
+  int MV;  // right shift that keeps the sum of two derivative sums (fix_mirror_sums) below 2^62
 };
 
 // one copy per translation unit; upload_ops_n<N>() fills it
@@ -187,6 +188,39 @@ __device__ __forceinline__ void block_copy(double* dst, const double* src, int n
   }
 }
 
+// asynchronous copies into shared memory
+__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// dst[0..n) = src[0..n) by the whole CTA, asynchronously; dst is 16-byte aligned, src is as its
+// place in the array has it (pieces of 16 bytes where it is too)
+__device__ __forceinline__ void block_copy_async(double* dst, const double* src, int n) {
+  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    for (int i = threadIdx.x; i < (n >> 1); i += blockDim.x) cp_async16(dst + 2 * i, src + 2 * i);
+    if ((n & 1) && threadIdx.x == 0) cp_async8(dst + n - 1, src + n - 1);
+  } else {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) cp_async8(dst + i, src + i);
+  }
+}
+
+// dst[0..n) = src[0..n) by the whole CTA, src in shared memory, in 16-byte stores from the first
+// 16-byte boundary of dst on
+__device__ __forceinline__ void block_copy_out(double* dst, const double* src, int n) {
+  const int head = (int)((reinterpret_cast<uintptr_t>(dst) >> 3) & 1);
+  double2* d2 = reinterpret_cast<double2*>(dst + head);
+  const int pairs = (n - head) >> 1;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < pairs; i += blockDim.x) d2[i] = make_double2(src[head + 2 * i], src[head + 2 * i + 1]);
+  if (threadIdx.x == 0 && head) dst[0] = src[0];
+  if (threadIdx.x == 0 && head + 2 * pairs < n) dst[n - 1] = src[n - 1];
+}
+
 // element-local flux-point index of the i-th interior flux point (i < 2N(N-1)):
 // family 1 with ifp = 1..N-1, then family 2 with jfp = 1..N-1
 template <int N>
@@ -255,9 +289,6 @@ __device__ __forceinline__ void deriv_line(const double* x, int xs, double (&y)[
   }
 }
 
-// ---------------------------------------------------------------------------
-// E3: viscous + AV flux, divergence, A_z advection, RK update
-// ---------------------------------------------------------------------------
 template <int N, class O>
 __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int epb, int sensor, double* sm) {
   constexpr int NS = D<N>::NS, NF1 = D<N>::NF1, NFP = D<N>::NFP, NINT = 2 * N * (N - 1);
@@ -452,16 +483,6 @@ static __device__ __noinline__ double rusanov_fp64(const double* pl, const doubl
   rusanov_core(ql, qr, fn->ux, fn->uy, gam, fn->msl, Fh, vnl, ev);
   return ev;
 }
-
-// asynchronous copies into shared memory
-__device__ __forceinline__ void cp_async8(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // shared memory of one warp of the face pass, for 32 points: two buffers of their traces
 // (left and right) and face normals, their flux records, the places of the traces, and the
@@ -821,38 +842,12 @@ __global__ void __launch_bounds__(256) k_f2(SolveDev s) {
   f2_point<N>(s, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+// the viscous, resistive and AV flux of the nact listed cells of the block, subtracted from
+// their total flux in shared memory: a call, so that the registers it needs are not those of
+// the whole pass
 template <int N, class O>
-__device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int epb, const RKStage& rk, int update, double* sm) {
-  constexpr int NS = D<N>::NS, NF1 = D<N>::NF1, NFP = D<N>::NFP;
-
-  double* sF = sm;                  // [epb][NFP][8] F - Fv, the negated total flux
-  double* sD = sF + epb * NFP * 8;  // [epb][NS] diagnostic partial sums
-  double* sR = sD + epb * NS;       // [epb][NS][9] residual
-  double* sJ = sR + epb * NS * 9;   // [epb][NS] 1/J
-  double* sZ = sJ + epb * NS;       // [epb][NFP][2] A_z * (S_x, S_y) at the flux points
-  double* sN = sZ + epb * NFP * 2;  // [epb][NS][2] grad A_z
-  __shared__ int list[64];
-  const int nact = active_cells(s, e0, cnt, 1, list);
-  {
-    // contiguous block copies (coalesced), issued together so their latencies overlap;
-    // the state itself is read where it is used (the update is elementwise over the
-    // block's contiguous state)
-    // (16-byte loads: Fc's per-cell block and each metric pair are 16-byte aligned)
-    const double2* fi = reinterpret_cast<const double2*>(s.Fc + (size_t)e0 * NFP * 8);
-    double2* sF2 = reinterpret_cast<double2*>(sF);
-#pragma unroll 4
-    for (int i = threadIdx.x; i < cnt * NFP * 4; i += blockDim.x) sF2[i] = fi[i];
-    for (int i = threadIdx.x; i < cnt * NS; i += blockDim.x) sJ[i] = s.invJ[(size_t)e0 * NS + i];
-    const double2* met2 = reinterpret_cast<const double2*>(s.met);
-    for (int i = threadIdx.x; i < cnt * NFP; i += blockDim.x) {
-      const size_t g = (size_t)e0 * NFP + i;
-      const double z = s.Azf[g];
-      const double2 m = met2[g];
-      sZ[2 * i] = z * m.x;
-      sZ[2 * i + 1] = z * m.y;
-    }
-  }
-  __syncthreads();
+static __device__ __noinline__ void e3_viscous(const SolveDev& s, int e0, int nact, const int* list, double* sF) {
+  constexpr int NF1 = D<N>::NF1, NFP = D<N>::NFP;
   for (int t = threadIdx.x; t < nact * NFP; t += blockDim.x) {
     const int le = t / NFP, fp = t - le * NFP, e = list[le], c = e0 + e;
     const size_t g = (size_t)c * NFP + fp;
@@ -901,82 +896,242 @@ __device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int 
       for (int k = 1; k < 8; k++) d[k] -= Fv[k];
     }
   }
-  __syncthreads();
+}
+
+// shared memory of the pass for epb cells (e3_body)
+constexpr size_t e3_smem(int N, int epb) {
+  return (size_t)epb * ((size_t)2 * (N + 1) * N * 10 * 8 + (size_t)N * N * (72 + 16 + 8 + 4) + (size_t)N * 10 * 4) + 16;
+}
+
+constexpr int kE3Fp64 = -(1 << 28);  // in place of an exponent: the value is a double
+
+// 1/J (sum of the two families' derivatives) where one of the three is not in integer form: a
+// call, because a branch of few FP64 instructions would be predicated, and an FP64 instruction
+// occupies its pipe whether its lanes are on or off.  k0, k1: exponents of the sums V0, V1 or
+// kE3Fp64 for doubles.
+static __device__ __noinline__ double e3_fp64(int64_t V0, int k0, int64_t V1, int k1, double j) {
+  const double y0 = k0 != kE3Fp64 ? ix_double(V0, k0) : __longlong_as_double(V0);
+  const double y1 = k1 != kE3Fp64 ? ix_double(V1, k1) : __longlong_as_double(V1);
+  return (y0 + y1) * j;
+}
+
+// does a stage only need its increment cR * resid, so that cR is folded into 1/J?
+__host__ __device__ inline bool e3_pre(const RKStage& rk, int update) {
+  return update && !rk.write_resid && !rk.save_R && !rk.diag;
+}
+
+// PRE = e3_pre(rk, update): two bodies, since FP64 instructions that a stage does not need
+// would be predicated and still take their time
+template <int N, class O, bool PRE>
+__device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int epb, const RKStage& rk, int update, double* sm) {
+  constexpr int NS = D<N>::NS, NF1 = D<N>::NF1, NFP = D<N>::NFP;
+  constexpr int NQ = 10;  // line quantities: eight flux components, two of A_z S
+
+  double* sF = sm;                                          // [epb][NFP][8] total flux, then the residual
+  double* sZ = sF + epb * NFP * 8;                          // [epb][NFP][2] A_z * (S_x, S_y), then grad A_z
+  double* sQ = sZ + epb * NFP * 2;                          // [epb][NS][9] state (16-byte aligned: NFP is even)
+  double* sU = sQ + ((epb * NS * 9 + 1) & ~1);              // [epb][NS][2] u, v; then the residual of A_z
+  int64_t* sJ = reinterpret_cast<int64_t*>(sU + epb * NS * 2);  // [epb][NS] 1/J as an integer
+  double* sD = sU + epb * NS * 2;                           // [epb][NS] diagnostic sums, in its place
+  int* sE = reinterpret_cast<int*>(sJ + epb * NS);          // [epb][NS] and its exponent
+  int* sK = sE + epb * NS;                                  // [epb][N][NQ] exponents of the xi-line sums
+  __shared__ int list[64];
+  // the residual of solution point p = (is, js) of a cell stands in the slot of family-1 flux
+  // point js (N+1) + is, which its xi line has consumed
+  auto slot = [](int e, int p) { return e * NFP + p + p / N; };
+  // the block's fluxes and state, copied while the rest of the inputs is read
+  block_copy_async(sF, s.Fc + (size_t)e0 * NFP * 8, cnt * NFP * 8);
+  block_copy_async(sQ, s.Q + (size_t)e0 * NS * 9, cnt * NS * 9);
+  cp_async_commit();
+  {
+    for (int i = threadIdx.x; i < cnt * NS; i += blockDim.x) {
+      double j = s.invJ[(size_t)e0 * NS + i];
+      if (PRE) j *= rk.cR;
+      const uint32_t m = ix_abs_word(j);
+      sJ[i] = ix_align<2>(j, m);
+      sE[i] = m >= kIxLow && m < kIxHigh ? ix_exp<2>(m) : kE3Fp64;
+    }
+    const double2* met2 = reinterpret_cast<const double2*>(s.met);
+    for (int i = threadIdx.x; i < cnt * NFP; i += blockDim.x) {
+      const size_t g = (size_t)e0 * NFP + i;
+      const double z = s.Azf[g];
+      const double2 m = met2[g];
+      sZ[2 * i] = z * m.x;
+      sZ[2 * i + 1] = z * m.y;
+    }
+  }
+  cp_async_wait();
+  const int nact = active_cells(s, e0, cnt, 1, list);  // (ends with a barrier)
+  if (nact) {
+    e3_viscous<N, O>(s, e0, nact, list, sF);
+    __syncthreads();
+  }
   // divergence of the total flux and grad A_z in the conservative form of nablaAsp
-  // (magnetic_potential.f90:1-42), (1/J) sum_r Mmat (A_z S): ten line quantities per
-  // cell (eight flux components, two A_z S components), each differentiated along its
-  // lines on the integer pipes, one (cell, line, quantity) per thread; first the
-  // family-1 lines (xi), then the family-2 lines (eta), which add to them and scale by
-  // 1/J
-  constexpr int NQ = 10;
+  // (magnetic_potential.f90:1-42), (1/J) sum_r Mmat (A_z S): ten line quantities per cell,
+  // each differentiated along its lines on the integer pipes, one (cell, line, quantity) per
+  // thread; first the family-1 lines (xi), whose sums stay integers with one exponent per
+  // line, then the family-2 lines (eta), which add theirs, multiply by 1/J and round once.
+  // In integers these two operations cost about 20 instructions a value on pipes that the
+  // FP64 work of the pass leaves idle, against 2 FP64 operations of 64 clocks a warp, and the
+  // xi sums are not rounded in between.
+  // 512x512 cells, N = 5 (GB300), a stage without terms of earlier states: 1.15 ms with the two
+  // operations in FP64, the state read from global memory where it is used and predicated FP64
+  // instructions (see PRE), 0.73 ms in this form; 9.2 kB per cell take 0.36 ms at the copy rate.
+  // (the stage update takes the state's place as the residual appears: what else reads the old
+  // state does so here)
+  if (update && rk.save_old) block_copy_out(rk.save_old + (size_t)e0 * NS * 9, sQ, cnt * NS * 9);
+  for (int t = threadIdx.x; t < cnt * NS; t += blockDim.x) {
+    const double* q = sQ + 9 * t;
+    const double ri = rcp_pos(q[0]);
+    sU[2 * t] = q[1] * ri;
+    sU[2 * t + 1] = q[2] * ri;
+  }
 #pragma unroll 1
   for (int fam = 0; fam < 2; fam++) {
     for (int t = threadIdx.x; t < cnt * N * NQ; t += blockDim.x) {
       const int k = t % NQ, el = t / NQ, e = el / N, ln = el - e * N;
       const bool fl = k < 8;
       // flux point r of line ln: family 1 at ln*(N+1) + r, family 2 at NF1 + r*N + ln
-      const int fp0 = fam ? NF1 + ln : ln * (N + 1), fps = fam ? N : 1;
-      const double* x = fl ? sF + (e * NFP + fp0) * 8 + k : sZ + (e * NFP + fp0) * 2 + (k - 8);
-      double y[N];
-      deriv_line<N, O>(x, fl ? fps * 8 : fps * 2, y);
-      // solution point i of line ln: family 1 at ln*N + i, family 2 at i*N + ln
-      const int p0 = e * NS + (fam ? ln : ln * N), ps = fam ? N : 1;
-      double* out = fl ? sR + p0 * 9 + k : sN + p0 * 2 + (k - 8);
-      const int os = fl ? ps * 9 : ps * 2;
+      const int fp0 = e * NFP + (fam ? NF1 + ln : ln * (N + 1)), fps = fam ? N : 1;
+      double* base = fl ? sF + k : sZ + (k - 8);
+      const int w = fl ? 8 : 2;
+      double v[N + 1];
+#pragma unroll
+      for (int r = 0; r <= N; r++) v[r] = base[(fp0 + r * fps) * w];
+      const uint32_t am = fix_amax(v);
+      const bool ok = fix_line_ok(am) && am < kIxHigh;
+      const int emax = max((int)(am >> 20), kFixEmaxMin), kv = ok ? emax - 1022 - O::ops().MS : kE3Fp64;
+      auto fp64_row = [&](int i) {
+        double a = 0.0;
+#pragma unroll
+        for (int r = 0; r <= N; r++) a += O::ops().M[r + (N + 1) * i] * v[r];
+        return a;
+      };
       if (!fam) {
+        sK[t] = kv;
+        if (ok) {
+          fix_mirror_sums<N, N + 1, -1>(v, emax, O::ops().MH, O::ops().ML, [&](int i, int64_t V) {
+            base[(fp0 + i) * w] = __longlong_as_double(V);
+          });
+        } else {
 #pragma unroll
-        for (int i = 0; i < N; i++) out[i * os] = fl ? negate(y[i]) : y[i];  // the flux enters negated
+          for (int i = 0; i < N; i++) base[(fp0 + i) * w] = fp64_row(i);
+        }
       } else {
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-          const double a = (fl ? out[i * os] - y[i] : out[i * os] + y[i]) * sJ[p0 + i * ps];
-          out[i * os] = a;
-          if (!fl) s.nAs[((size_t)e0 * NS + p0 + i * ps) * 2 + (k - 8)] = a;
+        // row i is the solution point p = i N + ln
+        auto finish = [&](int i, int64_t V) {
+          const int p = i * N + ln, ps = e * NS + p, eJ = sE[ps], k0 = sK[(e * N + i) * NQ + k];
+          double* at = base + slot(e, p) * w;
+          const int64_t V0 = __double_as_longlong(*at);
+          double a;
+          if (ok && k0 != kE3Fp64 && eJ != kE3Fp64) {
+            const int K = max(k0, kv);
+            const int64_t sum = ix_shr(V0, K - k0 + O::ops().MV) + ix_shr(V, K - kv + O::ops().MV);
+            a = fix_round_v<true>(ix_mul(fl ? -sum : sum, ix_limbs(sJ[ps])), K + O::ops().MV + eJ + 63);
+          } else {
+            double j = s.invJ[(size_t)e0 * NS + ps];
+            if (PRE) j *= rk.cR;
+            a = e3_fp64(V0, k0, V, kv, fl ? negate(j) : j);
+          }
+          *at = a;
+          if (fl && (PRE || update)) {  // RK_S5P3 / FiveStageRk, but for the terms of earlier states
+            double* q = sQ + 9 * ps + k;
+            *q = PRE ? fma(rk.cQ, *q, a) : rk.cQ * *q + rk.cR * a;
+          }
+        };
+        if (ok) {
+          fix_mirror_sums<N, N + 1, -1>(v, emax, O::ops().MH, O::ops().ML, finish);
+        } else {
+#pragma unroll 1
+          for (int i = 0; i < N; i++) finish(i, __double_as_longlong(fp64_row(i)));
         }
       }
     }
     __syncthreads();
   }
-  // A_z advection (resid(9), compresid.f90:45-47) at every solution point
-  for (int t = threadIdx.x; t < cnt * NS; t += blockDim.x) {
-    const double* q = s.Q + ((size_t)e0 * NS + t) * 9;
-    const double ri = rcp_pos(q[0]);
-    const double ax = sN[2 * t] - s.B0y, ay = sN[2 * t + 1] + s.B0x;
-    sR[t * 9 + 8] = negate(q[1] * ri * ax + q[2] * ri * ay);
+  // an earlier state's values go where the cells' family-2 fluxes were (8 NF1 >= 9 NS)
+  static_assert(8 * (N + 1) * N >= 9 * N * N, "a cell's state fits its family-2 fluxes");
+  auto src_slot = [&](int e) { return sF + (e * NFP + NF1) * 8; };
+  if (update && rk.nsrc > 0) {
+    for (int i = threadIdx.x; i < cnt * NS * 9; i += blockDim.x) {
+      const int e = i / (NS * 9);
+      cp_async8(src_slot(e) + (i - e * NS * 9), rk.src[0] + (size_t)e0 * NS * 9 + i);
+    }
+    cp_async_commit();
   }
-  if (rk.diag) {
-    __syncthreads();
-    for (int t = threadIdx.x; t < cnt * NS; t += blockDim.x) {
-      const double* r = sR + t * 9;
-      double acc = 0.0;
+  // A_z advection (resid(9), compresid.f90:45-47) at every solution point
+  const bool b0 = s.B0x != 0.0 || s.B0y != 0.0;
+  for (int t = threadIdx.x; t < cnt * NS; t += blockDim.x) {
+    const int e = t / NS;
+    const double* z = sZ + 2 * slot(e, t - e * NS);
+    double ax = z[0], ay = z[1];
+    if (!PRE && rk.write_resid) {  // kept for download; the last evaluation of a step writes it
+      s.nAs[((size_t)e0 * NS + t) * 2] = ax;
+      s.nAs[((size_t)e0 * NS + t) * 2 + 1] = ay;
+    }
+    if (b0) {  // (with cR folded in, the background gradient takes it too)
+      ax -= PRE ? rk.cR * s.B0y : s.B0y;
+      ay += PRE ? rk.cR * s.B0x : s.B0x;
+    }
+    const double r = negate(sU[2 * t] * ax + sU[2 * t + 1] * ay);
+    sU[2 * t] = r;
+    if (PRE || update) {
+      double* q = sQ + 9 * t + 8;
+      *q = PRE ? fma(rk.cQ, *q, r) : rk.cQ * *q + rk.cR * r;
+    }
+  }
+  cp_async_wait();
+  __syncthreads();
+  const size_t g0 = (size_t)e0 * NS * 9;
+  const int n = cnt * NS * 9;
+  if (update) {
+    if (rk.nsrc == 0 && !rk.R0) {
+      block_copy_out(s.Q + g0, sQ, n);
+      if (rk.save_new) block_copy_out(rk.save_new + g0, sQ, n);
+    } else if (rk.nsrc == 1 && !rk.R0 && !rk.save_new) {
+      const double c0 = rk.c[0];
+#pragma unroll 4
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const int e = i / (NS * 9);
+        s.Q[g0 + i] = fma(c0, src_slot(e)[i - e * NS * 9], sQ[i]);
+      }
+    } else {
+      // the terms of earlier states, elementwise over the block's contiguous state
+#pragma unroll 4
+      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const size_t g = g0 + i;
+        const int e = i / (NS * 9);
+        double qn = sQ[i];
+        if (rk.nsrc > 0) qn += rk.c[0] * src_slot(e)[i - e * NS * 9];
 #pragma unroll
-      for (int k = 0; k < 9; k++) acc += r[k] * r[k];
+        for (int j = 1; j < 3; j++)
+          if (j < rk.nsrc) qn += rk.c[j] * rk.src[j][g];
+        if (rk.R0) qn += rk.cR0 * rk.R0[g];
+        s.Q[g] = qn;
+        if (rk.save_new) rk.save_new[g] = qn;
+      }
+    }
+  }
+  if (!PRE && (rk.write_resid || rk.save_R)) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      const int pt = i / 9, k = i - 9 * pt, e = pt / NS;
+      const double r = k < 8 ? sF[8 * slot(e, pt - e * NS) + k] : sU[2 * pt];
+      if (rk.write_resid) s.resid[g0 + i] = r;
+      if (rk.save_R) rk.save_R[g0 + i] = r;
+    }
+  }
+  if (!PRE && rk.diag) {
+    for (int t = threadIdx.x; t < cnt * NS; t += blockDim.x) {
+      const int e = t / NS;
+      const double* r = sF + 8 * slot(e, t - e * NS);
+      double acc = sU[2 * t] * sU[2 * t];
+#pragma unroll
+      for (int k = 0; k < 8; k++) acc += r[k] * r[k];
       sD[t] = acc;
     }
+    __syncthreads();
   }
-  __syncthreads();
-  // stage update, elementwise over the block's contiguous state (RK_S5P3 / FiveStageRk):
-  // a streaming loop whose few FP64 operations hide under its memory traffic (the
-  // integer form of fixdot.cuh measured slower here)
-  {
-    const size_t g0 = (size_t)e0 * NS * 9;
-    const int n = cnt * NS * 9;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const size_t g = g0 + i;
-      const double q = s.Q[g], r = sR[i];
-      if (rk.write_resid) s.resid[g] = r;
-      if (!update) continue;
-      double qn = rk.cQ * q + rk.cR * r;
-      for (int j = 0; j < rk.nsrc; j++) qn += rk.c[j] * rk.src[j][g];
-      if (rk.R0) qn += rk.cR0 * rk.R0[g];
-      s.Q[g] = qn;
-      if (rk.save_old) rk.save_old[g] = q;
-      if (rk.save_new) rk.save_new[g] = qn;
-      if (rk.save_R) rk.save_R[g] = r;
-    }
-  }
-  if (rk.diag) {
+  if (!PRE && rk.diag) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     for (int e = warp; e < cnt; e += nwarp) {
       double acc = 0.0;
@@ -987,14 +1142,17 @@ __device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int 
   }
 }
 
-template <int N>
-__global__ void __launch_bounds__(512, 2) k_e3(SolveDev s, RKStage rk, int epb, int update, int c0, int c1) {
+// registers per thread of the pass: the line sums spill at 64, more cost resident CTAs
+constexpr int e3_regs(int N) { return N == 5 ? 80 : 72; }
+
+template <int N, bool PRE>
+__global__ void __maxnreg__(e3_regs(N)) k_e3(const __grid_constant__ SolveDev s, const __grid_constant__ RKStage rk, int epb, int update, int c0, int c1) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
   const int e0 = c0 + blockIdx.x * epb;
   const int cnt = min(epb, c1 - e0);
   if (cnt <= 0) return;
-  e3_body<N, OpsTU>(s, e0, cnt, epb, rk, update, sm);
+  e3_body<N, OpsTU, PRE>(s, e0, cnt, epb, rk, update, sm);
 }
 
 // ---------------------------------------------------------------------------

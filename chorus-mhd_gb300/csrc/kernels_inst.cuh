@@ -20,9 +20,6 @@ inline size_t smem_e1(int epb) {
 inline size_t smem_e2(int epb) {
   return sizeof(double) * ((size_t)epb * (D<kN>::NFP * 16 + D<kN>::NS * 17));
 }
-inline size_t smem_e3(int epb) {
-  return sizeof(double) * ((size_t)epb * (D<kN>::NFP * 8 + D<kN>::NS * (1 + 9 + 1 + 2) + D<kN>::NFP * 2));
-}
 inline size_t smem_ct(int epb) { return sizeof(double) * epb * (D<kN>::NFP * 2 + D<kN>::NS * 2); }
 inline int grid_cells(int nc, int epb) { return (nc + epb - 1) / epb; }
 
@@ -51,7 +48,8 @@ void set_smem_limits() {
   cudaFuncSetAttribute(k_e1<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_e2<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_f1<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_e3<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(k_e3<kN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(k_e3<kN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_ct_elem<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_diag_interp<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_nqsp<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
@@ -110,7 +108,7 @@ void launch_e3<kN>(const SolveDev& s, const RKStage& rk, const Launch& L, cudaSt
   const int update = (rk.cQ != 0.0 || rk.cR != 0.0 || rk.nsrc > 0) ? 1 : 0;
   if (c1 < 0) c1 = s.NC;
   if (c1 > c0)
-    launch_pdl(k_e3<kN>, grid_cells(c1 - c0, L.epb), L.threads, smem_e3(L.epb), st, s, rk, L.epb, update, c0, c1);
+    launch_pdl(e3_pre(rk, update) ? k_e3<kN, true> : k_e3<kN, false>, grid_cells(c1 - c0, L.epb), L.threads, e3_smem(kN, L.epb), st, s, rk, L.epb, update, c0, c1);
 }
 template <>
 void launch_ct<kN>(const SolveDev& s, const Launch& L, cudaStream_t st, int mode, int c0, int c1) {
