@@ -93,7 +93,7 @@ __device__ __forceinline__ void for_tiles(const BatchDev& b, int g, const int4* 
 // body, running the same per-N bodies as the single-solve kernels (so a solve gives the
 // same bits alone and in a batch).
 template <int N>
-__global__ void __launch_bounds__(512, 2) kg_e1(BatchDev b, int sensor_on) {
+__global__ void __maxnreg__(e1_regs(N)) kg_e1(BatchDev b, int sensor_on) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
   for_tiles(b, gidx(PE1, N), b.ctiles, [&](const int4& T, const SolveDev& s) {
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(512) kg_e2(BatchDev b, int epb) {
 }
 
 template <int N>
-__global__ void __launch_bounds__(512, 2) kg_e3(BatchDev b, int stage) {
+__global__ void __maxnreg__(e3_regs(N)) kg_e3(BatchDev b, int stage) {
   extern __shared__ __align__(16) double sm[];
   __shared__ __align__(16) RKStage srk;
   pdl_wait();

@@ -336,7 +336,7 @@ FIX_HD void fix_mirror_sums(const double (&v)[NI], int emax, const int* ch, cons
 
 template <int NO, int NI, int SIGMA, bool CHECK>
 FIX_HD void fix_mirror_line(const double (&v)[NI], int emax, const int* ch, const int* cl, int k, double (&y)[NO]) {
-  fix_mirror_sums<NO, NI, SIGMA>(v, emax, ch, cl, [&](int r, int64_t V) { y[r] = fix_round_v<CHECK>(V, k); });
+  fix_mirror_sums<NO, NI, SIGMA>(v, emax, ch, cl, [&](int r, int64_t V) { y[r] = r < NO / 2 ? fix_cvt_v<CHECK>(V, k) : fix_round_v<CHECK>(V, k); });
 }
 
 // the same for any finite line with emax <= kFixEmaxFast: lines below kFixEmaxMin are scaled

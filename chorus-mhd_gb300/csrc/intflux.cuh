@@ -198,6 +198,97 @@ FIX_HD int64_t ix_prod(Limbs a, Limbs b) {
   return p.value2();
 }
 
+// Contravariant ideal-MHD flux F sx + G sy (iflux_contra); q(k) reads variable k, out(j, a, b)
+// takes components 2 j and 2 j + 1.  Returns false, without output, where the integer form does
+// not apply.  [b] in the comments means a magnitude below 2^b.
+template <class Q, class Out>
+FIX_HD bool iflux_int(Q&& q, double sx, double sy, const IxGas& gas, Out&& out) {
+  const uint32_t zero = 66u << 20;  // a group of zeros: zeros are shifted out at this exponent
+  const uint32_t r = (uint32_t)(fix_bits(q(0)) >> 32), me = ix_abs_word(q(4));  // r: huge if the sign is set
+  const uint32_t mm = ix_max(zero, ix_max(ix_abs_word(q(1)), ix_abs_word(q(2)))), mz = ix_max(zero, ix_abs_word(q(3)));
+  const uint32_t mb = ix_max(zero, ix_max(ix_abs_word(q(5)), ix_abs_word(q(6)))), mw = ix_max(zero, ix_abs_word(q(7)));
+  const uint32_t ms = ix_max(ix_abs_word(sx), ix_abs_word(sy));
+  const uint32_t top = ix_max(ix_max(ix_max(r, me), ix_max(mm, mz)), ix_max(ix_max(mb, mw), ms));
+  if (top >= kIxHigh || r < kIxLow || me < kIxLow || ms < kIxLow) return false;
+  const int em = ix_exp<4>(mm), emz = ix_exp<4>(mz), eB = ix_exp<4>(mb), eBz = ix_exp<4>(mw), eE = ix_exp<3>(me);
+  const int eS = ix_exp<4>(ms), e_ri = -122 - ix_exp<2>(r);
+  const bool hasz = ix_max(mz, mw) != zero;
+  const Limbs nx = ix_limbs(ix_align<4>(sx, ms)), ny = ix_limbs(ix_align<4>(sy, ms));         // [60]
+  const Limbs mx = ix_limbs(ix_align<4>(q(1), mm)), my = ix_limbs(ix_align<4>(q(2), mm));     // [60]
+  const int64_t vby = ix_align<4>(q(6), mb);
+  const Limbs bx = ix_limbs(ix_align<4>(q(5), mb)), by = ix_limbs(vby);
+  const Limbs ri = ix_limbs(ix_rcp(ix_align<2>(q(0), r)));  // [61]
+  // mass flux, normal velocity
+  IxSum f;
+  f.add(mx, nx); f.add(my, ny);
+  const int64_t f0 = f.value4();  // [60.5]
+  const int eF0 = em + eS + 60;
+  const double F0 = ix_double(f0, eF0);
+  int64_t v = ix_mul(f0, ri);
+  const int nV = ix_room(v, 3), eV = eF0 + e_ri + 62 - nV;  // (slow flows keep their bits)
+  const Limbs V = ix_limbs(ix_shl(v, nV));                  // [60]
+  // v Bx - u By
+  IxSum w;
+  w.add(my, bx); w.add(mx, ix_limbs(-vby));
+  const Limbs W = ix_limbs(ix_mul(w.value4(), ri));
+  const int eW = em + eB + 60 + e_ri + 62;
+  // normal field, also over rho
+  IxSum b;
+  b.add(bx, nx); b.add(by, ny);
+  const int64_t bn = b.value4();  // [60.5]
+  const Limbs Bn = ix_limbs(bn), bnl = ix_limbs(ix_mul(bn, ri));
+  const int eBn = eB + eS + 60, ebn = eBn + e_ri + 62;
+  IxSum k2, b2, mB;
+  k2.square(mx); k2.square(my);
+  b2.square(bx); b2.square(by);
+  mB.add(mx, bx); mB.add(my, by);
+  int64_t kv = k2.value4_squares(), bv = b2.value4_squares(), mBv = mB.value4();  // [61]
+  int ek = 2 * em + 60, eB2 = 2 * eB + 60, emB = em + eB + 60;
+  double F3 = 0.0, F7 = 0.0;
+  if (hasz) {  // the z squares and products align with those of the plane
+    const int km = ix_max(em, emz), kb = ix_max(eB, eBz), kc = ix_max(em + eB, emz + eBz);
+    const Limbs mzl = ix_limbs(ix_align<4>(q(3), mz)), bzl = ix_limbs(ix_align<4>(q(7), mw));
+    IxSum kz, bz, mbz;
+    kz.square(mzl); bz.square(bzl); mbz.add(mzl, bzl);
+    kv = ix_shr(kv, 2 * (km - em)) + ix_shr(kz.value4_squares(), 2 * (km - emz));  // [61.6]
+    bv = ix_shr(bv, 2 * (kb - eB)) + ix_shr(bz.value4_squares(), 2 * (kb - eBz));
+    mBv = ix_shr(mBv, kc - em - eB) + ix_shr(mbz.value4(), kc - emz - eBz);
+    ek = 2 * km + 60;
+    eB2 = 2 * kb + 60;
+    emB = kc + 60;
+    const int ea = emz + eV + 61, eb = eBz + eBn + 61, K3 = ix_max(ea, eb);
+    F3 = ix_double(ix_shr(ix_prod(mzl, V), K3 - ea) - ix_shr(ix_prod(bzl, Bn), K3 - eb), K3);
+    const int ec = eBz + eV + 61, ed = emz + ebn + 61, K7 = ix_max(ec, ed);
+    F7 = ix_double(ix_shr(ix_prod(bzl, V), K7 - ec) - ix_shr(ix_prod(mzl, bnl), K7 - ed), K7);
+  }
+  // pressure and total pressure
+  ek += e_ri + 62;
+  const int KS = ix_max(ix_max(eE + 1, ek), eB2);
+  const int ep = KS + gas.eg + 62, ept = ix_max(ep, eB2 - 1);
+  const int64_t E = ix_align<3>(q(4), me);  // [61]
+  const int64_t S = ix_shr(E, KS - eE - 1) - ix_shr(ix_mul(kv, ri), KS - ek) - ix_shr(bv, KS - eB2);
+  if (S < 0) return false;
+  const int64_t pt = ix_shr(ix_mul(S, gas.g), ept - ep) + ix_shr(bv, ept - eB2 + 1);  // [62.3]
+  {
+    const int64_t ps = pt >> 1;
+    const int np = ix_room(ps, 2), epn = ept + 1 - np + eS + 61;
+    const Limbs P = ix_limbs(ix_shl(ps, np));  // [61.3]
+    const int ea = em + eV + 61, eb = eB + eBn + 61, K = ix_max(ix_max(ea, eb), epn) + 1;
+    const double F1 = ix_double(ix_shr(ix_prod(mx, V), K - ea) - ix_shr(ix_prod(bx, Bn), K - eb) + ix_shr(ix_prod(P, nx), K - epn), K);
+    out(0, F0, F1);
+    const double F2 = ix_double(ix_shr(ix_prod(my, V), K - ea) - ix_shr(ix_prod(by, Bn), K - eb) + ix_shr(ix_prod(P, ny), K - epn), K);
+    out(1, F2, F3);
+  }
+  {
+    const int eEp = eE + gas.eh, ea = eEp + eV + 61, eb = emB + ebn + 61, K = ix_max(ea, eb);
+    const Limbs Ep = ix_limbs(ix_shr(E, gas.eh) + ix_shift(pt, eEp - ept));  // [61.7]
+    const double F4 = ix_double(ix_shr(ix_prod(Ep, V), K - ea) - ix_shr(ix_prod(ix_limbs(mBv), bnl), K - eb), K);
+    out(2, F4, ix_double(ix_prod(W, ny), eW + eS + 61));
+    out(3, ix_double(-ix_prod(W, nx), eW + eS + 61), F7);
+  }
+  return true;
+}
+
 // Rusanov flux along the unit normal (ux, uy) times `scale` (rusanov_core): Fh = scale
 // (Fl + Fr - eigv (qr - ql)).  q(side, k) reads variable k of the left (0) or right (1)
 // state, out(j, a, b) takes components 2 j and 2 j + 1.  Returns false, without output, where

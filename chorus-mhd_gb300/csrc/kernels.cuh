@@ -289,6 +289,15 @@ __device__ __forceinline__ void deriv_line(const double* x, int xs, double (&y)[
   }
 }
 
+// the FP64 form of an interior point's flux, in the place of its state, for the states that the
+// integer form leaves out: a call, so that it takes no registers from the other points
+static __device__ __noinline__ void iflux_fp64(double* q, double sx, double sy, double gam) {
+  double F[8];
+  iflux_contra(q, sx, sy, gam - 1.0, F);
+#pragma unroll
+  for (int k = 0; k < 8; k++) q[k] = F[k];
+}
+
 template <int N, class O>
 __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int epb, int sensor, double* sm) {
   constexpr int NS = D<N>::NS, NF1 = D<N>::NF1, NFP = D<N>::NFP, NINT = 2 * N * (N - 1);
@@ -322,24 +331,34 @@ __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int 
     for (int f = 0; f <= N; f++) ob[f * os] = y[f];
   }
   __syncthreads();
+  // the flux-point values go out before the fluxes take their place
+  block_copy(s.Qvf + (size_t)e0 * NFP * 9, sV, cnt * NFP * 9);
+  __syncthreads();
   // contravariant inviscid flux at the interior flux points only (face points of Fc and
-  // Azf belong to the face pass), written straight out: consecutive threads take
-  // consecutive interior points, whose 64-byte flux records mostly adjoin
-  const double gm1 = s.gam - 1.0;
+  // Azf belong to the face pass), one point per thread, in the place of the point's state
+  // 512x512 cells, N = 5 (GB300): the pass took 1.14 ms a stage with 40 FP64 operations a point
+  // (84% of that pipe), 0.84 ms with some 700 integer instructions (issue slots 66% busy, the
+  // FP64 pipe 34% with the sensor).  A quarter of the points left in FP64 form beside them:
+  // 0.92 ms (part-filled warps in two loops).  64 registers (32 warps per SM): 0.95 ms at 80,
+  // 1.06 at 96 without the spill of 28 bytes.
   for (int t = threadIdx.x; t < cnt * NINT; t += blockDim.x) {
     const int e = t / NINT, fp = interior_fp<N>(t - e * NINT);
-    const double* qf = sV + (e * NFP + fp) * 9;
-    const size_t g = (size_t)(e0 + e) * NFP + fp;
-    const double2 m = reinterpret_cast<const double2*>(s.met)[g];  // 16-byte metric pair
-    double F[8];
-    iflux_contra(qf, m.x, m.y, gm1, F);
-    double2* fo = reinterpret_cast<double2*>(s.Fc + g * 8);  // 64-byte flux record
-#pragma unroll
-    for (int k = 0; k < 4; k++) fo[k] = make_double2(F[2 * k], F[2 * k + 1]);
-    s.Azf[g] = qf[8];
+    volatile double* q = sV + (e * NFP + fp) * 9;
+    const double2 m = reinterpret_cast<const double2*>(s.met)[(size_t)(e0 + e) * NFP + fp];  // 16-byte metric pair
+    auto put = [&](int j, double a, double b) {
+      q[2 * j] = a;
+      q[2 * j + 1] = b;
+    };
+    if (!iflux_int([&](int k) { return q[k]; }, m.x, m.y, s.gas, put)) iflux_fp64(sV + (e * NFP + fp) * 9, m.x, m.y, s.gam);
   }
-  {
-    block_copy(s.Qvf + (size_t)e0 * NFP * 9, sV, cnt * NFP * 9);
+  __syncthreads();
+  // the flux records, four threads to a record: consecutive points of a line adjoin
+  for (int t = threadIdx.x; t < cnt * NINT * 4; t += blockDim.x) {
+    const int i = t >> 2, j = t & 3, e = i / NINT, fp = interior_fp<N>(i - e * NINT);
+    const double* F = sV + (e * NFP + fp) * 9;
+    const size_t g = (size_t)(e0 + e) * NFP + fp;
+    reinterpret_cast<double2*>(s.Fc + g * 8)[j] = make_double2(F[2 * j], F[2 * j + 1]);
+    if (j == 0) s.Azf[g] = F[8];
   }
   if (!sensor) {
     if (s.skip)
@@ -417,9 +436,12 @@ __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int 
   }
 }
 
+// registers per thread of the pass (101x90 cells, N = 8: 98 us at 64, 94 us at 80)
+constexpr int e1_regs(int N) { return N > 6 ? 80 : 64; }
+
 // cells [c0, c1) of the solve, epb per CTA
 template <int N>
-__global__ void __launch_bounds__(512, 2) k_e1(SolveDev s, int epb, int sensor, int c0, int c1) {
+__global__ void __maxnreg__(e1_regs(N)) k_e1(const __grid_constant__ SolveDev s, int epb, int sensor, int c0, int c1) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
   // bit 4: the first pass of a stage, which starts the stage's wave-speed maximum

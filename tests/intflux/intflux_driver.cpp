@@ -28,10 +28,8 @@ int main(int argc, char** argv) {
     };
     if (kind == 0)
       o[0] = rusanov_int([&](int side, int k) { return a[8 * side + k]; }, a[16], a[17], ix_gas(a[19]), a[18], o[9], put);
-#ifdef INTFLUX_INTERIOR
     else
       o[0] = iflux_int([&](int k) { return a[k]; }, a[8], a[9], ix_gas(a[10]), put);
-#endif
   }
   FILE* g = std::fopen(argv[2], "wb");
   if (!g) return 2;

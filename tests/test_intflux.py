@@ -136,6 +136,25 @@ def test_rusanov_against_extended_precision(driver, tmp_path, kind, axis):
     assert np.all(out[:, 1:9][zero] == 0)  # what is exactly zero stays so
 
 
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("axis", [False, True], ids=["any metric", "axis metric"])
+def test_interior_flux_against_extended_precision(driver, tmp_path, kind, axis):
+    rng = np.random.default_rng(50 + len(kind) + 100 * axis)
+    n, gam = 2000, 5.0 / 3
+    q = states(rng, kind, n)
+    th = rng.integers(0, 4, n) * (np.pi / 2) if axis else rng.uniform(0, 2 * np.pi, n)
+    S = np.stack([np.cos(th), np.sin(th)], 1)
+    S = (np.rint(S) if axis else S) * np.exp(rng.uniform(-8, 8, (n, 1)))
+    out = evaluate(driver, tmp_path, 1, np.concatenate([q, S, np.full((n, 1), gam)], 1))
+    assert np.all(out[:, 0] == 1)
+    F, _, _, scale = physics(q.astype(LD), S.astype(LD), LD(gam))
+    assert np.all(abs(out[:, 1:] - F) <= 2.0 ** -52 * scale)
+    if kind in ("planar", "hydro"):
+        assert np.all(out[:, 8] == 0)  # what is exactly zero stays so
+    if kind == "hydro":
+        assert np.all(out[:, 6:8] == 0)
+
+
 def test_states_outside_the_integer_form_are_refused(driver, tmp_path):
     """Non-finite values, densities that are not positive or not normal, a density ratio above 16,
     scales beyond the window: left to the FP64 form."""
@@ -152,4 +171,9 @@ def test_states_outside_the_integer_form_are_refused(driver, tmp_path):
     cold[4] *= 0.01  # negative pressure on one side
     bad.append(cold)
     out = evaluate(driver, tmp_path, 0, np.array([good] + bad))
+    assert out[0, 0] == 1 and np.all(out[1:, 0] == 0)
+    # the same states at an interior point, without the density ratio and with the metric's bounds
+    inner = [[*r[:8], *r[16:18], r[19]] for r in bad if r[0] != 20 * good[0] and r[18] == 1.0]
+    inner += [[*good[:8], v, v, good[19]] for v in (0.0, 1e-100, 1e100, np.nan)]
+    out = evaluate(driver, tmp_path, 1, np.array([[*good[:8], 0.6, 0.8, good[19]]] + inner))
     assert out[0, 0] == 1 and np.all(out[1:, 0] == 0)
