@@ -39,7 +39,7 @@ void upload_ops_all(int N, const OpsN& o) {
 }
 
 // passes of a step, in the order of the tile tables
-enum { PE1 = 0, PF1, PE2, PE3, PCT, PCTF, kPasses };
+enum { PE1 = 0, PF1, PE2, PV, PE3, PCT, PCTF, kPasses };
 constexpr int kGroups = kPasses * (kMaxN + 1);
 __host__ __device__ constexpr int gidx(int pass, int N) { return pass * (kMaxN + 1) + N; }
 
@@ -97,7 +97,10 @@ __global__ void __maxnreg__(e1_regs(N)) kg_e1(BatchDev b, int sensor_on) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
   for_tiles(b, gidx(PE1, N), b.ctiles, [&](const int4& T, const SolveDev& s) {
-    if (T.y == 0 && threadIdx.x == 0) *s.eig = 0ull;  // the solve's stage starts its wave-speed maximum
+    if (T.y == 0 && threadIdx.x == 0) {  // the solve's stage starts its wave-speed maximum and list
+      *s.eig = 0ull;
+      *s.vcount = 0;
+    }
     // 1: variable-1 sensor; 3: also variable 6 when the solve's plot flag is set
     const int sensor = s.artiv ? ((sensor_on & 2) && !*s.plot_flag ? 1 : sensor_on) : 0;
     e1_body<N, OpsAll<N>>(s, T.y, T.z, T.z, sensor, sm);
@@ -115,14 +118,23 @@ __global__ void __launch_bounds__(kF1Threads, 2) kg_f1(BatchDev b) {
   });
 }
 
-// E2 tiles are chunks of up to blockDim.x cells, compacted to the cells that need
-// gradients and run in groups of epb (as k_e2)
+// E2 and V tiles are (slot, number of the tile, tiles of the solve): a tile walks the solve's
+// cells or list (as k_e2, k_v)
 template <int N>
-__global__ void __launch_bounds__(512) kg_e2(BatchDev b, int epb) {
+__global__ void __launch_bounds__(512) kg_e2(BatchDev b, int epb, int keep) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
   for_tiles(b, gidx(PE2, N), b.ctiles, [&](const int4& T, const SolveDev& s) {
-    e2_chunk<N, OpsAll<N>>(s, T.y, T.z, epb, sm);
+    e2_all<N, OpsAll<N>>(s, T.y, T.z, epb, keep, sm);
+  });
+}
+
+template <int N>
+__global__ void __launch_bounds__(v_threads(N)) kg_v(BatchDev b, int keep) {
+  extern __shared__ __align__(16) double sm[];
+  pdl_wait();
+  for_tiles(b, gidx(PV, N), b.ctiles, [&](const int4& T, const SolveDev& s) {
+    v_all<N, OpsAll<N>>(s, T.y, T.z, keep ? s.Ft : s.Fc, sm);
   });
 }
 
@@ -134,8 +146,8 @@ __global__ void __maxnreg__(e3_regs(N)) kg_e3(BatchDev b, int stage) {
   for_tiles(b, gidx(PE3, N), b.ctiles, [&](const int4& T, const SolveDev& s) {
     if (threadIdx.x == 0) srk = b.rk[stage * b.cap + T.x];
     __syncthreads();
-    if (e3_pre(srk, 1)) e3_body<N, OpsAll<N>, true>(s, T.y, T.z, T.z, srk, 1, sm);
-    else e3_body<N, OpsAll<N>, false>(s, T.y, T.z, T.z, srk, 1, sm);
+    if (e3_pre(srk, 1)) e3_body<N, OpsAll<N>, true>(s, T.y, T.z, T.z, srk, 1, e3_visc(s, false), sm);
+    else e3_body<N, OpsAll<N>, false>(s, T.y, T.z, T.z, srk, 1, e3_visc(s, srk.write_resid), sm);
   });
 }
 
@@ -162,7 +174,7 @@ size_t cell_smem_bytes(int N, int epb, int pass) {
   size_t d = 0;
   switch (pass) {
     case 0: d = (size_t)epb * (NS * 9 + 2 * NS + NFP * 9) + N * N; break;
-    case 1: d = (size_t)epb * (NFP * 16 + NS * 17); break;
+    case 1: return e2_smem(N, epb);
     case 2: return e3_smem(N, epb);
     default: d = (size_t)epb * (NFP * 2 + NS * 2); break;
   }
@@ -184,11 +196,12 @@ static void pass_shapes(int nsm, const int (&epb)[4], const int (&threads)[4], P
   cudaFuncSetAttribute(kg_e1<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_f1<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_e2<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(kg_v<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_e3<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_ct<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   // every pass kernel asks for the same shared-memory carveout, so that CTAs of the
   // concurrent order chains share an SM without reconfiguring it
-  const void* fns[6] = {(const void*)kg_e1<N>, (const void*)kg_f1<N>, (const void*)kg_e2<N>,
+  const void* fns[7] = {(const void*)kg_e1<N>, (const void*)kg_f1<N>, (const void*)kg_e2<N>, (const void*)kg_v<N>,
                         (const void*)kg_e3<N>, (const void*)kg_ct<N>, (const void*)kg_ctface<N>};
   for (const void* f : fns)
     cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
@@ -203,6 +216,7 @@ static void pass_shapes(int nsm, const int (&epb)[4], const int (&threads)[4], P
   fill(sh[PE1], (const void*)kg_e1<N>, threads[0], epb[0], cell_smem_bytes(N, epb[0], 0));
   fill(sh[PF1], (const void*)kg_f1<N>, kF1Threads, 0, f1_smem(kF1Threads));
   fill(sh[PE2], (const void*)kg_e2<N>, threads[1], epb[1], cell_smem_bytes(N, epb[1], 1));
+  fill(sh[PV], (const void*)kg_v<N>, v_threads(N), v_epb(N), v_smem(N));
   fill(sh[PE3], (const void*)kg_e3<N>, threads[2], epb[2], cell_smem_bytes(N, epb[2], 2));
   fill(sh[PCT], (const void*)kg_ct<N>, threads[3], epb[3], cell_smem_bytes(N, epb[3], 3));
   fill(sh[PCTF], (const void*)kg_ctface<N>, 256, 0, 0);
@@ -213,7 +227,8 @@ static void launch_pass(const BatchDev& a, int pass, const PassShape& p, cudaStr
   switch (pass) {
     case PE1: launch_pdl(kg_e1<N>, p.grid, p.threads, p.smem, st, a, arg); break;
     case PF1: launch_pdl(kg_f1<N>, p.grid, p.threads, p.smem, st, a); break;
-    case PE2: launch_pdl(kg_e2<N>, p.grid, p.threads, p.smem, st, a, p.epb); break;
+    case PE2: launch_pdl(kg_e2<N>, p.grid, p.threads, p.smem, st, a, p.epb, arg); break;
+    case PV: launch_pdl(kg_v<N>, p.grid, p.threads, p.smem, st, a, arg); break;
     case PE3: launch_pdl(kg_e3<N>, p.grid, p.threads, p.smem, st, a, arg); break;
     case PCT: launch_pdl(kg_ct<N>, p.grid, p.threads, p.smem, st, a, arg); break;
     default: launch_pdl(kg_ctface<N>, p.grid, p.threads, 0, st, a); break;
@@ -341,9 +356,6 @@ static int batch_rebuild(ChorusBatch* b) {
   std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return b->slots[a].NC > b->slots[c].NC; });
   std::vector<int4> grp[kGroups];
   unsigned orders = 0;
-  // E2 chunks as the single-solve launch sizes them: up to one cell per thread, but small
-  // enough for about 16 CTAs per SM over all the order's cells, so that small solves whose
-  // cells all need gradients spread over the GPU
   long long order_cells[kMaxN + 1] = {0};
   for (int i : order) order_cells[b->slots[i].N] += b->slots[i].NC;
   for (int i : order) {
@@ -356,11 +368,16 @@ static int batch_rebuild(ChorusBatch* b) {
     };
     cut(PE1, sl.NC, o.epb[0]);
     cut(PF1, sl.nfp_faces, kFluxTile);
-    long long chunk = order_cells[sl.N] / (16LL * b->nsm);
-    chunk = std::max<long long>(o.epb[1], std::min<long long>(chunk, o.threads[1]));
-    chunk -= chunk % o.epb[1];
-    if (!sl.sd.skip) chunk = o.epb[1];
-    cut(PE2, sl.NC, (int)std::max<long long>(chunk, 1));
+    // a tile per group where every cell has work, else as many as would share the GPU with the
+    // order's other solves at about eight CTAs per SM
+    auto walk = [&](int pass, int group) {
+      const long long all = (sl.NC + group - 1) / group;
+      const long long part = std::max<long long>(1, 8LL * b->nsm * sl.NC / std::max<long long>(1, order_cells[sl.N]));
+      const int n = (int)(sl.sd.skip ? std::min(all, part) : all);
+      for (int k = 0; k < n; k++) grp[gidx(pass, sl.N)].push_back(make_int4(i, k, n, 0));
+    };
+    walk(PE2, o.epb[1]);
+    if (v_pass(sl.sd) && (sl.sd.artiv || !sl.sd.skip)) walk(PV, o.pass[PV].epb);
     cut(PE3, sl.NC, o.epb[2]);
     cut(PCT, sl.NC, o.epb[3]);
     cut(PCTF, sl.nfp_two, kFaceTile);
@@ -462,7 +479,8 @@ static void batch_enqueue_step(ChorusBatch* b) {
     for (int stage = 0; stage < 5; stage++) {
       pass(PE1, stage == 4 ? 3 : 1);
       pass(PF1, 0);
-      pass(PE2, 0);  // also the face AV viscosities
+      pass(PE2, stage == 4 ? 1 : 0);
+      pass(PV, stage == 4 ? 1 : 0);
       pass(PE3, stage);
     }
     pass(PCT, 0);

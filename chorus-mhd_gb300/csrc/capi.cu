@@ -130,7 +130,7 @@ struct Dispatch {
   void (*e1)(const SolveDev&, const Launch&, cudaStream_t, int, int, int);
   void (*e1ns)(const SolveDev&, const Launch&, cudaStream_t);
   void (*f1)(const SolveDev&, cudaStream_t, int, int, int, int);
-  void (*e2)(const SolveDev&, const Launch&, cudaStream_t);
+  void (*e2)(const SolveDev&, const Launch&, cudaStream_t, bool);
   void (*f2)(const SolveDev&, cudaStream_t);
   void (*qavg)(const SolveDev&, cudaStream_t);
   void (*e3)(const SolveDev&, const RKStage&, const Launch&, cudaStream_t, int, int);
@@ -294,7 +294,8 @@ static size_t arena_plan_bytes(int N, int NC, int nface2, int nface1, int k_stag
   P.take<int4>(nface2 + 1); P.take<int2>(nface1 + 1); P.take<FaceNorm>((size_t)nface2 * N + 1);
   P.take<FaceNorm>((size_t)nface1 * N + 1); P.take<unsigned long long>(4); P.take<unsigned int>(4);
   P.take<double>(8); P.take<int>(NC); P.take<int>(NC); P.take<int4>(NC); P.take<int4>(NC);
-  P.take<double>((size_t)NC * NS * 2);
+  P.take<double>((size_t)NC * NS * 2); P.take<double>(NC); P.take<double>(nfp * 8);
+  P.take<int>(NC); P.take<int>(NC);
   return P.off;
 }
 
@@ -497,7 +498,8 @@ int chorus_gpu_bind(const ChorusDims* dims, const int32_t* IF2C, const int32_t* 
          ofn2 = P.take<FaceNorm>(fn2.size() + 1), ofn1 = P.take<FaceNorm>(fn1.size() + 1),
          oeig = P.take<unsigned long long>(4), oerr = P.take<unsigned int>(4), ored = P.take<double>(8),
          oact = P.take<int>(NC), onv = P.take<int>(NC), onbr = P.take<int4>(NC), onbrlf = P.take<int4>(NC),
-         onQs9 = P.take<double>((size_t)NC * NS * 2);
+         onQs9 = P.take<double>((size_t)NC * NS * 2), oSw = P.take<double>(NC), oFt = P.take<double>(nfp * 8),
+         ovl = P.take<int>(NC), ogr = P.take<int>(NC);
   c->arena_bytes = P.off;
   if (P.off != arena_plan_bytes(N, NC, c->nface2, c->nface1, params->k_stage))
     return fail(set_err(CHORUS_EINVAL, "internal: arena plan mismatch"));
@@ -546,11 +548,16 @@ int chorus_gpu_bind(const ChorusDims* dims, const int32_t* IF2C, const int32_t* 
   s.nbr = (const int4*)(A + onbr);
   s.nbrlf = (const int4*)(A + onbrlf);
   s.nQs9 = (double*)(A + onQs9);
+  s.Sw = (double*)(A + oSw);
+  s.Ft = (double*)(A + oFt);
+  s.vlist = (int*)(A + ovl);
+  s.gr = (int*)(A + ogr);
   c->skip_option = 1;
   s.skip = (params->mu == 0.0 && params->eta0 == 0.0) ? 1 : 0;
   s.eig = (unsigned long long*)(A + oeig);
   s.err = (unsigned int*)(A + oerr);
   s.plot_flag = (const int*)(s.err + 1);  // zeroed with the arena
+  s.vcount = (int*)(s.err + 2);
   c->red = (double*)(A + ored);
   if (cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->cp, cudaStreamNonBlocking) != cudaSuccess)
@@ -712,7 +719,7 @@ void enqueue_stage(ChorusCtx* c, const RKStage& rk, bool last) {
   c->D->e1(s, c->L[0], c->st, last ? 1 : 0, 0, -1);  // also zeroes the stage's wave speed
   c->qvf9_pending = false;
   c->D->f1(s, c->st, 0, -1, 0, -1);
-  c->D->e2(s, c->L[1], c->st);  // also the face AV viscosities
+  c->D->e2(s, c->L[1], c->st, rk.write_resid != 0);  // also the face AV viscosities
   c->D->e3(s, rk, c->L[2], c->st, 0, -1);  // averages the grad Q traces where it reads them
 }
 
@@ -885,12 +892,12 @@ void enqueue_step_host(ChorusCtx* c, bool diag, const double* Qin, double* Qout)
     c->D->e1(s, c->L[0], c->st, 0, 0, -1);
     c->D->f1(s, c->st, 0, -1, 0, -1);
   }
-  c->D->e2(s, c->L[1], c->st);
+  c->D->e2(s, c->L[1], c->st, false);
   c->D->e3(s, r[0], c->L[2], c->st, 0, -1);
   for (int k = 1; k < 4; k++) enqueue_stage(c, r[k], false);
   c->D->e1(s, c->L[0], c->st, 1, 0, -1);
   c->D->f1(s, c->st, 0, -1, 0, -1);
-  c->D->e2(s, c->L[1], c->st);
+  c->D->e2(s, c->L[1], c->st, true);
   if (Qout) {
     for (int k = 0; k < K; k++) {
       c->D->e3(s, r[4], c->L[2], c->st, h.cut[k], h.cut[k + 1]);
@@ -1161,7 +1168,8 @@ int64_t chorus_gpu_device_bytes(ChorusCtx* c) { return c ? (int64_t)c->arena_byt
 int chorus_gpu_launch_counts(ChorusCtx* c, int32_t* per_step, int32_t* per_diag) {
   if (!c) return set_err(CHORUS_EINVAL, "null context");
   const int nf = (c->nface2 + c->nface1) > 0 ? 1 : 0;
-  const int stage = 3 + nf;             // E1 E2 E3 (+ F1)
+  const int nv = v_pass(c->sd) && (c->sd.artiv || !c->sd.skip) ? 1 : 0;
+  const int stage = 3 + nf + nv;        // E1 E2 E3 (+ F1, V)
   const int ct = 2 + (c->nface2 > 0);   // element passes + face average
   if (per_step) *per_step = 5 * stage + ct;
   if (per_diag) *per_diag = 1 + (c->nface2 > 0) + 4;  // B traces, face average, nablaQsp, divB, reduce, record
@@ -1186,7 +1194,7 @@ int chorus_gpu_profile_stage(ChorusCtx* c, int32_t reps, double* ms) {
     CK(cudaEventRecord(ev[1], c->st));
     c->D->f1(s, c->st, 0, -1, 0, -1);
     CK(cudaEventRecord(ev[2], c->st));
-    c->D->e2(s, c->L[1], c->st);
+    c->D->e2(s, c->L[1], c->st, false);
     CK(cudaEventRecord(ev[3], c->st));
     CK(cudaEventRecord(ev[4], c->st));  // the former F2 pass lives in E2 and E3
     c->D->e3(s, r, c->L[2], c->st, 0, -1);

@@ -57,6 +57,7 @@ void initial_point(int problem, double gam, double x, double y, const double* B,
 //                            fp = family-1 points (jfp*(N+1)+ifp), then family-2
 //                            points ((N+1)N + jfp*N+ifp): one block per cell
 //   Fc         [e][fp][8]    inviscid contravariant flux (F1 / G2)
+//   Ft         [e][fp][8]    inviscid - viscous flux, of cells with a viscous flux
 //   Azf        [e][fp]       A_z at the flux points (upwinded on faces after a stage,
 //                            face-averaged after the CT projection)
 //   nQs        [e][js][is][2][9]   (variable 9 is not stored here: see nQs9)
@@ -66,6 +67,7 @@ void initial_point(int problem, double gam, double x, double y, const double* B,
 //   met        [e][fp][2]    (S1(1,1),S1(1,2)) on family 1, (S2(2,1),S2(2,2)) on 2
 //   invJ       [e][js][is]
 //   Se         [e]           AV sensor sum of variable 1 (the reference's SM_IND(1) is log10 of it)
+//   Sw         [e]           its ramp: muAV(1) = epsilon0 / 2 * Sw
 //   muf        [e][4]        face-averaged AV viscosity per local face 1..4
 // ---------------------------------------------------------------------------
 struct FaceNorm {  // per face point: unit normal, magnorm*sign_l/2, sign_l*sign_r (+-1)
@@ -87,6 +89,7 @@ struct SolveDev {
   double* resid;
   double* Qvf;
   double* Fc;
+  double* Ft;                   // total flux of the cells with a viscous flux (pass V)
   double* Azf;
   double* nQs;
   double* nQvf;
@@ -107,6 +110,9 @@ struct SolveDev {
   int pad1;
   int* act;
   int* nv;
+  int* vlist;                   // the cells with nv set, in the order F1 found them
+  int* vcount;                  // and their number
+  int* gr;                      // E2 has taken the cell
   const int4* nbr;
   const int4* nbrlf;            // the neighbour's local face (1..4) across each face, 0 at FREE faces
   unsigned long long* eig;      // bit pattern of the stage's max wave speed (>= 0)
@@ -115,6 +121,7 @@ struct SolveDev {
   const int* plot_flag;         // nonzero: the last stage records Se6 (read by E1 at run time)
   double* nQs9;                 // [e][sp][2] grad A_z of variable 9 (nablaQs(9,:,...)), kept apart from nQs
   IxGas gas;                    // gamma for the integer fluxes
+  double* Sw;                   // [e] the AV ramp of the sensor (av_ramp)
   void* pad3;                   // keeps the size a multiple of 16 bytes
 };
 
@@ -148,7 +155,9 @@ struct Launch {
 template <int N> void launch_e1(const SolveDev& s, const Launch& L, cudaStream_t st, int plot, int c0 = 0, int c1 = -1);
 // two-sided faces [a2, b2) and FREE faces [a1, b1) (b < 0: to the end of the list)
 template <int N> void launch_f1(const SolveDev& s, cudaStream_t st, int a2 = 0, int b2 = -1, int a1 = 0, int b1 = -1);
-template <int N> void launch_e2(const SolveDev& s, const Launch& L, cudaStream_t st);
+// keep: the evaluation whose arrays stay downloadable (the last stage of a step, a single
+// compresid): the inviscid fluxes are not replaced by total ones
+template <int N> void launch_e2(const SolveDev& s, const Launch& L, cudaStream_t st, bool keep);
 template <int N> void launch_f2(const SolveDev& s, cudaStream_t st);
 template <int N> void launch_qavg(const SolveDev& s, cudaStream_t st);
 template <int N> void launch_e3(const SolveDev& s, const RKStage& rk, const Launch& L, cudaStream_t st, int c0 = 0,

@@ -271,21 +271,11 @@ FIX_HD double fix_cvt_v(int64_t V, int k) {
 // over U or W alone < 4 2^60 + 2^59; |B| < 9 (2^58 + 2^58) + 2^28: all below 2^63.
 //
 // fix_mirror_sums hands out the sums V of the rows as they are formed, put(row, V): y =
-// V 2^(k-1) with k as in fix_dot, |V| at most the row's sum of |c|, below 2^62.2.
+// V 2^(k-1) with k as in fix_dot, |V| at most the row's sum of |c|, below 2^62.2;
+// fix_mirror_core the same from aligned integers X of exponent e: y = V 2^(e + 58 - S).
 template <int NO, int NI, int SIGMA, class Put>
-FIX_HD void fix_mirror_sums(const double (&v)[NI], int emax, const int* ch, const int* cl, Put&& put) {
+FIX_HD void fix_mirror_core(const int64_t (&X)[NI], const int* ch, const int* cl, Put&& put) {  // |X| < 2^58
   constexpr int NP = NI / 2;
-  int64_t X[NI];
-  const uint32_t eb = ((uint32_t)emax << 20) | 0xfffffu;
-#pragma unroll
-  for (int j = 0; j < NI; j++) {
-    const uint64_t u = fix_bits(v[j]);
-    const uint32_t a = (uint32_t)(u >> 32) & 0x7fffffffu;
-    const uint32_t d = (eb + (6u << 20) - a) >> 20;  // emax - exponent + 6
-    const uint64_t t = (u << 11) | 0x8000000000000000ull;
-    const int64_t x = (int64_t)fix_shru(t, (int)d);
-    X[j] = (int64_t)u < 0 ? -x : x;
-  }
   constexpr int64_t kHalfL = (int64_t)1 << (kFixSplit - 1);
   auto split = [](int64_t x, int& h, int& l) {  // x offset by half a limb
     h = (int)(x >> kFixSplit);
@@ -332,6 +322,22 @@ FIX_HD void fix_mirror_sums(const double (&v)[NI], int emax, const int* ch, cons
       put(NO - 1 - r, SIGMA > 0 ? V : -V);
     }
   }
+}
+
+template <int NO, int NI, int SIGMA, class Put>
+FIX_HD void fix_mirror_sums(const double (&v)[NI], int emax, const int* ch, const int* cl, Put&& put) {
+  int64_t X[NI];
+  const uint32_t eb = ((uint32_t)emax << 20) | 0xfffffu;
+#pragma unroll
+  for (int j = 0; j < NI; j++) {
+    const uint64_t u = fix_bits(v[j]);
+    const uint32_t a = (uint32_t)(u >> 32) & 0x7fffffffu;
+    const uint32_t d = (eb + (6u << 20) - a) >> 20;  // emax - exponent + 6
+    const uint64_t t = (u << 11) | 0x8000000000000000ull;
+    const int64_t x = (int64_t)fix_shru(t, (int)d);
+    X[j] = (int64_t)u < 0 ? -x : x;
+  }
+  fix_mirror_core<NO, NI, SIGMA>(X, ch, cl, put);
 }
 
 template <int NO, int NI, int SIGMA, bool CHECK>

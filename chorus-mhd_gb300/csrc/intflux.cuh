@@ -169,12 +169,27 @@ FIX_HD int ix_room(int64_t v, int keep) {
 #endif
 }
 
+// limbs of v shifted up to [60] where it is below that, with its exponent; and of a pair
+FIX_HD Limbs ix_up(int64_t v, int& e) {
+  const int n = ix_room(v, 3);
+  e -= n;
+  return ix_limbs(ix_shl(v, n));
+}
+FIX_HD void ix_up2(int64_t a, int64_t b, int& e, Limbs& la, Limbs& lb) {
+  const int n = ix_room((a ^ (a >> 63)) | (b ^ (b >> 63)), 3);
+  e -= n;
+  la = ix_limbs(ix_shl(a, n));
+  lb = ix_limbs(ix_shl(b, n));
+}
+
 // constants of a solve, prepared once (host or device): half of gamma - 1, gamma, as limbs
 // of normalised integers in [2^60, 2^61) with their exponents
 struct IxGas {
   Limbs g, gam;
   int eg, egam;
-  int eh, pad;  // E + p + B^2/2 <= (1 + gamma) E, as p >= 0 and B^2/2 <= E: below 2^(eh + 0.7) E
+  Limbs kap;  // gamma / Pr
+  int ekap;
+  int eh;  // E + p + B^2/2 <= (1 + gamma) E, as p >= 0 and B^2/2 <= E: below 2^(eh + 0.7) E
 };
 FIX_HD IxGas ix_gas(double gamma) {
   IxGas c;
@@ -183,7 +198,9 @@ FIX_HD IxGas ix_gas(double gamma) {
   c.eg = ix_exp<3>(ix_abs_word(gm));
   c.gam = ix_limbs(ix_align<3>(gamma, ix_abs_word(gamma)));
   c.egam = ix_exp<3>(ix_abs_word(gamma));
-  c.pad = 0;
+  const double kp = gamma / 0.72;
+  c.kap = ix_limbs(ix_align<3>(kp, ix_abs_word(kp)));
+  c.ekap = ix_exp<3>(ix_abs_word(kp));
   for (c.eh = 1; c.eh < 60 && 1.0 + gamma > 1.62 * (double)(1LL << c.eh); c.eh++) {
   }
   return c;
@@ -286,6 +303,167 @@ FIX_HD bool iflux_int(Q&& q, double sx, double sy, const IxGas& gas, Out&& out) 
     out(2, F4, ix_double(ix_prod(W, ny), eW + eS + 61));
     out(3, ix_double(-ix_prod(W, nx), eW + eS + 61), F7);
   }
+  return true;
+}
+
+// Contravariant viscous, resistive and artificial-viscosity flux (vflux_contra, whose formulas
+// these are): q(k) the state, g(d, k) its gradient, mut and eta the viscosity and resistivity.
+// out(k, value) takes components 1..7; false, without output, where the integer form does not
+// apply.  [b] in the comments means a magnitude below 2^b.
+template <class Q, class G, class Out>
+FIX_HD bool vflux_int(Q&& q, G&& g, double mut, double eta, double sx, double sy, const IxGas& gas, Out&& out) {
+  const uint32_t zero = 66u << 20;  // a group of zeros: zeros are shifted out at this exponent
+  auto w1 = [&](int k) { return ix_max(zero, ix_abs_word(q(k))); };
+  auto w2 = [&](int k) { return ix_max(zero, ix_max(ix_abs_word(g(0, k)), ix_abs_word(g(1, k)))); };
+  const uint32_t r = (uint32_t)(fix_bits(q(0)) >> 32);  // huge if the sign is set
+  const uint32_t mm = ix_max(w1(1), w1(2)), mz = w1(3), me = w1(4), mb = ix_max(w1(5), w1(6)), mw = w1(7);
+  const uint32_t gr = w2(0), gm = ix_max(w2(1), w2(2)), gz = w2(3), ge = w2(4), gb = ix_max(w2(5), w2(6)), gw = w2(7);
+  const uint32_t ms = ix_max(ix_abs_word(sx), ix_abs_word(sy));
+  const uint32_t mu = ix_max(zero, ix_abs_word(mut)), mt = ix_max(zero, ix_abs_word(eta));
+  const uint32_t top = ix_max(ix_max(ix_max(ix_max(r, mm), ix_max(mz, me)), ix_max(ix_max(mb, mw), ix_max(ms, mu))),
+                              ix_max(ix_max(ix_max(gr, gm), ix_max(gz, ge)), ix_max(ix_max(gb, gw), mt)));
+  if (top >= kIxHigh || r < kIxLow || ms < kIxLow) return false;
+  const bool hasz = ix_max(ix_max(mz, mw), ix_max(gz, gw)) != zero;
+  const int em = ix_exp<4>(mm), eB = ix_exp<4>(mb), eS = ix_exp<4>(ms), e_ri = -122 - ix_exp<2>(r);
+  const int egr = ix_exp<4>(gr), egm = ix_exp<4>(gm), egB = ix_exp<4>(gb);
+  const Limbs nx = ix_limbs(ix_align<4>(sx, ms)), ny = ix_limbs(ix_align<4>(sy, ms));  // [60]
+  const Limbs ri = ix_limbs(ix_rcp(ix_align<2>(q(0), r)));                             // [61]
+  int eM = ix_exp<3>(mu) + e_ri + 62;
+  const Limbs M = ix_up(ix_mul(ix_align<3>(mut, mu), ri), eM);                         // [60] mu / rho
+  auto contracted = [&](Limbs a, Limbs b) {  // a sx + b sy: [60.5], exponent of a + eS + 60
+    IxSum t;
+    t.add(a, nx); t.add(b, ny);
+    return t.value4();
+  };
+  // velocities, m^2 + ... of the internal energy: X = |u|^2 + B^2/(2 rho) - E/rho
+  const Limbs mx = ix_limbs(ix_align<4>(q(1), mm)), my = ix_limbs(ix_align<4>(q(2), mm));  // [60]
+  int eu = em + e_ri + 61;
+  Limbs u, v;  // [60]
+  ix_up2(ix_prod(mx, ri), ix_prod(my, ri), eu, u, v);
+  const Limbs bx = ix_limbs(ix_align<4>(q(5), mb)), by = ix_limbs(ix_align<4>(q(6), mb));
+  IxSum k2, b2;
+  k2.square(mx); k2.square(my);
+  b2.square(bx); b2.square(by);
+  int64_t kv = k2.value4_squares(), bv = b2.value4_squares();  // [61]
+  int ek = 2 * em + 60, eB2 = 2 * eB + 60;
+  Limbs w{0, 0}, bz{0, 0};
+  int ew = 0, eBz = 0;
+  if (hasz) {
+    const int emz = ix_exp<4>(mz);
+    eBz = ix_exp<4>(mw);
+    const int km = ix_max(em, emz), kb = ix_max(eB, eBz);
+    const Limbs mzl = ix_limbs(ix_align<4>(q(3), mz));
+    bz = ix_limbs(ix_align<4>(q(7), mw));
+    IxSum a, b;
+    a.square(mzl); b.square(bz);
+    kv = ix_shr(kv, 2 * (km - em)) + ix_shr(a.value4_squares(), 2 * (km - emz));  // [61.6]
+    bv = ix_shr(bv, 2 * (kb - eB)) + ix_shr(b.value4_squares(), 2 * (kb - eBz));
+    ek = 2 * km + 60;
+    eB2 = 2 * kb + 60;
+    ew = emz + e_ri + 61;
+    w = ix_up(ix_prod(mzl, ri), ew);
+  }
+  ek += e_ri + 62;
+  const int eE = ix_exp<3>(me), KY = ix_max(ix_max(ek, eB2 - 1), eE) + 1;
+  int eX = KY + e_ri + 62;
+  const Limbs X = ix_up(ix_mul(ix_shr(ix_mul(kv, ri), KY - ek) + ix_shr(bv, KY - eB2 + 1) - ix_shr(ix_align<3>(q(4), me), KY - eE), ri), eX);  // [60]
+  // gradients of the density, and rho times those of the plane's velocity
+  const Limbs rx = ix_limbs(ix_align<4>(g(0, 0), gr)), ry = ix_limbs(ix_align<4>(g(1, 0), gr));
+  int erS = egr + eS + 60;
+  const Limbs rS = ix_up(contracted(rx, ry), erS);  // [60]
+  const int ep = egr + eu + 61, Kw = ix_max(egm, ep) + 1;
+  Limbs c1, c2;
+  int64_t t2;  // u.(grad m . S) of the plane
+  int ec = Kw + eS + 61, e2 = egm + eS + 60;
+  {
+    const int64_t ax = ix_align<4>(g(0, 1), gm), ay = ix_align<4>(g(1, 1), gm);
+    const int64_t bx_ = ix_align<4>(g(0, 2), gm), by_ = ix_align<4>(g(1, 2), gm);
+    Limbs mxS, myS;
+    ix_up2(contracted(ix_limbs(ax), ix_limbs(ay)), contracted(ix_limbs(bx_), ix_limbs(by_)), e2, mxS, myS);
+    t2 = ix_prod(mxS, u) + ix_prod(myS, v);  // [60]
+    e2 += eu + 61;
+    auto rel = [&](int64_t a, Limbs r_, Limbs u_) { return ix_shr(a, Kw - egm) - ix_shr(ix_prod(r_, u_), Kw - ep); };  // [60]
+    const int64_t ux = rel(ax, rx, u), uy = rel(ay, ry, u), vx = rel(bx_, rx, v), vy = rel(by_, ry, v);
+    const Limbs two3{(int)(1537228672809129301LL >> 31), (int)(1537228672809129301LL & 0x7fffffff)};  // 2^62 / 3
+    const int64_t ld = ix_prod(ix_limbs(ux + vy), two3);  // 2/3 of the divergence: [60.5]
+    const Limbs a = ix_limbs(ux + ux - ld), b = ix_limbs(uy + vx), d = ix_limbs(vy + vy - ld);  // [61.7]
+    ix_up2(ix_prod(a, nx) + ix_prod(b, ny), ix_prod(b, nx) + ix_prod(d, ny), ec, c1, c2);  // [61.4], [60] if shifted
+  }
+  out(1, ix_double(ix_mul(c1, M), ec + eM + 62));
+  out(2, ix_double(ix_mul(c2, M), ec + eM + 62));
+  // energy: M (u.c + gamma/Pr H), H = grad E.S - u.(grad m.S) - B.(grad B.S) + X grad rho.S
+  const uint32_t gE = ge;
+  const int e1 = ix_exp<4>(gE) + eS + 60, e4 = eX + erS + 61;
+  int e3 = egB + eS + 60;
+  const int64_t t1 = contracted(ix_limbs(ix_align<4>(g(0, 4), gE)), ix_limbs(ix_align<4>(g(1, 4), gE)));
+  const int64_t yx = ix_align<4>(g(0, 6), gb), xy = ix_align<4>(g(1, 5), gb);
+  Limbs bxS, byS;
+  ix_up2(contracted(ix_limbs(ix_align<4>(g(0, 5), gb)), ix_limbs(xy)), contracted(ix_limbs(yx), ix_limbs(ix_align<4>(g(1, 6), gb))), e3,
+         bxS, byS);
+  const int64_t t3 = ix_prod(bxS, bx) + ix_prod(byS, by);
+  e3 += eB + 61;
+  const int64_t t4 = ix_prod(X, rS);
+  int KH = ix_max(ix_max(e1, e2), ix_max(e3, e4)) + 2;
+  int64_t H, uc = ix_prod(c1, u) + ix_prod(c2, v);  // [61.4]
+  int euc = ec + eu + 61;
+  double F3 = 0.0;
+  int64_t bzS = 0;
+  int ebz = 0;
+  if (hasz) {
+    const int egz = ix_exp<4>(gz), ez = egz + eS + 60;
+    ebz = ix_exp<4>(gw) + eS + 60;
+    const int64_t mzS = contracted(ix_limbs(ix_align<4>(g(0, 3), gz)), ix_limbs(ix_align<4>(g(1, 3), gz)));
+    bzS = contracted(ix_limbs(ix_align<4>(g(0, 7), gw)), ix_limbs(ix_align<4>(g(1, 7), gw)));
+    const int er = erS + ew + 61, K3 = ix_max(ez, er) + 1;
+    const int64_t c3 = ix_shr(mzS, K3 - ez) - ix_shr(ix_prod(rS, w), K3 - er);  // [60.5]
+    F3 = ix_double(ix_mul(c3, M), K3 + eM + 62);
+    const int e5 = ez + ew + 61, e6 = ebz + eBz + 61;
+    KH = ix_max(KH, ix_max(e5, e6) + 2);
+    H = -ix_shr(ix_prod(ix_limbs(mzS), w), KH - e5) - ix_shr(ix_prod(ix_limbs(bzS), bz), KH - e6);
+    const int e7 = K3 + ew + 61, K = ix_max(euc, e7) + 1;
+    uc = ix_shr(uc, K - euc) + ix_shr(ix_prod(ix_limbs(c3), w), K - e7);
+    euc = K;
+  } else {
+    H = 0;
+  }
+  out(3, F3);
+  H += ix_shr(t1, KH - e1) - ix_shr(t2, KH - e2) - ix_shr(t3, KH - e3) + ix_shr(t4, KH - e4);  // [61.1]
+  const Limbs Hl = ix_up(H, KH);
+  const int eH = KH + gas.ekap + 61, K4 = ix_max(euc, eH) + 1;
+  int64_t F4 = ix_mul(ix_shr(uc, K4 - euc) + ix_shr(ix_prod(Hl, gas.kap), K4 - eH), M);  // [60]
+  int eF4 = K4 + eM + 62;
+  double F5 = 0.0, F6 = 0.0, F7 = 0.0;
+  if (eta != 0.0) {  // resistive terms: F_B = eta (-Jz sy, Jz sx, grad Bz.S), the energy takes B.F_B
+    const Limbs et = ix_limbs(ix_align<3>(eta, mt));
+    const int eet = ix_exp<3>(mt);
+    int eJ = egB + eet + 62, eR = eB + eS + 60;
+    const int64_t j = ix_mul(yx - xy, et);  // [60]
+    Limbs jl, jn;
+    ix_up2(j, -j, eJ, jl, jn);
+    F5 = ix_double(ix_prod(jn, ny), eJ + eS + 61);
+    F6 = ix_double(ix_prod(jl, nx), eJ + eS + 61);
+    IxSum t;  // By sx - Bx sy
+    t.add(by, nx);
+    IxSum t_;
+    t_.add(bx, ny);
+    const Limbs Rl = ix_up(t.value4() - t_.value4(), eR);
+    int64_t R = ix_prod(jl, Rl);  // [60.5]
+    eR += eJ + 61;
+    if (hasz) {
+      const int64_t f7 = ix_mul(bzS, et);  // [59.5]
+      const int e7 = ebz + eet + 62, e8 = e7 + eBz + 61, K = ix_max(eR, e8) + 1;
+      F7 = ix_double(f7, e7);
+      R = ix_shr(R, K - eR) + ix_shr(ix_prod(ix_limbs(f7), bz), K - e8);
+      eR = K;
+    }
+    const int K = ix_max(eF4, eR) + 1;
+    F4 = ix_shr(F4, K - eF4) + ix_shr(R, K - eR);
+    eF4 = K;
+  }
+  out(4, ix_double(F4, eF4));
+  out(5, F5);
+  out(6, F6);
+  out(7, F7);
   return true;
 }
 

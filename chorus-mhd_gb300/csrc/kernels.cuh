@@ -365,6 +365,7 @@ __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int 
       for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
         s.act[e0 + e] = 0;
         s.nv[e0 + e] = 0;
+        s.gr[e0 + e] = 0;
       }
     return;
   }
@@ -398,13 +399,19 @@ __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int 
     acc = warp_sum(acc);
     if (lane == 0) {
       s.Se[e0 + e] = acc;
+      sU[e * NS] = acc;
       if (s.skip) {
         const int a = (acc < 1e-6) ? 0 : 1;  // NaN counts as active
         s.act[e0 + e] = a;
-        s.nv[e0 + e] = a;
+        s.nv[e0 + e] = 0;  // F1 marks the active cells and their face neighbours
+        s.gr[e0 + e] = 0;
       }
     }
   }
+  // the AV ramp of the cells (log10 and sin, once per cell and by neighbouring lanes: in the pass
+  // that reads it for a cell and its four neighbours it took 14 us of a small mesh's stage)
+  __syncthreads();
+  for (int e = threadIdx.x; e < cnt; e += blockDim.x) s.Sw[e0 + e] = av_ramp(sU[e * NS]);
   if (!(sensor & 2)) return;
   // the same sensor of variable 6 (B_x), whose muAV(6) only the plot output reads
   // (tecplotter.f90:39 from AV.f90:60-73); in the reference's division form, so a zero
@@ -444,8 +451,11 @@ template <int N>
 __global__ void __maxnreg__(e1_regs(N)) k_e1(const __grid_constant__ SolveDev s, int epb, int sensor, int c0, int c1) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
-  // bit 4: the first pass of a stage, which starts the stage's wave-speed maximum
-  if ((sensor & 4) && c0 == 0 && blockIdx.x == 0 && threadIdx.x == 0) *s.eig = 0ull;
+  // bit 4: the first pass of a stage, which starts the stage's wave-speed maximum and list
+  if ((sensor & 4) && c0 == 0 && blockIdx.x == 0 && threadIdx.x == 0) {
+    *s.eig = 0ull;
+    *s.vcount = 0;
+  }
   sensor &= 3;
   const int e0 = c0 + blockIdx.x * epb;
   const int cnt = min(epb, c1 - e0);
@@ -454,9 +464,8 @@ __global__ void __maxnreg__(e1_regs(N)) k_e1(const __grid_constant__ SolveDev s,
   e1_body<N, OpsTU>(s, e0, cnt, epb, sensor, sm);
 }
 
-// cells of this CTA whose gradients (mode 0) or viscous fluxes (mode 1) are needed,
-// compacted into a shared list; returns the count
-__device__ __forceinline__ int active_cells(const SolveDev& s, int e0, int cnt, int mode, int* list) {
+// cells of this CTA with a viscous flux, compacted into a shared list; returns the count
+__device__ __forceinline__ int active_cells(const SolveDev& s, int e0, int cnt, int* list) {
   // the first warp tests 32 cells at a time (their flag loads in flight together) and
   // compacts them in cell order with a ballot
   __shared__ int n_act;
@@ -465,21 +474,8 @@ __device__ __forceinline__ int active_cells(const SolveDev& s, int e0, int cnt, 
     int n = 0;
     for (int base = 0; base < cnt; base += 32) {
       const int e = base + lane;
-      int need = 0;
-      if (e < cnt) {
-        const int c = e0 + e;
-        need = 1;
-        if (s.skip) {
-          need = s.nv[c];
-          if (mode == 0) {
-            const int4 b = s.nbr[c];
-            const int nx = b.x >= 0 ? s.nv[b.x] : 0, ny = b.y >= 0 ? s.nv[b.y] : 0;
-            const int nz = b.z >= 0 ? s.nv[b.z] : 0, nw = b.w >= 0 ? s.nv[b.w] : 0;
-            need |= nx | ny | nz | nw;
-          }
-        }
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, need != 0);
+      const bool need = e < cnt && (!s.skip || s.nv[e0 + e]);
+      const unsigned m = __ballot_sync(0xffffffffu, need);
       if (need) list[n + __popc(m & ((1u << lane) - 1u))] = e;
       n += __popc(m);
     }
@@ -518,6 +514,11 @@ struct F1Warp {
 };
 constexpr int kF1Threads = 160;
 constexpr size_t f1_smem(int threads) { return (size_t)(threads / 32) * sizeof(F1Warp); }
+
+// put cell c on the list of the cells with viscous flux, the first time
+__device__ __forceinline__ void mark_viscous(const SolveDev& s, int c) {
+  if (atomicExch(&s.nv[c], 1) == 0) s.vlist[atomicAdd(s.vcount, 1)] = c;
+}
 
 // Face points first .. first + 31, then on by step, ... < n of a warp (first and step are the
 // warp's, the same for its lanes); map(i) is the point's number among the solve's two-sided
@@ -591,6 +592,7 @@ __device__ __forceinline__ unsigned long long f1_points(const SolveDev& s, int f
     cp_async_commit();
     if (i < n) {
       const int t = map(i);
+      const bool nfp0 = (t < n2 ? t : t - n2) % N == 0;
       const long long gl = w.g[buf][0][lane], gr = w.g[buf][1][lane];
       const double2 nrm = w.fn[buf][lane][0];
       // (the states are read from shared memory where they are used, not kept)
@@ -615,12 +617,12 @@ __device__ __forceinline__ unsigned long long f1_points(const SolveDev& s, int f
       s.Azf[gl] = az;
       if (gr >= 0) {
         s.Azf[gr] = az;
-        if (s.skip && t % N == 0) {
-          const int4 fc = w.rec[slot][lane];
-          if (s.act[fc.x] | s.act[fc.z]) {
-            s.nv[fc.x] = 1;
-            s.nv[fc.z] = 1;
-          }
+      }
+      if (s.skip && nfp0) {  // once per face: AV-active cells and their neighbours carry viscous flux
+        const int4 fc = w.rec[slot][lane];
+        if (s.act[fc.x] || (gr >= 0 && s.act[fc.z])) {
+          mark_viscous(s, fc.x);
+          if (gr >= 0) mark_viscous(s, fc.z);
         }
       }
     }
@@ -692,71 +694,156 @@ __device__ __forceinline__ long long across(const SolveDev& s, int c, int fp) {
 // ---------------------------------------------------------------------------
 // E2: gradients at solution points and their values at every flux point
 // ---------------------------------------------------------------------------
-// the AV viscosity on the four faces of cell c (compAVflux / interfaceAVflux /
-// cyclocAVflux, AV.f90:199-303, 494-564): the mean of the two cells' muAV(1) on a
-// two-sided face (the same bits from either side: the sum commutes), the cell's own on a
-// FREE face; muAV(1) from the stage's sensor and epsilon0 = eigvmax h/(N-1) (AV.f90:147)
+// the AV viscosity on local face lf of cell c (compAVflux / interfaceAVflux / cyclocAVflux,
+// AV.f90:199-303, 494-564): the mean of the two cells' muAV(1) on a two-sided face (the same
+// bits from either side: the sum commutes), the cell's own on a FREE face; muAV(1) from the
+// stage's sensor and epsilon0 = eigvmax h/(N-1) (AV.f90:147)
+template <int N>
+__device__ __forceinline__ double face_mu(const SolveDev& s, int c, int lf) {
+  const double eps0 = __longlong_as_double((long long)*s.eig) * s.hmsh / (double)(N - 1) * 1.0, h0 = eps0 / 2.0;
+  const double mc = h0 * s.Sw[c];
+  const int o = (&s.nbr[c].x)[lf - 1];
+  return o >= 0 ? half(mc + h0 * s.Sw[o]) : mc;
+}
+
 template <int N>
 __device__ __forceinline__ void cell_face_mu(const SolveDev& s, int c) {
-  double m[4] = {0.0, 0.0, 0.0, 0.0};
-  if (s.artiv) {
-    const double eps0 = __longlong_as_double((long long)*s.eig) * s.hmsh / (double)(N - 1) * 1.0;
-    const double mc = av_mu(s.Se[c], eps0);
-    const int4 b = s.nbr[c];
-    const int o[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int k = 0; k < 4; k++) m[k] = o[k] >= 0 ? 0.5 * (mc + av_mu(s.Se[o[k]], eps0)) : mc;
-  }
-#pragma unroll
-  for (int k = 0; k < 4; k++) s.muf[4 * c + k] = m[k];
+  for (int k = 0; k < 4; k++) s.muf[4 * c + k] = s.artiv ? face_mu<N>(s, c, k + 1) : 0.0;
+}
+
+constexpr int kE3Fp64 = -(1 << 28);  // in place of an exponent: the value is a double
+
+// 1/J (sum of the two families' derivatives) where one of the three is not in integer form: a
+// call, because a branch of few FP64 instructions would be predicated, and an FP64 instruction
+// occupies its pipe whether its lanes are on or off.  k0, k1: exponents of the sums V0, V1 or
+// kE3Fp64 for doubles.
+static __device__ __noinline__ double e3_fp64(int64_t V0, int k0, int64_t V1, int k1, double j) {
+  const double y0 = k0 != kE3Fp64 ? ix_double(V0, k0) : __longlong_as_double(V0);
+  const double y1 = k1 != kE3Fp64 ? ix_double(V1, k1) : __longlong_as_double(V1);
+  return (y0 + y1) * j;
+}
+
+// shared memory of the pass for epb cells (e2_cells)
+constexpr size_t e2_smem(int N, int epb) {
+  return (size_t)epb * ((size_t)2 * (N + 1) * N * (72 + 16) + (size_t)N * N * (128 + 8 + 4) + (size_t)N * 8 * 4 + 2 * N * 4) + 64;
 }
 
 template <int N, class O>
-__device__ __forceinline__ void e2_cells(const SolveDev& s, const int* cells, int n, double* sm) {
+__device__ __forceinline__ void e2_cells(const SolveDev& s, const int* cells, int n, int keep, double* sm) {
   // gradients of the n (<= epb) listed cells; grad A_z (nablaAsp) is computed with the
   // divergence in the last pass.  nablaQsp (compflux.f90:107-157) in its conservative
   // form: grad_x Q = (1/J) [d/dxi (S1(1,1) Q) + d/deta (S2(2,1) Q)], grad_y the same with
-  // the second metric entries, i.e. the divergence of the products of the face-corrected
-  // flux-point states with the metric terms, differentiated along the lines on the
-  // integer pipes as in E3.
+  // the second metric entries, i.e. the divergence of the products of the face-averaged
+  // flux-point states with the metric terms, differentiated along the lines on the integer
+  // pipes as in E3.  The products are integers too: a line's states aligned once serve both
+  // metric entries.  (128x128 cells, N = 5, every cell: 0.173 ms a stage with the products, the
+  // family sums and 1/J in FP64, 0.138 ms like this.)  An
+  // operand is cut at 2^-58 of its line's largest, a product at 2^-61.
   constexpr int NS = D<N>::NS, NF1 = D<N>::NF1, NFP = D<N>::NFP;
-  double* sP = sm;                // [n][NFP][16] Q_k * (S_x, S_y): k + 8 d
-  double* sG = sP + n * NFP * 16;  // [n][NS][16] grad Q (d*8 + k)
-  double* sJ = sG + n * NS * 16;   // [n][NS] 1/J
-  for (int i = threadIdx.x; i < n * NFP * 8; i += blockDim.x) {
-    const int le = i / (NFP * 8), r = i - le * (NFP * 8), fp = r >> 3, k = r & 7;
-    const size_t g = (size_t)cells[le] * NFP + fp;
-    const long long o = across<N>(s, cells[le], fp);  // face traces enter as the mean of both sides
-    const double own = s.Qvf[g * 9 + k], q = o >= 0 ? half(own + s.Qvf[o * 9 + k]) : own;
-    sP[(le * NFP + fp) * 16 + k] = q * s.met[2 * g];
-    sP[(le * NFP + fp) * 16 + 8 + k] = q * s.met[2 * g + 1];
-  }
+  double* sQ = sm;                                              // [n][NFP][9] Q
+  Limbs* sS = reinterpret_cast<Limbs*>(sQ + n * NFP * 9);       // [n][NFP][2] metric entries, aligned per line
+  double* sG = reinterpret_cast<double*>(sS + n * NFP * 2);     // [n][NS][16] grad Q (d*8 + k)
+  int64_t* sJ = reinterpret_cast<int64_t*>(sG + n * NS * 16);   // [n][NS] 1/J as an integer
+  int* sE = reinterpret_cast<int*>(sJ + n * NS);                // [n][NS] and its exponent
+  int* sK = sE + n * NS;                                        // [n][N][8] exponents of the xi-line sums
+  int* sM = sK + n * N * 8;                                     // [n][2N] exponents of the lines' metric entries
+  for (int le = 0; le < n; le++)
+    block_copy_async(sQ + le * NFP * 9, s.Qvf + (size_t)cells[le] * NFP * 9, NFP * 9);
+  cp_async_commit();
   for (int i = threadIdx.x; i < n * NS; i += blockDim.x) {
-    const int le = i / NS, p = i - le * NS;
-    sJ[i] = s.invJ[(size_t)cells[le] * NS + p];
+    const int le = i / NS;
+    const double j = s.invJ[(size_t)cells[le] * NS + i - le * NS];
+    const uint32_t m = ix_abs_word(j);
+    sJ[i] = ix_align<2>(j, m);
+    sE[i] = m >= kIxLow && m < kIxHigh ? ix_exp<2>(m) : kE3Fp64;
+  }
+  // flux point r of line l of a cell: the xi lines, then the eta lines
+  auto line_point = [](int l, int r) { return l < N ? l * (N + 1) + r : NF1 + r * N + (l - N); };
+  for (int i = threadIdx.x; i < n * 2 * N; i += blockDim.x) {
+    const int le = i / (2 * N), l = i - le * 2 * N;
+    const double2* met = reinterpret_cast<const double2*>(s.met) + (size_t)cells[le] * NFP;
+    uint32_t m = 0;
+#pragma unroll 1
+    for (int r = 0; r <= N; r++) {
+      const double2 a = met[line_point(l, r)];
+      m = ix_max(m, ix_max(ix_abs_word(a.x), ix_abs_word(a.y)));
+    }
+    sM[i] = m >= kIxLow && m < kIxHigh ? ix_exp<4>(m) : kE3Fp64;
+#pragma unroll 1
+    for (int r = 0; r <= N; r++) {
+      const double2 a = met[line_point(l, r)];
+      Limbs* o = sS + (le * NFP + line_point(l, r)) * 2;
+      o[0] = ix_limbs(ix_align<4>(a.x, m));
+      o[1] = ix_limbs(ix_align<4>(a.y, m));
+    }
+  }
+  cp_async_wait();
+  __syncthreads();
+  // face traces enter as the mean of both sides
+  for (int i = threadIdx.x; i < n * 4 * N * 8; i += blockDim.x) {
+    const int k = i & 7, r = i >> 3, le = r / (4 * N), f = r - le * 4 * N, lf = f / N + 1, nfp = f - (lf - 1) * N;
+    const int c = cells[le], o = (&s.nbr[c].x)[lf - 1];
+    if (o < 0) continue;
+    double* q = sQ + (le * NFP + face_fp<N>(lf, nfp)) * 9 + k;
+    *q = half(*q + s.Qvf[((size_t)o * NFP + face_fp<N>((&s.nbrlf[c].x)[lf - 1], N - 1 - nfp)) * 9 + k]);
   }
   __syncthreads();
-  // grad Q (variables 1-8) at the solution points: one (cell, line, quantity) per thread,
-  // the xi lines first, then the eta lines adding to them and scaling by 1/J
+  // grad Q (variables 1-8) at the solution points: one (cell, line, variable) per thread,
+  // the xi lines first, then the eta lines adding to them and multiplying by 1/J
 #pragma unroll 1
   for (int fam = 0; fam < 2; fam++) {
-    for (int t = threadIdx.x; t < n * N * 16; t += blockDim.x) {
-      const int c = t & 15, el = t >> 4, le = el / N, ln = el - le * N;
-      const int fp0 = fam ? NF1 + ln : ln * (N + 1), fps = fam ? N : 1;
-      double y[N];
-      deriv_line<N, O>(sP + (le * NFP + fp0) * 16 + c, fps * 16, y);
-      const int p0 = fam ? ln : ln * N, ps = fam ? N : 1;
-      double* g = sG + (le * NS + p0) * 16 + c;
-      if (!fam) {
+    for (int t = threadIdx.x; t < n * N * 8; t += blockDim.x) {
+      const int k = t & 7, el = t >> 3, le = el / N, ln = el - le * N;
+      const int fp0 = le * NFP + (fam ? NF1 + ln : ln * (N + 1)), fps = fam ? N : 1, eS = sM[le * 2 * N + fam * N + ln];
+      uint32_t m = 66u << 20;
 #pragma unroll
-        for (int i = 0; i < N; i++) g[i * ps * 16] = y[i];
-      } else {
-        double* out = s.nQs + ((size_t)cells[le] * NS + p0) * 18 + (c < 8 ? c : c + 1);
+      for (int r = 0; r <= N; r++) m = ix_max(m, ix_abs_word(sQ[(fp0 + r * fps) * 9 + k]));
+      const bool ok = m < kIxHigh && eS != kE3Fp64;
+      const int kv = ok ? ix_exp<4>(m) + eS + 62 + 58 - O::ops().MS : kE3Fp64;
+      Limbs q[N + 1];
 #pragma unroll
-        for (int i = 0; i < N; i++) {
-          const double a = (g[i * ps * 16] + y[i]) * sJ[le * NS + p0 + i * ps];
-          g[i * ps * 16] = a;
-          out[(size_t)i * ps * 18] = a;
+      for (int r = 0; r <= N; r++) q[r] = ix_limbs(ix_align<4>(sQ[(fp0 + r * fps) * 9 + k], m));
+      if (!fam) sK[t] = kv;
+#pragma unroll 1
+      for (int d = 0; d < 2; d++) {
+        double* g = sG + le * NS * 16 + d * 8 + k;
+        auto finish = [&](int i, int64_t V) {
+          if (!fam) {
+            g[(ln * N + i) * 16] = __longlong_as_double(V);
+            return;
+          }
+          const int p = i * N + ln, ps = le * NS + p, eJ = sE[ps], k0 = sK[(le * N + i) * 8 + k];
+          const int64_t V0 = __double_as_longlong(g[p * 16]);
+          double a;
+          if (ok && k0 != kE3Fp64 && eJ != kE3Fp64) {
+            const int K = max(k0, kv);
+            const int64_t sum = ix_shr(V0, K - k0 + O::ops().MV) + ix_shr(V, K - kv + O::ops().MV);
+            a = ix_double(ix_mul(sum, ix_limbs(sJ[ps])), K + O::ops().MV + eJ + 62);
+          } else {
+            a = e3_fp64(V0, k0, V, kv, s.invJ[(size_t)cells[le] * NS + p]);
+          }
+          g[p * 16] = a;
+          // (only the evaluation whose arrays can be downloaded stores them)
+          if (keep) s.nQs[((size_t)cells[le] * NS + p) * 18 + 9 * d + k] = a;
+        };
+        if (ok) {
+          int64_t X[N + 1];
+#pragma unroll
+          for (int r = 0; r <= N; r++) X[r] = ix_mul(q[r], sS[(fp0 + r * fps) * 2 + d]);
+          fix_mirror_core<N, N + 1, -1>(X, O::ops().MH, O::ops().ML, finish);
+        } else {
+          const double* met = s.met + (size_t)cells[le] * NFP * 2 + d;
+#pragma unroll 1
+          for (int i = 0; i < N; i++) {
+            double a = 0.0;
+#pragma unroll 1
+            for (int r = 0; r <= N; r++) {
+              const int fp = fp0 + r * fps;
+              a += O::ops().M[r + (N + 1) * i] * (sQ[fp * 9 + k] * met[2 * (fp - le * NFP)]);
+            }
+            finish(i, __double_as_longlong(a));
+          }
         }
       }
     }
@@ -781,65 +868,159 @@ __device__ __forceinline__ void e2_cells(const SolveDev& s, const int* cells, in
   }
 }
 
-// tile form (batched kernels): the cells of [e0, e0+cnt) whose gradients are needed
+// E2 by a CTA that is number `first` of `stride`.  Every cell (skip = 0): groups of epb cells.
+// Otherwise the listed cells with a viscous flux and their face neighbours: a CTA takes epb
+// list entries at a time and those of their neighbours that are not listed and that no other
+// CTA has claimed (a cell's gradients do not depend on who computes them), in groups.  The
+// work is spread evenly however the active cells lie: with one CTA per range of cells E2 and V
+// took 0.235 ms a stage for the 2% of active cells of a rotor (256x256, N = 4), 0.060 ms like this.
+// keep: also every cell's face viscosities, which can be downloaded.
 template <int N, class O>
-__device__ __forceinline__ void e2_body(const SolveDev& s, int e0, int cnt, int epb, double* sm) {
-  __shared__ int list[64];
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) cell_face_mu<N>(s, e0 + e);
-  const int nact = active_cells(s, e0, cnt, 0, list);
-  if (nact == 0) return;
-  for (int i = threadIdx.x; i < nact; i += blockDim.x) list[i] += e0;
-  __syncthreads();
-  e2_cells<N, O>(s, list, nact, sm);
+__device__ __forceinline__ void e2_all(const SolveDev& s, int first, int stride, int epb, int keep, double* sm) {
+  __shared__ int list[5 * 64];
+  __shared__ int taken;
+  if (keep)
+    for (int c = first * blockDim.x + threadIdx.x; c < s.NC; c += stride * blockDim.x) cell_face_mu<N>(s, c);
+  const int total = s.skip ? *s.vcount : s.NC;
+  for (int base = first * epb; base < total; base += stride * epb) {
+    const int m = min(epb, total - base);
+    if (threadIdx.x == 0) taken = s.skip ? 0 : m;
+    __syncthreads();
+    for (int t = threadIdx.x; t < (s.skip ? 5 * m : m); t += blockDim.x) {
+      if (!s.skip) {
+        list[t] = base + t;
+        continue;
+      }
+      const int v = s.vlist[base + t / 5], k = t % 5, c = k == 4 ? v : (&s.nbr[v].x)[k];
+      if (k == 4 || (c >= 0 && !s.nv[c] && atomicExch(&s.gr[c], 1) == 0)) list[atomicAdd(&taken, 1)] = c;
+    }
+    __syncthreads();
+    const int n = taken;
+    for (int g = 0; g < n; g += epb) {
+      e2_cells<N, O>(s, list + g, min(epb, n - g), keep, sm);
+      __syncthreads();
+    }
+  }
 }
 
-// does cell c need its gradients (itself or a face neighbour has viscous work)?
-__device__ __forceinline__ bool needs_gradients(const SolveDev& s, int c) {
-  if (!s.skip || s.nv[c]) return true;
-  const int4 b = s.nbr[c];
-  return (b.x >= 0 && s.nv[b.x]) || (b.y >= 0 && s.nv[b.y]) || (b.z >= 0 && s.nv[b.z]) || (b.w >= 0 && s.nv[b.w]);
+template <int N>
+__global__ void __launch_bounds__(512, 2) k_e2(const __grid_constant__ SolveDev s, int epb, int keep) {
+  extern __shared__ __align__(16) double sm[];
+  pdl_wait();
+  e2_all<N, OpsTU>(s, blockIdx.x, gridDim.x, epb, keep, sm);
 }
 
-// E2 over a chunk of `chunk` (<= blockDim.x) cells starting at c0: every thread tests
-// one cell, the CTA compacts the cells that need gradients into an ordered list and runs
-// them in groups of epb, so chunks without viscous work cost one coalesced test
+// ---------------------------------------------------------------------------
+// V: the total flux Ft = Fc - viscous, resistive and AV flux of the cells that carry one, in
+// Fc's place or (where the inviscid flux stays downloadable) beside it (interfaceVISflux /
+// BCVISFLUX / CYCLOCVISFLUX, comp_viscous_flux).  One flux point per thread with the integer
+// form of the flux; the FP64 form inside E3 kept that pass at 0.37 ms over its inviscid time
+// (128x128 cells, N = 5, every cell viscous), V takes 0.171 ms.  Bound by instruction issue
+// (43%) and the loads of Q and grad Q (292 MB, 1.7 TB/s) about equally.
+// ---------------------------------------------------------------------------
+// cells per group and threads per CTA: one flux point per thread
+constexpr int v_epb(int N) { return N >= 6 ? 1 : 128 / (2 * (N + 1) * N); }
+constexpr int v_threads(int N) { return (v_epb(N) * 2 * (N + 1) * N + 31) / 32 * 32; }
+constexpr size_t v_smem(int N) { return (size_t)v_epb(N) * 2 * (N + 1) * N * 36 * 8; }
+
+// the viscosity of flux point fp of a cell with AV viscosities mf[4] on its local faces 1..4:
+// mu + the AV viscosity, linear between the faces
 template <int N, class O>
-__device__ __forceinline__ void e2_chunk(const SolveDev& s, int c0, int chunk, int epb, double* sm) {
-  __shared__ int list[512];
-  __shared__ int woff[17];
-  const int c = c0 + threadIdx.x;
-  const bool mine = (int)threadIdx.x < chunk && c < s.NC;
-  if (mine) cell_face_mu<N>(s, c);
-  const bool need = mine && needs_gradients(s, c);
-  const unsigned m = __ballot_sync(0xffffffffu, need);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) woff[w + 1] = __popc(m);
+__device__ __forceinline__ double point_mu(const SolveDev& s, const double* mf, int fp) {
+  constexpr int NF1 = D<N>::NF1;
+  if (!s.artiv) return s.mu;
+  const double x = O::ops().Xf[fp < NF1 ? fp % (N + 1) : (fp - NF1) / N];
+  const double a = fp < NF1 ? mf[3] : mf[0], b = fp < NF1 ? mf[1] : mf[2];
+  return s.mu + (a * (1.0 - x) + b * x);
+}
+
+// the FP64 form of a point's flux, for the states that the integer form leaves out (a call, so
+// that it takes no registers from the other points)
+static __device__ __noinline__ void vflux_fp64(const double* q, const double* g, double mut, double eta, double gam,
+                                               double sx, double sy, double* F) {
+  double Fv[8];
+  vflux_contra(q, g, mut, eta, gam, sx, sy, Fv);
+#pragma unroll
+  for (int k = 1; k < 8; k++) F[k] = Fv[k];
+}
+
+template <int N, class O>
+__device__ __forceinline__ void v_cells(const SolveDev& s, const int* cells, int n, double* Ft, double* sm) {
+  constexpr int NFP = D<N>::NFP;
+  double* sG = sm;                // [n][NFP][18] grad Q
+  double* sQ = sG + n * NFP * 18;  // [n][NFP][9] Q
+  double* sV = sQ + n * NFP * 9;   // [n][NFP][9] the viscous flux (components 1..7)
+  for (int le = 0; le < n; le++) {
+    block_copy_async(sG + le * NFP * 18, s.nQvf + (size_t)cells[le] * NFP * 18, NFP * 18);
+    block_copy_async(sQ + le * NFP * 9, s.Qvf + (size_t)cells[le] * NFP * 9, NFP * 9);
+  }
+  cp_async_commit();
+  __shared__ double smu[v_epb(N)][4];
+  if (s.artiv && (int)threadIdx.x < 4 * n) smu[threadIdx.x >> 2][threadIdx.x & 3] = face_mu<N>(s, cells[threadIdx.x >> 2], (threadIdx.x & 3) + 1);
+  cp_async_wait();
   __syncthreads();
-  if (threadIdx.x == 0) {
-    woff[0] = 0;
-    for (int i = 1; i <= (int)(blockDim.x >> 5); i++) woff[i] += woff[i - 1];
+  // on a two-sided face the traces of Q and of grad Q are the means of both sides'
+  // (interfaceflux_all.f90:79-91, 118-199, cyclocflux_all.f90:118-208); a FREE face keeps its
+  // own (BCVISFLUX): 24 values of each of a cell's 4 N face points
+  for (int i = threadIdx.x; i < n * 4 * N * 24; i += blockDim.x) {
+    const int j = i % 24, r = i / 24, le = r / (4 * N), k = r - le * 4 * N, lf = k / N + 1, nfp = k - (lf - 1) * N;
+    const int c = cells[le], o = (&s.nbr[c].x)[lf - 1];
+    if (o < 0) continue;
+    const size_t go = (size_t)o * NFP + face_fp<N>((&s.nbrlf[c].x)[lf - 1], N - 1 - nfp);
+    const int at = le * NFP + face_fp<N>(lf, nfp);
+    if (j < 16) {
+      const int m = j < 8 ? j : j + 1;
+      sG[at * 18 + m] = half(sG[at * 18 + m] + s.nQvf[go * 18 + m]);
+    } else {
+      sQ[at * 9 + j - 16] = half(sQ[at * 9 + j - 16] + s.Qvf[go * 9 + j - 16]);
+    }
   }
   __syncthreads();
-  if (need) list[woff[w] + __popc(m & ((1u << lane) - 1u))] = c;
-  const int n = woff[blockDim.x >> 5];
+  for (int t = threadIdx.x; t < n * NFP; t += blockDim.x) {
+    const int le = t / NFP, fp = t - le * NFP, c = cells[le];
+    const double2 m = reinterpret_cast<const double2*>(s.met)[(size_t)c * NFP + fp];
+    const double mut = point_mu<N, O>(s, smu[le], fp);
+    volatile double* q = sQ + 9 * t;
+    const volatile double* gr = sG + 18 * t;
+    if (!vflux_int([&](int k) { return q[k]; }, [&](int d, int k) { return gr[9 * d + k]; }, mut, s.eta0, m.x, m.y, s.gas,
+                   [&](int k, double f) { sV[t * 9 + k] = f; }))
+      vflux_fp64(sQ + 9 * t, sG + 18 * t, mut, s.eta0, s.gam, m.x, m.y, sV + 9 * t);
+  }
   __syncthreads();
-  for (int g = 0; g < n; g += epb) {
-    e2_cells<N, O>(s, list + g, min(epb, n - g), sm);
+  for (int i = threadIdx.x; i < n * NFP * 4; i += blockDim.x) {
+    const int t = i >> 2, j = i & 3, le = t / NFP;
+    const size_t g = ((size_t)cells[le] * NFP + (t - le * NFP)) * 8 + 2 * j;
+    const double2 a = *reinterpret_cast<const double2*>(s.Fc + g);
+    *reinterpret_cast<double2*>(Ft + g) = make_double2(j ? a.x - sV[9 * t + 2 * j] : a.x, a.y - sV[9 * t + 2 * j + 1]);
+  }
+}
+
+// V by a CTA that is number `first` of `stride`
+template <int N, class O>
+__device__ __forceinline__ void v_all(const SolveDev& s, int first, int stride, double* Ft, double* sm) {
+  __shared__ int list[v_epb(N)];
+  const int total = s.skip ? *s.vcount : s.NC;
+  for (int base = first * v_epb(N); base < total; base += stride * v_epb(N)) {
+    const int m = min(v_epb(N), total - base);
+    if ((int)threadIdx.x < m) list[threadIdx.x] = s.skip ? s.vlist[base + threadIdx.x] : base + threadIdx.x;
+    __syncthreads();
+    v_cells<N, O>(s, list, m, Ft, sm);
     __syncthreads();
   }
 }
 
 template <int N>
-__global__ void __launch_bounds__(512, 2) k_e2(SolveDev s, int epb, int chunk) {
+__global__ void __launch_bounds__(v_threads(N)) k_v(const __grid_constant__ SolveDev s, double* Ft) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
-  e2_chunk<N, OpsTU>(s, blockIdx.x * chunk, chunk, epb, sm);
+  v_all<N, OpsTU>(s, blockIdx.x, gridDim.x, Ft, sm);
 }
+
 // ---------------------------------------------------------------------------
 // F2: face-averaged gradients and face AV viscosity
 // ---------------------------------------------------------------------------
 // face averages of the grad Q traces in place (interfaceVISflux, CYCLOCVISFLUX).  The
-// stage itself averages them where the viscous flux reads them (E3); this pass makes the
+// stage itself averages them where the viscous flux reads them (V, E3); this pass makes the
 // stored traces equal to the reference's nablaQvfi/nablaQvfj when they are downloaded.
 template <int N>
 __device__ __forceinline__ void f2_point(const SolveDev& s, int t) {
@@ -868,22 +1049,15 @@ __global__ void __launch_bounds__(256) k_f2(SolveDev s) {
 // their total flux in shared memory: a call, so that the registers it needs are not those of
 // the whole pass
 template <int N, class O>
-static __device__ __noinline__ void e3_viscous(const SolveDev& s, int e0, int nact, const int* list, double* sF) {
-  constexpr int NF1 = D<N>::NF1, NFP = D<N>::NFP;
+static __device__ __noinline__ void e3_viscous(const SolveDev& s, int e0, int nact, const int* list, double* sF, double* smu) {
+  constexpr int NFP = D<N>::NFP;
+  if (s.artiv)
+    for (int i = threadIdx.x; i < 4 * nact; i += blockDim.x) smu[i] = face_mu<N>(s, e0 + list[i >> 2], (i & 3) + 1);
+  __syncthreads();
   for (int t = threadIdx.x; t < nact * NFP; t += blockDim.x) {
     const int le = t / NFP, fp = t - le * NFP, e = list[le], c = e0 + e;
     const size_t g = (size_t)c * NFP + fp;
-    double mut = s.mu;
-    if (s.artiv) {
-      const double* mf = s.muf + 4 * c;
-      if (fp < NF1) {
-        const double x = O::ops().Xf[fp % (N + 1)];
-        mut += mf[3] * (1.0 - x) + mf[1] * x;
-      } else {
-        const double x = O::ops().Xf[(fp - NF1) / N];
-        mut += mf[0] * (1.0 - x) + mf[2] * x;
-      }
-    }
+    const double mut = point_mu<N, O>(s, smu + 4 * le, fp);
     if (mut != 0.0 || s.eta0 != 0.0) {
       double q[9], gq[18], Fv[8];
       const double* pq = s.Qvf + g * 9;
@@ -925,16 +1099,17 @@ constexpr size_t e3_smem(int N, int epb) {
   return (size_t)epb * ((size_t)2 * (N + 1) * N * 10 * 8 + (size_t)N * N * (72 + 16 + 8 + 4) + (size_t)N * 10 * 4) + 16;
 }
 
-constexpr int kE3Fp64 = -(1 << 28);  // in place of an exponent: the value is a double
+constexpr long long kVPassPoints = 49152;
 
-// 1/J (sum of the two families' derivatives) where one of the three is not in integer form: a
-// call, because a branch of few FP64 instructions would be predicated, and an FP64 instruction
-// occupies its pipe whether its lanes are on or off.  k0, k1: exponents of the sums V0, V1 or
-// kE3Fp64 for doubles.
-static __device__ __noinline__ double e3_fp64(int64_t V0, int k0, int64_t V1, int k1, double j) {
-  const double y0 = k0 != kE3Fp64 ? ix_double(V0, k0) : __longlong_as_double(V0);
-  const double y1 = k1 != kE3Fp64 ? ix_double(V1, k1) : __longlong_as_double(V1);
-  return (y0 + y1) * j;
+// Does the viscous flux get its own pass?  On meshes large enough for the extra launch to be
+// small beside a stage; E3 then runs without the registers, the shared memory and the uneven
+// load that the flux needs.  (By the size alone: the two forms round differently, and skipping
+// work that is exactly zero must not change a result.)
+__host__ __device__ inline bool v_pass(const SolveDev& s) { return (long long)s.NC * s.N * s.N >= kVPassPoints; }
+
+// what E3 does about the viscous flux (e3_body): keep = the inviscid flux stays downloadable
+__host__ __device__ inline int e3_visc(const SolveDev& s, bool keep) {
+  return !s.artiv && s.skip ? 0 : !v_pass(s) ? 1 : keep ? 2 : 0;
 }
 
 // does a stage only need its increment cR * resid, so that cR is folded into 1/J?
@@ -945,7 +1120,7 @@ __host__ __device__ inline bool e3_pre(const RKStage& rk, int update) {
 // PRE = e3_pre(rk, update): two bodies, since FP64 instructions that a stage does not need
 // would be predicated and still take their time
 template <int N, class O, bool PRE>
-__device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int epb, const RKStage& rk, int update, double* sm) {
+__device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int epb, const RKStage& rk, int update, int visc, double* sm) {
   constexpr int NS = D<N>::NS, NF1 = D<N>::NF1, NFP = D<N>::NFP;
   constexpr int NQ = 10;  // line quantities: eight flux components, two of A_z S
 
@@ -962,7 +1137,7 @@ __device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int 
   // point js (N+1) + is, which its xi line has consumed
   auto slot = [](int e, int p) { return e * NFP + p + p / N; };
   // the block's fluxes and state, copied while the rest of the inputs is read
-  block_copy_async(sF, s.Fc + (size_t)e0 * NFP * 8, cnt * NFP * 8);
+  block_copy_async(sF, (visc == 2 && !s.skip ? s.Ft : s.Fc) + (size_t)e0 * NFP * 8, cnt * NFP * 8);
   block_copy_async(sQ, s.Q + (size_t)e0 * NS * 9, cnt * NS * 9);
   cp_async_commit();
   {
@@ -983,9 +1158,20 @@ __device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int 
     }
   }
   cp_async_wait();
-  const int nact = active_cells(s, e0, cnt, 1, list);  // (ends with a barrier)
+  // the viscous flux: visc = 0 nothing left to do, 1 evaluated here, 2 by pass V, whose total
+  // fluxes replace those of the cells that have one
+  int nact = 0;
+  if (visc == 1 || (visc == 2 && s.skip)) nact = active_cells(s, e0, cnt, list);  // (ends with a barrier)
+  else __syncthreads();
   if (nact) {
-    e3_viscous<N, O>(s, e0, nact, list, sF);
+    if (visc == 1) {
+      e3_viscous<N, O>(s, e0, nact, list, sF, sU);  // (sU: free until the velocities)
+    } else {
+      for (int i = 0; i < nact; i++)
+        block_copy_async(sF + list[i] * NFP * 8, s.Ft + (size_t)(e0 + list[i]) * NFP * 8, NFP * 8);
+      cp_async_commit();
+      cp_async_wait();
+    }
     __syncthreads();
   }
   // divergence of the total flux and grad A_z in the conservative form of nablaAsp
@@ -1168,13 +1354,13 @@ __device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int 
 constexpr int e3_regs(int N) { return N == 5 ? 80 : 72; }
 
 template <int N, bool PRE>
-__global__ void __maxnreg__(e3_regs(N)) k_e3(const __grid_constant__ SolveDev s, const __grid_constant__ RKStage rk, int epb, int update, int c0, int c1) {
+__global__ void __maxnreg__(e3_regs(N)) k_e3(const __grid_constant__ SolveDev s, const __grid_constant__ RKStage rk, int epb, int update, int visc, int c0, int c1) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
   const int e0 = c0 + blockIdx.x * epb;
   const int cnt = min(epb, c1 - e0);
   if (cnt <= 0) return;
-  e3_body<N, OpsTU, PRE>(s, e0, cnt, epb, rk, update, sm);
+  e3_body<N, OpsTU, PRE>(s, e0, cnt, epb, rk, update, visc, sm);
 }
 
 // ---------------------------------------------------------------------------

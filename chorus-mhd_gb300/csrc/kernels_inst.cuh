@@ -17,9 +17,6 @@ constexpr int kN = CHORUS_N;
 inline size_t smem_e1(int epb) {
   return sizeof(double) * ((size_t)epb * (D<kN>::NS * 9 + 2 * D<kN>::NS + D<kN>::NFP * 9) + kN * kN);
 }
-inline size_t smem_e2(int epb) {
-  return sizeof(double) * ((size_t)epb * (D<kN>::NFP * 16 + D<kN>::NS * 17));
-}
 inline size_t smem_ct(int epb) { return sizeof(double) * epb * (D<kN>::NFP * 2 + D<kN>::NS * 2); }
 inline int grid_cells(int nc, int epb) { return (nc + epb - 1) / epb; }
 
@@ -47,6 +44,7 @@ void set_smem_limits() {
   const int lim = 200 * 1024;
   cudaFuncSetAttribute(k_e1<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_e2<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(k_v<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_f1<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_e3<kN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_e3<kN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
@@ -84,14 +82,15 @@ void launch_f1<kN>(const SolveDev& s, cudaStream_t st, int a2, int b2, int a1, i
     launch_pdl(k_f1<kN>, grid, thr, f1_smem(thr), st, s, a2 * kN, n2, (s.nface2 + a1) * kN, n);
 }
 template <>
-void launch_e2<kN>(const SolveDev& s, const Launch& L, cudaStream_t st) {
-  // chunks of up to one cell per thread, but small enough for about 16 CTAs per SM
+void launch_e2<kN>(const SolveDev& s, const Launch& L, cudaStream_t st, bool keep) {
+  // every cell: a CTA per group; a list of unknown length: eight CTAs per SM walk it
   const int nsm = sm_count();
-  int chunk = s.NC / (16 * nsm);
-  chunk = chunk < L.epb ? L.epb : (chunk > L.threads ? L.threads : chunk);
-  chunk -= chunk % L.epb;
-  if (!s.skip) chunk = L.epb;  // every cell needs its gradients: one group per CTA
-  launch_pdl(k_e2<kN>, grid_cells(s.NC, chunk), L.threads, smem_e2(L.epb), st, s, L.epb, chunk);
+  const int all2 = grid_cells(s.NC, L.epb);
+  launch_pdl(k_e2<kN>, s.skip ? std::min(all2, 8 * nsm) : all2, L.threads, e2_smem(kN, L.epb), st, s, L.epb, (int)keep);
+  if (v_pass(s) && (s.artiv || !s.skip)) {
+    const int allv = grid_cells(s.NC, v_epb(kN));
+    launch_pdl(k_v<kN>, s.skip ? std::min(allv, 8 * nsm) : allv, v_threads(kN), v_smem(kN), st, s, keep ? s.Ft : s.Fc);
+  }
 }
 template <>
 void launch_qavg<kN>(const SolveDev& s, cudaStream_t st) {
@@ -108,7 +107,8 @@ void launch_e3<kN>(const SolveDev& s, const RKStage& rk, const Launch& L, cudaSt
   const int update = (rk.cQ != 0.0 || rk.cR != 0.0 || rk.nsrc > 0) ? 1 : 0;
   if (c1 < 0) c1 = s.NC;
   if (c1 > c0)
-    launch_pdl(e3_pre(rk, update) ? k_e3<kN, true> : k_e3<kN, false>, grid_cells(c1 - c0, L.epb), L.threads, e3_smem(kN, L.epb), st, s, rk, L.epb, update, c0, c1);
+    launch_pdl(e3_pre(rk, update) ? k_e3<kN, true> : k_e3<kN, false>, grid_cells(c1 - c0, L.epb), L.threads,
+               e3_smem(kN, L.epb), st, s, rk, L.epb, update, e3_visc(s, rk.write_resid), c0, c1);
 }
 template <>
 void launch_ct<kN>(const SolveDev& s, const Launch& L, cudaStream_t st, int mode, int c0, int c1) {

@@ -177,3 +177,49 @@ def test_states_outside_the_integer_form_are_refused(driver, tmp_path):
     inner += [[*good[:8], v, v, good[19]] for v in (0.0, 1e-100, 1e100, np.nan)]
     out = evaluate(driver, tmp_path, 1, np.array([[*good[:8], 0.6, 0.8, good[19]]] + inner))
     assert out[0, 0] == 1 and np.all(out[1:, 0] == 0)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("coef", ["both", "viscous", "resistive"])
+def test_viscous_flux_against_extended_precision(driver, tmp_path, kind, coef):
+    """The scale leaves out factors of up to four (2 du/dx, two thirds of the divergence, two
+    terms to a sum): 2^-50 of it."""
+    rng = np.random.default_rng(200 + len(kind) + 50 * len(coef))
+    n, gam, Pr = 2000, 5.0 / 3, 0.72
+    q = states(rng, kind, n)
+    size = abs(q) + 0.1 * np.sqrt(q[:, :1]) * (kind not in ("tiny", "huge"))  # of the variables' gradients
+    size *= np.exp(rng.uniform(-4, 2, (n, 8)))
+    if kind in ("planar", "hydro"):
+        size[:, [3, 7]] = 0
+    if kind == "hydro":
+        size[:, 5:] = 0
+    G = size[:, None, :] * rng.uniform(-1, 1, (n, 2, 8))
+    th = rng.uniform(0, 2 * np.pi, n)
+    S = np.stack([np.cos(th), np.sin(th)], 1) * np.exp(rng.uniform(-8, 8, (n, 1)))
+    mu = 1e-3 * np.exp(rng.uniform(-2, 2, (n, 1))) * (coef != "resistive")
+    eta = 1e-3 * np.exp(rng.uniform(-2, 2, (n, 1))) * (coef != "viscous")
+    out = evaluate(driver, tmp_path, 2, np.concatenate([q, G.reshape(n, 16), mu, eta, S, np.full((n, 1), gam)], 1))
+    assert np.all(out[:, 0] == 1)
+    Q, D, M, H, N = (a.astype(LD) for a in (q, G, mu[:, 0], eta[:, 0], S))
+    rho, B, g = Q[:, 0], Q[:, 5:8], LD(gam)
+    u = Q[:, 1:4] / rho[:, None]
+    v2, b2 = (u * u).sum(1), (B * B).sum(1)
+    e = (Q[:, 4] - rho * v2 / 2 - b2 / 2) / rho
+    du = (D[:, :, 1:4] - D[:, :, :1] * u[:, None]) / rho[:, None, None]
+    de = (D[:, :, 4] - v2[:, None] / 2 * D[:, :, 0] - rho[:, None] * (u[:, None] * du).sum(2)
+          - (B[:, None] * D[:, :, 5:8]).sum(2) - D[:, :, 0] * e[:, None]) / rho[:, None]
+    div = du[:, 0, 0] + du[:, 1, 1]
+    txx, tyy, txy = 2 * du[:, 0, 0] - 2 * div / 3, 2 * du[:, 1, 1] - 2 * div / 3, du[:, 0, 1] + du[:, 1, 0]
+    tau = M[:, None] * np.stack([txx * N[:, 0] + txy * N[:, 1], txy * N[:, 0] + tyy * N[:, 1], (du[:, :, 2] * N).sum(1)], 1)
+    J = np.stack([D[:, 1, 7], -D[:, 0, 7], D[:, 0, 6] - D[:, 1, 5]], 1)
+    NJ = H[:, None] * np.stack([-J[:, 2] * N[:, 1], J[:, 2] * N[:, 0], J[:, 0] * N[:, 1] - J[:, 1] * N[:, 0]], 1)
+    heat = M * (g / LD(Pr)) * (de * N).sum(1)
+    F = np.concatenate([0 * tau[:, :1], tau, ((u * tau).sum(1) + heat + (B * NJ).sum(1))[:, None], NJ], 1)
+    s, V, b = np.sqrt((N * N).sum(1)), np.sqrt(v2), np.sqrt(b2)
+    gr, gm, gz, ge, gb, gw = (a.astype(LD) for a in (size[:, 0], np.hypot(size[:, 1], size[:, 2]), size[:, 3], size[:, 4],
+                                                     np.hypot(size[:, 5], size[:, 6]), size[:, 7]))
+    st, sz = M / rho * (gm + gr * V) * s, M / rho * (gz + gr * abs(u[:, 2])) * s
+    en = V * (st + sz) + M / rho * (g / LD(Pr)) * s * (ge + V * (gm + gz) + b * (gb + gw) + gr * (v2 + abs(Q[:, 4]) / rho)) \
+        + H * s * b * (gb + gw)
+    scale = np.stack([0 * s, st, st, sz, en, H * gb * s, H * gb * s, H * gw * s], 1)
+    assert np.all(abs(out[:, 1:9] - F) <= 2.0 ** -50 * scale)
