@@ -153,7 +153,7 @@ Launch default_launch(int N, int which) {
   // which: 0 = E1, 1 = E2, 2 = E3, 3 = CT; cells per CTA and threads per CTA as the
   // autotuner's sweep picked them on GB300 (2 M solution points); the CT passes take about
   // 128/(2N) cells so that their (cell, line) loop fills the 128 threads
-  static const int epb[kMaxN + 1][4] = {{0}, {0}, {16, 6, 16, 32}, {8, 4, 8, 21}, {4, 4, 6, 16},
+  static const int epb[kMaxN + 1][4] = {{0}, {0}, {16, 6, 16, 32}, {8, 4, 8, 21}, {4, 2, 6, 16},
                                         {4, 2, 5, 12}, {4, 2, 3, 10}, {2, 1, 3, 9}, {2, 1, 2, 8}};
   static const int thr[kMaxN + 1][4] = {{0}, {0}, {64, 96, 96, 128}, {96, 128, 96, 128}, {96, 128, 128, 128},
                                         {128, 128, 128, 128}, {160, 192, 128, 128}, {128, 128, 224, 128},

@@ -36,6 +36,18 @@ int sm_count() {
   return nsm_of[dev];
 }
 
+// Cells per CTA of a launch over n cells: the tuned number, or fewer where that leaves an SM
+// fewer than four CTAs, since the pass then lasts as long as one CTA takes for its cells.  A step
+// of all passes and the CT projection, tuned -> spread (us a step; GB300, without AV): N = 3,
+// 1024 cells 116 -> 96; N = 4, 784 cells 117 -> 103; N = 5, 576 cells 134 -> 107; N = 6, 256 cells
+// 140 -> 109; N = 8, 324 cells 150 -> 132; N = 5, 2304 cells 183 -> 175; N = 2, 10000 cells 161.
+// A line at six CTAs: N = 6, 1600 cells 177 instead of 191, but N = 8, 784 cells 184 against 168.
+// From four CTAs per SM on the tuned number is as good or better.
+inline int spread(int n, int epb) {
+  const int ctas = 4 * sm_count();
+  return std::max(1, std::min(epb, (n + ctas - 1) / ctas));
+}
+
 void set_smem_limits() {
   static bool done[64] = {false};
   int dev = 0;
@@ -64,7 +76,8 @@ template <>
 void launch_e1<kN>(const SolveDev& s, const Launch& L, cudaStream_t st, int plot, int c0, int c1) {
   const int sensor = (s.artiv ? (plot ? 3 : 1) : 0) | 4;  // 4: also reset the stage's wave speed
   if (c1 < 0) c1 = s.NC;
-  if (c1 > c0) launch_pdl(k_e1<kN>, grid_cells(c1 - c0, L.epb), L.threads, smem_e1(L.epb), st, s, L.epb, sensor, c0, c1);
+  const int epb = spread(c1 - c0, L.epb);
+  if (c1 > c0) launch_pdl(k_e1<kN>, grid_cells(c1 - c0, epb), L.threads, smem_e1(epb), st, s, epb, sensor, c0, c1);
 }
 void CHORUS_CAT(launch_e1_nosensor_n, CHORUS_N)(const SolveDev& s, const Launch& L, cudaStream_t st) {
   launch_pdl(k_e1<kN>, grid_cells(s.NC, L.epb), L.threads, smem_e1(L.epb), st, s, L.epb, 0, 0, s.NC);
@@ -106,9 +119,10 @@ template <>
 void launch_e3<kN>(const SolveDev& s, const RKStage& rk, const Launch& L, cudaStream_t st, int c0, int c1) {
   const int update = (rk.cQ != 0.0 || rk.cR != 0.0 || rk.nsrc > 0) ? 1 : 0;
   if (c1 < 0) c1 = s.NC;
+  const int epb = spread(c1 - c0, L.epb);
   if (c1 > c0)
-    launch_pdl(e3_pre(rk, update) ? k_e3<kN, true> : k_e3<kN, false>, grid_cells(c1 - c0, L.epb), L.threads,
-               e3_smem(kN, L.epb), st, s, rk, L.epb, update, e3_visc(s, rk.write_resid), c0, c1);
+    launch_pdl(e3_pre(rk, update) ? k_e3<kN, true> : k_e3<kN, false>, grid_cells(c1 - c0, epb), L.threads,
+               e3_smem(kN, epb), st, s, rk, epb, update, e3_visc(s, rk.write_resid), c0, c1);
 }
 template <>
 void launch_ct<kN>(const SolveDev& s, const Launch& L, cudaStream_t st, int mode, int c0, int c1) {
@@ -119,8 +133,8 @@ void launch_ct<kN>(const SolveDev& s, const Launch& L, cudaStream_t st, int mode
       launch_pdl(k_ct_face<kN>, (n + face_threads(n) - 1) / face_threads(n), face_threads(n), 0, st, s, c0, c1);
   } else {
     if (c1 < 0) c1 = s.NC;
-    if (c1 > c0)
-      launch_pdl(k_ct_elem<kN>, grid_cells(c1 - c0, L.epb), L.threads, smem_ct(L.epb), st, s, L.epb, mode, c0, c1);
+    const int epb = spread(c1 - c0, L.epb);
+    if (c1 > c0) launch_pdl(k_ct_elem<kN>, grid_cells(c1 - c0, epb), L.threads, smem_ct(epb), st, s, epb, mode, c0, c1);
   }
 }
 template <>

@@ -64,3 +64,16 @@ def test_batch_membership_changes_between_steps(case_root):
     assert np.abs(s0.state() - _alone(case_root, MIX[0], 5)).max() <= 1e-14 * 50
     ref1 = _alone(case_root, MIX[2], 6)
     assert np.abs(s1.state() - ref1).max() <= 1e-14 * np.abs(ref1).max()
+
+
+@pytest.mark.parametrize("N,nx,ny", [(2, 1, 1), (3, 19, 32), (3, 21, 29), (4, 42, 29), (5, 16, 38), (6, 29, 21), (8, 13, 47)])
+def test_small_meshes_equal_their_batched_form(case_root, N, nx, ny):
+    """Alone, a mesh too small to fill the device takes fewer cells per CTA than in a batch: the
+    same values to the last bit (cells do not depend on their grouping)."""
+    spec = dict(problem="orszag_tang", nx=nx, ny=ny, N=N, jitter=0.1, seed=N)
+    s = Solver(Mesh(make_case(case_root, **spec)))
+    b = Batch()
+    b.add(s)
+    b.step(3)
+    b.sync()
+    assert np.array_equal(s.state(), _alone(case_root, spec, 3))
