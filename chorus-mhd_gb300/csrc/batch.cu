@@ -138,16 +138,20 @@ __global__ void __launch_bounds__(v_threads(N)) kg_v(BatchDev b, int keep) {
   });
 }
 
-template <int N>
-__global__ void __maxnreg__(e3_regs(N)) kg_e3(BatchDev b, int stage) {
+// E3 of the solves whose stage record is of the kind PRE (e3_pre), in two kernels: with both
+// bodies in one the compiler spills in the line loops.  A composition of one scheme launches one of
+// them a stage.  Sixteen solves of 16 to 96 cells a side, N = 3..6: 3.39 ms a step with one kernel,
+// 3.33 with two, 3.31 with the eight registers more that the solve's descriptor in shared memory
+// wants (16 more: 3.45).
+template <int N, bool PRE>
+__global__ void __maxnreg__(e3_regs(N) + 8) kg_e3(BatchDev b, int stage) {
   extern __shared__ __align__(16) double sm[];
   __shared__ __align__(16) RKStage srk;
   pdl_wait();
   for_tiles(b, gidx(PE3, N), b.ctiles, [&](const int4& T, const SolveDev& s) {
     if (threadIdx.x == 0) srk = b.rk[stage * b.cap + T.x];
     __syncthreads();
-    if (e3_pre(srk, 1)) e3_body<N, OpsAll<N>, true>(s, T.y, T.z, T.z, srk, 1, e3_visc(s, false), sm);
-    else e3_body<N, OpsAll<N>, false>(s, T.y, T.z, T.z, srk, 1, e3_visc(s, srk.write_resid), sm);
+    if (e3_pre(srk, 1) == PRE) e3_body<N, OpsAll<N>, PRE>(s, T.y, T.z, T.z, srk, 1, e3_visc(s, srk.write_resid), sm);
   });
 }
 
@@ -197,12 +201,13 @@ static void pass_shapes(int nsm, const int (&epb)[4], const int (&threads)[4], P
   cudaFuncSetAttribute(kg_f1<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_e2<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_v<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(kg_e3<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(kg_e3<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(kg_e3<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_ct<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   // every pass kernel asks for the same shared-memory carveout, so that CTAs of the
   // concurrent order chains share an SM without reconfiguring it
-  const void* fns[7] = {(const void*)kg_e1<N>, (const void*)kg_f1<N>, (const void*)kg_e2<N>, (const void*)kg_v<N>,
-                        (const void*)kg_e3<N>, (const void*)kg_ct<N>, (const void*)kg_ctface<N>};
+  const void* fns[8] = {(const void*)kg_e1<N>, (const void*)kg_f1<N>, (const void*)kg_e2<N>, (const void*)kg_v<N>,
+                        (const void*)kg_e3<N, true>, (const void*)kg_e3<N, false>, (const void*)kg_ct<N>, (const void*)kg_ctface<N>};
   for (const void* f : fns)
     cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
   auto fill = [&](PassShape& p, const void* fn, int thr, int e, size_t smem) {
@@ -217,7 +222,7 @@ static void pass_shapes(int nsm, const int (&epb)[4], const int (&threads)[4], P
   fill(sh[PF1], (const void*)kg_f1<N>, kF1Threads, 0, f1_smem(kF1Threads));
   fill(sh[PE2], (const void*)kg_e2<N>, threads[1], epb[1], cell_smem_bytes(N, epb[1], 1));
   fill(sh[PV], (const void*)kg_v<N>, v_threads(N), v_epb(N), v_smem(N));
-  fill(sh[PE3], (const void*)kg_e3<N>, threads[2], epb[2], cell_smem_bytes(N, epb[2], 2));
+  fill(sh[PE3], (const void*)kg_e3<N, true>, threads[2], epb[2], cell_smem_bytes(N, epb[2], 2));
   fill(sh[PCT], (const void*)kg_ct<N>, threads[3], epb[3], cell_smem_bytes(N, epb[3], 3));
   fill(sh[PCTF], (const void*)kg_ctface<N>, 256, 0, 0);
 }
@@ -229,7 +234,10 @@ static void launch_pass(const BatchDev& a, int pass, const PassShape& p, cudaStr
     case PF1: launch_pdl(kg_f1<N>, p.grid, p.threads, p.smem, st, a); break;
     case PE2: launch_pdl(kg_e2<N>, p.grid, p.threads, p.smem, st, a, p.epb, arg); break;
     case PV: launch_pdl(kg_v<N>, p.grid, p.threads, p.smem, st, a, arg); break;
-    case PE3: launch_pdl(kg_e3<N>, p.grid, p.threads, p.smem, st, a, arg); break;
+    case PE3:  // arg: the stage, and above it the kinds of stage record present (bit 0: not e3_pre, bit 1: e3_pre)
+      if (arg & 16) launch_pdl(kg_e3<N, true>, p.grid, p.threads, p.smem, st, a, arg & 7);
+      if (arg & 8) launch_pdl(kg_e3<N, false>, p.grid, p.threads, p.smem, st, a, arg & 7);
+      break;
     case PCT: launch_pdl(kg_ct<N>, p.grid, p.threads, p.smem, st, a, arg); break;
     default: launch_pdl(kg_ctface<N>, p.grid, p.threads, 0, st, a); break;
   }
@@ -295,6 +303,7 @@ struct ChorusBatch {
   int4* d_ftiles = nullptr;
   int* d_gcount = nullptr;  // [kGroups] then d_goff [kGroups]
   RKStage* d_rk = nullptr;
+  unsigned char kinds[5][kMaxN + 1] = {}, graph_kinds[5][kMaxN + 1] = {};  // kinds of stage record: present, captured
   unsigned long long* d_eig = nullptr;
   unsigned int* d_err = nullptr;
   OrderShape shape[kMaxN + 1];
@@ -398,13 +407,17 @@ static int batch_rebuild(ChorusBatch* b) {
   }
   std::vector<SolveDev> sd(ns);
   std::vector<RKStage> rk((size_t)5 * b->cap_solves);
+  std::memset(b->kinds, 0, sizeof b->kinds);
   for (int i = 0; i < ns; i++) {
     sd[i] = b->slots[i].sd;
     sd[i].eig = b->d_eig + 2 * i;
     sd[i].err = b->d_err + i;
     RKStage r[5];
     rk_stage_records(sd[i], b->slots[i].dt, b->slots[i].k_stage, false, r);
-    for (int k = 0; k < 5; k++) rk[(size_t)k * b->cap_solves + i] = r[k];
+    for (int k = 0; k < 5; k++) {
+      rk[(size_t)k * b->cap_solves + i] = r[k];
+      if (b->slots[i].active) b->kinds[k][b->slots[i].N] |= e3_pre(r[k], 1) ? 2 : 1;
+    }
   }
   std::vector<int> counts(cnt, cnt + kGroups);
   counts.insert(counts.end(), off, off + kGroups);
@@ -426,8 +439,11 @@ static int batch_rebuild(ChorusBatch* b) {
   b->ftiles = 0;
   for (int N = kMinN; N <= kMaxN; N++) b->ftiles += cnt[gidx(PF1, N)];
   // the graph launches one CTA per tile as captured; more tiles than that (a new order, or
-  // a larger composition) need a new capture, fewer leave CTAs that find no tile
+  // a larger composition) or another kind of stage record need a new capture, fewer leave CTAs
+  // that find no tile
   bool grew = false;
+  for (int k = 0; k < 5; k++)
+    for (int N = kMinN; N <= kMaxN; N++) grew = grew || (b->kinds[k][N] & ~b->graph_kinds[k][N]);
   for (int g = 0; g < kGroups; g++) {
     b->cnt[g] = cnt[g];
     grew = grew || cnt[g] > b->graph_grid[g];
@@ -481,7 +497,8 @@ static void batch_enqueue_step(ChorusBatch* b) {
       pass(PF1, 0);
       pass(PE2, stage == 4 ? 1 : 0);
       pass(PV, stage == 4 ? 1 : 0);
-      pass(PE3, stage);
+      b->graph_kinds[stage][N] = b->kinds[stage][N];
+      pass(PE3, stage | b->kinds[stage][N] << 3);
     }
     pass(PCT, 0);
     pass(PCTF, 0);

@@ -77,3 +77,22 @@ def test_small_meshes_equal_their_batched_form(case_root, N, nx, ny):
     b.step(3)
     b.sync()
     assert np.array_equal(s.state(), _alone(case_root, spec, 3))
+
+
+def test_another_scheme_joins_a_captured_batch(case_root):
+    """A solve of the other RK scheme takes the place of one of the same size and order, so that
+    its stages are of a kind that the captured step does not launch."""
+    spec = dict(problem="orszag_tang", nx=9, ny=8, N=4, jitter=0.1, seed=8)
+    five = dict(spec, k_stage=5)
+    b = Batch()
+    s, f = (Solver(Mesh(make_case(case_root, **k))) for k in (spec, five))
+    slot = b.add(s)
+    b.step(2)
+    b.remove(slot)
+    b.add(f)
+    b.step(3)
+    b.add(s)
+    b.step(1)
+    b.sync()
+    assert np.array_equal(s.state(), _alone(case_root, spec, 3))
+    assert np.array_equal(f.state(), _alone(case_root, five, 4))
