@@ -101,6 +101,20 @@ static void make_ops(int N, const double* Lmat, const double* Mmat, const double
       for (int l = 0; l < N - 1; l++) a += lagrange(xsl, N - 1, l, Xs[i]) * lagrange(Xs, N, m, xsl[l]);
       o.A[i * N + m] = a;
     }
+  // what A takes away is the degree N-1 part of the N-point interpolant: its leading coefficient
+  // (a divided difference) times the polynomial that vanishes at the N-1 points
+  double top = 0.0;
+  for (int i = 0; i < N; i++) {
+    o.Ar[i] = o.Al[i] = 1.0;
+    for (int l = 0; l < N - 1; l++) o.Ar[i] *= Xs[i] - xsl[l];
+    for (int k = 0; k < N; k++)
+      if (k != i) o.Al[i] /= Xs[i] - Xs[k];
+    top = std::max(top, std::fabs(o.Ar[i]));
+  }
+  for (int i = 0; i < N; i++) {
+    o.Ar[i] /= top;
+    o.Al[i] *= top;
+  }
 }
 
 static int ensure_ops(int dev, int N, const double* Lmat, const double* Mmat, const double* Xs, const double* Xf) {
@@ -156,7 +170,7 @@ Launch default_launch(int N, int which) {
   static const int epb[kMaxN + 1][4] = {{0}, {0}, {16, 6, 16, 32}, {8, 4, 8, 21}, {4, 2, 6, 16},
                                         {4, 2, 5, 12}, {4, 2, 3, 10}, {2, 1, 3, 9}, {2, 1, 2, 8}};
   static const int thr[kMaxN + 1][4] = {{0}, {0}, {64, 96, 96, 128}, {96, 128, 96, 128}, {96, 128, 128, 128},
-                                        {128, 128, 128, 128}, {160, 192, 128, 128}, {128, 128, 224, 128},
+                                        {128, 128, 128, 128}, {160, 192, 128, 128}, {96, 128, 224, 128},
                                         {128, 128, 160, 128}};
   return Launch{epb[N][which], thr[N][which]};
 }

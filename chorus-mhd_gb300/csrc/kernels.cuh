@@ -64,6 +64,7 @@ struct OpsN {
   double L[(kMaxN + 1) * kMaxN];  // Lmat(N+1,N) column-major
   double M[(kMaxN + 1) * kMaxN];  // Mmat(N+1,N)
   double A[kMaxN * kMaxN];        // AV smoothing operator A[i*N+m] (projection to N-1 points and back)
+  double Ar[kMaxN], Al[kMaxN];    // A = 1 - Ar Al^T: the projection drops one polynomial
   double Xf[kMaxN + 1];
   double Xs[kMaxN];
   // Lmat split by the mirror symmetry of the points (Xs and Xf symmetric about 1/2):
@@ -305,10 +306,10 @@ __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int 
   double* sT = sQ + epb * NS * 9;     // [epb][NS]      sensor scratch
   double* sU = sT + epb * NS;         // [epb][NS]
   double* sV = sU + epb * NS;         // [epb][NFP][9]  flux-point values
-  double* sA = sV + epb * NFP * 9;    // AV smoothing operator (N, N)
+  double* sA = sV + epb * NFP * 9;    // [N] Ar; for variable 6 the AV smoothing operator (N, N)
   // all global traffic of the pass is contiguous block copies (coalesced)
   block_copy(sQ, s.Q + (size_t)e0 * NS * 9, cnt * NS * 9);
-  for (int i = threadIdx.x; i < N * N; i += blockDim.x) sA[i] = O::ops().A[i];
+  for (int i = threadIdx.x; i < N; i += blockDim.x) sA[i] = O::ops().Ar[i];
   __syncthreads();
   // interpolation to every flux point, one (cell, line, variable) per thread so that
   // every lane of every warp does work; the line operator runs on the integer pipes,
@@ -372,50 +373,60 @@ __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int 
   // AV sensor of variable 1 (AV.f90:15-82): Qsm = A rho A^T, sum ((Qsm-rho)/rho)^2.
   // Se = log10(sum) is compared with -6 and -1 only; the sum itself is kept (Se < -6
   // exactly when sum < 1e-6) and the logarithm is taken where the ramp needs it.
-  for (int t = threadIdx.x; t < cnt * NS; t += blockDim.x) {
-    const int e = t / NS, p = t - e * NS, is = p % N, n = p / N;
+  // With A = 1 - r l^T, Qsm - rho = -(r_i t_j + r_j u_i - r_i r_j w): t and u are the sums of
+  // l rho along the two families of lines and w that of l t, so a point takes 3 FP64
+  // operations where the products with A take 10 and a subtraction that cancels.  A few lanes of
+  // one warp sum a cell, so that a warp's FP64 instruction, which takes its time however many
+  // lanes are on, serves several cells.  The pass with the products and a warp per cell -> like
+  // this (ms a stage; GB300): 301x277 cells, N = 3 0.120 -> 0.104; 256x256, N = 4 0.143 -> 0.136;
+  // 512x512, N = 5 0.847 -> 0.836.
+  for (int t = threadIdx.x; t < cnt * 2 * N; t += blockDim.x) {
+    const int e = t / (2 * N), j = t - e * 2 * N;
+    const double* q = sQ + e * NS * 9 + (j < N ? j * N * 9 : (j - N) * 9);
+    const int qs = j < N ? 9 : N * 9;
+    double a = 0.0;
+#pragma unroll
+    for (int m = 0; m < N; m++) a += O::ops().Al[m] * q[m * qs];
+    sT[t] = a;  // [e][2N]: t, u
+  }
+  __syncthreads();
+  constexpr int LPC = N <= 2 ? 2 : N == 3 ? 4 : N <= 6 ? 8 : 16;  // lanes per cell
+  const int lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+  for (int t = threadIdx.x; t < cnt * LPC; t += blockDim.x) {
+    const int e = t / LPC, l = t - e * LPC;
     const double* q = sQ + e * NS * 9;
-    double a = 0.0;
+    const double* T = sT + e * 2 * N;
+    double w = 0.0;
 #pragma unroll
-    for (int m = 0; m < N; m++) a += sA[is * N + m] * q[(n * N + m) * 9];
-    sT[e * NS + p] = a;  // T(is, n)
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < cnt * NS; t += blockDim.x) {
-    const int e = t / NS, p = t - e * NS, is = p % N, js = p / N;
-    double a = 0.0;
-#pragma unroll
-    for (int n = 0; n < N; n++) a += sA[js * N + n] * sT[e * NS + n * N + is];
-    const double rho = sQ[(e * NS + p) * 9];
-    const double d = (a - rho) * rcp_pos(rho);
-    sU[e * NS + p] = d * d;
-  }
-  __syncthreads();
-  // one warp per cell sums its points
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  for (int e = warp; e < cnt; e += nwarp) {
+    for (int n = 0; n < N; n++) w += O::ops().Al[n] * T[n];
     double acc = 0.0;
-    for (int p = lane; p < NS; p += 32) acc += sU[e * NS + p];
-    acc = warp_sum(acc);
-    if (lane == 0) {
+#pragma unroll 1
+    for (int p = l; p < NS; p += LPC) {
+      const int i = p % N, j = p / N;
+      const double d = (sA[i] * T[j] + sA[j] * (T[N + i] - sA[i] * w)) * rcp_pos(q[p * 9]);
+      acc += d * d;
+    }
+    const unsigned group = (LPC == 32 ? 0xffffffffu : (1u << LPC) - 1) << (lane & ~(LPC - 1));
+#pragma unroll
+    for (int o = LPC / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(group, acc, o);
+    if (l == 0) {
       s.Se[e0 + e] = acc;
-      sU[e * NS] = acc;
       if (s.skip) {
-        const int a = (acc < 1e-6) ? 0 : 1;  // NaN counts as active
-        s.act[e0 + e] = a;
+        s.act[e0 + e] = (acc < 1e-6) ? 0 : 1;  // NaN counts as active
         s.nv[e0 + e] = 0;  // F1 marks the active cells and their face neighbours
         s.gr[e0 + e] = 0;
       }
+      // the AV ramp (log10 and sin) once per cell: in the pass that reads it for a cell and its
+      // four neighbours it took 14 us of a small mesh's stage
+      s.Sw[e0 + e] = av_ramp(acc);
     }
   }
-  // the AV ramp of the cells (log10 and sin, once per cell and by neighbouring lanes: in the pass
-  // that reads it for a cell and its four neighbours it took 14 us of a small mesh's stage)
-  __syncthreads();
-  for (int e = threadIdx.x; e < cnt; e += blockDim.x) s.Sw[e0 + e] = av_ramp(sU[e * NS]);
   if (!(sensor & 2)) return;
   // the same sensor of variable 6 (B_x), whose muAV(6) only the plot output reads
   // (tecplotter.f90:39 from AV.f90:60-73); in the reference's division form, so a zero
   // B_x gives the reference's inf or NaN
+  __syncthreads();
+  for (int i = threadIdx.x; i < N * N; i += blockDim.x) sA[i] = O::ops().A[i];
   __syncthreads();
   for (int t = threadIdx.x; t < cnt * NS; t += blockDim.x) {
     const int e = t / NS, p = t - e * NS, is = p % N, n = p / N;
@@ -435,7 +446,7 @@ __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int 
     sU[e * NS + p] = ((a - b) * (a - b)) / (b * b);
   }
   __syncthreads();
-  for (int e = warp; e < cnt; e += nwarp) {
+  for (int e = threadIdx.x >> 5; e < cnt; e += nwarp) {
     double acc = 0.0;
     for (int p = lane; p < NS; p += 32) acc += sU[e * NS + p];
     acc = warp_sum(acc);
