@@ -309,7 +309,8 @@ FIX_HD bool iflux_int(Q&& q, double sx, double sy, const IxGas& gas, Out&& out) 
 // Contravariant viscous, resistive and artificial-viscosity flux (vflux_contra, whose formulas
 // these are): q(k) the state, g(d, k) its gradient, mut and eta the viscosity and resistivity.
 // out(k, value) takes components 1..7; false, without output, where the integer form does not
-// apply.  [b] in the comments means a magnitude below 2^b.
+// apply.  The first output comes after the last use of q, which may therefore lie in the outputs'
+// place.  [b] in the comments means a magnitude below 2^b.
 template <class Q, class G, class Out>
 FIX_HD bool vflux_int(Q&& q, G&& g, double mut, double eta, double sx, double sy, const IxGas& gas, Out&& out) {
   const uint32_t zero = 66u << 20;  // a group of zeros: zeros are shifted out at this exponent

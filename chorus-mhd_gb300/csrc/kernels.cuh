@@ -711,10 +711,15 @@ __device__ __forceinline__ long long across(const SolveDev& s, int c, int fp) {
 // stage's sensor and epsilon0 = eigvmax h/(N-1) (AV.f90:147)
 template <int N>
 __device__ __forceinline__ double face_mu(const SolveDev& s, int c, int lf) {
-  const double eps0 = __longlong_as_double((long long)*s.eig) * s.hmsh / (double)(N - 1) * 1.0, h0 = eps0 / 2.0;
-  const double mc = h0 * s.Sw[c];
   const int o = (&s.nbr[c].x)[lf - 1];
-  return o >= 0 ? half(mc + h0 * s.Sw[o]) : mc;
+  const double rc = s.Sw[c], ro = o >= 0 ? s.Sw[o] : 0.0;
+  const long long eig = (long long)*s.eig;
+  // (no ramp and a finite wave speed: leave before the FP64 operations, which a warp's few lanes
+  // that come here do not share)
+  if (((__double_as_longlong(rc) | __double_as_longlong(ro)) << 1) == 0 && (unsigned)(eig >> 52) < 0x7ffu) return 0.0;
+  const double eps0 = __longlong_as_double(eig) * s.hmsh / (double)(N - 1) * 1.0, h0 = eps0 / 2.0;
+  const double mc = h0 * rc;
+  return o >= 0 ? half(mc + h0 * ro) : mc;
 }
 
 template <int N>
@@ -749,7 +754,7 @@ __device__ __forceinline__ void e2_cells(const SolveDev& s, const int* cells, in
   // flux-point states with the metric terms, differentiated along the lines on the integer
   // pipes as in E3.  The products are integers too: a line's states aligned once serve both
   // metric entries.  (128x128 cells, N = 5, every cell: 0.173 ms a stage with the products, the
-  // family sums and 1/J in FP64, 0.138 ms like this.)  An
+  // family sums and 1/J in FP64, 0.125 ms like this.)  An
   // operand is cut at 2^-58 of its line's largest, a product at 2^-61.
   constexpr int NS = D<N>::NS, NF1 = D<N>::NF1, NFP = D<N>::NFP;
   double* sQ = sm;                                              // [n][NFP][9] Q
@@ -774,19 +779,18 @@ __device__ __forceinline__ void e2_cells(const SolveDev& s, const int* cells, in
   for (int i = threadIdx.x; i < n * 2 * N; i += blockDim.x) {
     const int le = i / (2 * N), l = i - le * 2 * N;
     const double2* met = reinterpret_cast<const double2*>(s.met) + (size_t)cells[le] * NFP;
+    double2 a[N + 1];
     uint32_t m = 0;
-#pragma unroll 1
-    for (int r = 0; r <= N; r++) {
-      const double2 a = met[line_point(l, r)];
-      m = ix_max(m, ix_max(ix_abs_word(a.x), ix_abs_word(a.y)));
-    }
+#pragma unroll
+    for (int r = 0; r <= N; r++) a[r] = met[line_point(l, r)];
+#pragma unroll
+    for (int r = 0; r <= N; r++) m = ix_max(m, ix_max(ix_abs_word(a[r].x), ix_abs_word(a[r].y)));
     sM[i] = m >= kIxLow && m < kIxHigh ? ix_exp<4>(m) : kE3Fp64;
-#pragma unroll 1
+#pragma unroll
     for (int r = 0; r <= N; r++) {
-      const double2 a = met[line_point(l, r)];
       Limbs* o = sS + (le * NFP + line_point(l, r)) * 2;
-      o[0] = ix_limbs(ix_align<4>(a.x, m));
-      o[1] = ix_limbs(ix_align<4>(a.y, m));
+      o[0] = ix_limbs(ix_align<4>(a[r].x, m));
+      o[1] = ix_limbs(ix_align<4>(a[r].y, m));
     }
   }
   cp_async_wait();
@@ -926,13 +930,15 @@ __global__ void __launch_bounds__(512, 2) k_e2(const __grid_constant__ SolveDev 
 // Fc's place or (where the inviscid flux stays downloadable) beside it (interfaceVISflux /
 // BCVISFLUX / CYCLOCVISFLUX, comp_viscous_flux).  One flux point per thread with the integer
 // form of the flux; the FP64 form inside E3 kept that pass at 0.37 ms over its inviscid time
-// (128x128 cells, N = 5, every cell viscous), V takes 0.171 ms.  Bound by instruction issue
-// (43%) and the loads of Q and grad Q (292 MB, 1.7 TB/s) about equally.
+// (128x128 cells, N = 5, every cell viscous), V takes 0.148 ms.  Bound by latency with the integer
+// issue (49%), the FP64 pipe (54%: averages, conversions) and the loads of Q and grad Q (292 MB,
+// 2.0 TB/s) all about half used: 27 doubles of shared memory a point (the flux in the place of
+// the state) and 64 registers for eight CTAs per SM, against 0.171 ms with 36 and 72 for six.
 // ---------------------------------------------------------------------------
 // cells per group and threads per CTA: one flux point per thread
 constexpr int v_epb(int N) { return N >= 6 ? 1 : 128 / (2 * (N + 1) * N); }
 constexpr int v_threads(int N) { return (v_epb(N) * 2 * (N + 1) * N + 31) / 32 * 32; }
-constexpr size_t v_smem(int N) { return (size_t)v_epb(N) * 2 * (N + 1) * N * 36 * 8; }
+constexpr size_t v_smem(int N) { return (size_t)v_epb(N) * 2 * (N + 1) * N * 27 * 8; }
 
 // the viscosity of flux point fp of a cell with AV viscosities mf[4] on its local faces 1..4:
 // mu + the AV viscosity, linear between the faces
@@ -942,6 +948,7 @@ __device__ __forceinline__ double point_mu(const SolveDev& s, const double* mf, 
   if (!s.artiv) return s.mu;
   const double x = O::ops().Xf[fp < NF1 ? fp % (N + 1) : (fp - NF1) / N];
   const double a = fp < NF1 ? mf[3] : mf[0], b = fp < NF1 ? mf[1] : mf[2];
+  if (((__double_as_longlong(a) | __double_as_longlong(b)) << 1) == 0) return s.mu;
   return s.mu + (a * (1.0 - x) + b * x);
 }
 
@@ -959,8 +966,7 @@ template <int N, class O>
 __device__ __forceinline__ void v_cells(const SolveDev& s, const int* cells, int n, double* Ft, double* sm) {
   constexpr int NFP = D<N>::NFP;
   double* sG = sm;                // [n][NFP][18] grad Q
-  double* sQ = sG + n * NFP * 18;  // [n][NFP][9] Q
-  double* sV = sQ + n * NFP * 9;   // [n][NFP][9] the viscous flux (components 1..7)
+  double* sQ = sG + n * NFP * 18;  // [n][NFP][9] Q, then the viscous flux (components 1..7)
   for (int le = 0; le < n; le++) {
     block_copy_async(sG + le * NFP * 18, s.nQvf + (size_t)cells[le] * NFP * 18, NFP * 18);
     block_copy_async(sQ + le * NFP * 9, s.Qvf + (size_t)cells[le] * NFP * 9, NFP * 9);
@@ -993,16 +999,17 @@ __device__ __forceinline__ void v_cells(const SolveDev& s, const int* cells, int
     const double mut = point_mu<N, O>(s, smu[le], fp);
     volatile double* q = sQ + 9 * t;
     const volatile double* gr = sG + 18 * t;
+    // (the flux takes the place of the point's state, which vflux_int has read by its first output)
     if (!vflux_int([&](int k) { return q[k]; }, [&](int d, int k) { return gr[9 * d + k]; }, mut, s.eta0, m.x, m.y, s.gas,
-                   [&](int k, double f) { sV[t * 9 + k] = f; }))
-      vflux_fp64(sQ + 9 * t, sG + 18 * t, mut, s.eta0, s.gam, m.x, m.y, sV + 9 * t);
+                   [&](int k, double f) { q[k] = f; }))
+      vflux_fp64(sQ + 9 * t, sG + 18 * t, mut, s.eta0, s.gam, m.x, m.y, sQ + 9 * t);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < n * NFP * 4; i += blockDim.x) {
     const int t = i >> 2, j = i & 3, le = t / NFP;
     const size_t g = ((size_t)cells[le] * NFP + (t - le * NFP)) * 8 + 2 * j;
     const double2 a = *reinterpret_cast<const double2*>(s.Fc + g);
-    *reinterpret_cast<double2*>(Ft + g) = make_double2(j ? a.x - sV[9 * t + 2 * j] : a.x, a.y - sV[9 * t + 2 * j + 1]);
+    *reinterpret_cast<double2*>(Ft + g) = make_double2(j ? a.x - sQ[9 * t + 2 * j] : a.x, a.y - sQ[9 * t + 2 * j + 1]);
   }
 }
 
@@ -1021,7 +1028,7 @@ __device__ __forceinline__ void v_all(const SolveDev& s, int first, int stride, 
 }
 
 template <int N>
-__global__ void __launch_bounds__(v_threads(N)) k_v(const __grid_constant__ SolveDev s, double* Ft) {
+__global__ void __maxnreg__(64) k_v(const __grid_constant__ SolveDev s, double* Ft) {
   extern __shared__ __align__(16) double sm[];
   pdl_wait();
   v_all<N, OpsTU>(s, blockIdx.x, gridDim.x, Ft, sm);
