@@ -1,9 +1,9 @@
 // batch.cu -- many independent solves of mixed size and order advanced together:
 // one launch per pass for the whole ensemble.
 //
-// Each pass is one launch per order N present in the batch: a persistent kernel (a grid
-// of CTAs sized by occupancy to fill the GPU) specialised for N, with the launch shape
-// tuned for N, walking that order's tiles with a static stride.  A cell tile is
+// Each pass is one launch per order N present in the batch (E3 one per kind of stage record):
+// a kernel specialised for N, with the launch shape tuned for N and a CTA per tile of that
+// order.  A cell tile is
 // (solve, first cell, cells), a face tile (solve, first face point, points); the kernel
 // copies the tile's solve descriptor to shared memory and runs the same per-N pass body
 // as the single-solve kernels, so a solve gives the same bits alone and in a batch.
@@ -201,8 +201,8 @@ static void pass_shapes(int nsm, const int (&epb)[4], const int (&threads)[4], P
   cudaFuncSetAttribute(kg_f1<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_e2<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(kg_v<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(kg_e3<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(kg_e3<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(kg_e3<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, e3_smem_limit(N));
+  cudaFuncSetAttribute(kg_e3<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, e3_smem_limit(N));
   cudaFuncSetAttribute(kg_ct<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   // every pass kernel asks for the same shared-memory carveout, so that CTAs of the
   // concurrent order chains share an SM without reconfiguring it

@@ -1,27 +1,27 @@
 // kernels.cuh -- stage kernels of the residual-and-time-step path, templated on N.
 //
 // One RK stage (compresid.f90:1-67 + the stage update of iterations.f90:162-217) is
-// four launches, one per grid-wide dependency level of the reference's compflux:
+// four launches (five on large meshes), one per grid-wide dependency level of the reference's
+// compflux:
 //   E1  cell pass  Q -> flux-point values (all 2N(N+1) points), interior inviscid
-//                  flux, interior A_z, AV sensor           inviscid_flux_interior,
+//                  flux, interior A_z, AV sensor and ramp  inviscid_flux_interior,
 //                                                          comp_artificial_viscosity
-//   F1  face pass  Rusanov flux on every face point, upwinded A_z, face-averaged Q,
-//                  max wave speed                          interfaceflux, CYCLOCFLUX,
+//   F1  face pass  Rusanov flux on every face point, upwinded A_z, max wave speed,
+//                  list of the cells with viscous work     interfaceflux, CYCLOCFLUX,
 //                                                          BCFLUX, getrusanovflux
-//   E2  cell pass  face AV viscosities; grad Q (vars 1-8) at the solution and flux
-//                  points of the cells that carry viscous work
-//                                                          compAVflux, nablaQsp,
-//                                                          nablaQ_interior_FP
-//   E3  cell pass  viscous + AV flux with the face-averaged grad Q traces, divergence,
-//                  grad A_z, A_z advection, RK update      interfaceVISflux,
-//                                                          comp_viscous_flux, nablaAsp,
-//                                                          compresid, RK_S5P3
+//   E2  cell pass  grad Q (vars 1-8) at the solution and flux points of the listed cells
+//                  and their neighbours                    nablaQsp, nablaQ_interior_FP
+//   V   cell pass  face AV viscosities, viscous + AV flux of the listed cells with the
+//                  face-averaged traces                    compAVflux, interfaceVISflux,
+//                                                          comp_viscous_flux
+//   E3  cell pass  (V's work on small meshes,) divergence, grad A_z, A_z advection, RK
+//                  update                                  nablaAsp, compresid, RK_S5P3
 // (k_f2 stores the face-averaged grad Q traces only when they are downloaded.)
 // Cell passes stage a block of `epb` cells in shared memory; face passes run one
 // thread per face point.  Values are IEEE doubles throughout; the fixed line operators
 // (Lmat interpolation, Mmat differentiation, which carry no data-dependent
-// coefficients) run as exact integer dot products on the integer pipes (fixdot.cuh),
-// all other arithmetic is FP64.
+// coefficients) run as exact integer dot products on the integer pipes (fixdot.cuh), the
+// point fluxes in block fixed point there too (intflux.cuh), all other arithmetic is FP64.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -338,8 +338,8 @@ __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int 
   // contravariant inviscid flux at the interior flux points only (face points of Fc and
   // Azf belong to the face pass), one point per thread, in the place of the point's state
   // 512x512 cells, N = 5 (GB300): the pass took 1.14 ms a stage with 40 FP64 operations a point
-  // (84% of that pipe), 0.84 ms with some 700 integer instructions (issue slots 66% busy, the
-  // FP64 pipe 34% with the sensor).  A quarter of the points left in FP64 form beside them:
+  // (84% of that pipe), 0.84 ms with some 700 integer instructions (issue slots 61% busy, the
+  // FP64 pipe 45% with conversions and sensor).  A quarter of the points left in FP64 form beside them:
   // 0.92 ms (part-filled warps in two loops).  64 registers (32 warps per SM): 0.95 ms at 80,
   // 1.06 at 96 without the spill of 28 bytes.
   for (int t = threadIdx.x; t < cnt * NINT; t += blockDim.x) {
@@ -596,7 +596,7 @@ __device__ __forceinline__ unsigned long long f1_points(const SolveDev& s, int f
 #pragma unroll 1
   for (int i0 = first; i0 < n; i0 += step) {
     const int next = slot == 2 ? 0 : slot + 1, i = i0 + lane;
-    cp_async_wait();  // this round's traces, the next round's records
+    cp_async_wait();  // this turn's traces, the next turn's records
     __syncwarp();
     fetch_data(i + step, next, buf ^ 1);
     fetch_rec(i + 2 * step, next == 2 ? 0 : next + 1);
@@ -1115,6 +1115,14 @@ static __device__ __noinline__ void e3_viscous(const SolveDev& s, int e0, int na
 // shared memory of the pass for epb cells (e3_body)
 constexpr size_t e3_smem(int N, int epb) {
   return (size_t)epb * ((size_t)2 * (N + 1) * N * 10 * 8 + (size_t)N * N * (72 + 16 + 8 + 4) + (size_t)N * 10 * 4) + 16;
+}
+
+// The most of it that a launch may ask for: 200 kB, or what as many cells take as fitted into 200 kB
+// while a cell's exponents were not kept (42 of N = 4 want 1.7% more).
+constexpr int e3_smem_limit(int N) {
+  const int cells = 200 * 1024 / (8 * (20 * (N + 1) * N + 13 * N * N));
+  const size_t need = e3_smem(N, cells < 64 ? cells : 64);
+  return need > 200 * 1024 ? (int)need : 200 * 1024;
 }
 
 constexpr long long kVPassPoints = 49152;

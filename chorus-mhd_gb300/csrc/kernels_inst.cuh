@@ -58,8 +58,8 @@ void set_smem_limits() {
   cudaFuncSetAttribute(k_e2<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_v<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_f1<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_e3<kN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-  cudaFuncSetAttribute(k_e3<kN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+  cudaFuncSetAttribute(k_e3<kN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, e3_smem_limit(kN));
+  cudaFuncSetAttribute(k_e3<kN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, e3_smem_limit(kN));
   cudaFuncSetAttribute(k_ct_elem<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_diag_interp<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
   cudaFuncSetAttribute(k_nqsp<kN>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);

@@ -79,3 +79,17 @@ def test_skipping_and_batch_change_nothing(case_root, size, share):
     assert np.all(np.isfinite(out[0]))
     assert np.array_equal(out[0], out[1])
     assert np.array_equal(members[0].state(), out[0])
+
+
+@pytest.mark.parametrize("N,side,epb", [(2, 200, 64), (4, 164, 42), (5, 130, 27), (8, 84, 11)])
+def test_most_cells_per_cta_of_the_last_pass(case_root, N, side, epb):
+    """The largest option values that fit the shared memory give the same bits as the tuned one."""
+    d = make_case(case_root, **spec(N, side, side))
+    out = []
+    for e in (None, epb):
+        s = Solver(Mesh(d))
+        if e:
+            s.set_option("epb_e3", e)
+        s.iterations(1)
+        out.append(s.state())
+    assert np.array_equal(out[0], out[1])
