@@ -48,6 +48,22 @@ inline int spread(int n, int epb) {
   return std::max(1, std::min(epb, (n + ctas - 1) / ctas));
 }
 
+// The same for E3, whose loops are over the 10 N line quantities of a cell and family: on a
+// launch of few CTAs, down to half as many cells, the number whose lines fill the threads best,
+// since little covers a CTA's part-filled last turn there.
+// Tuned -> this (us a step; GB300): N = 6, 3969 cells 338 -> 321, 1600 cells 185 -> 179; N = 3, 8100
+// cells 197 -> 189; N = 2, 10000 cells 162 -> 158.  From some 12 CTAs per SM on the bigger CTAs
+// are as good or better: N = 3, 19600 cells (16 per SM) 400 -> 403; N = 2, 32400 cells (13) 345 -> 348.
+inline int e3_cells(int n, const Launch& L) {
+  const int epb = spread(n, L.epb), lines = 10 * kN;
+  if (grid_cells(n, epb) >= 12 * sm_count()) return epb;
+  auto idle = [&](int e) { return (e * lines + L.threads - 1) / L.threads * L.threads / (double)(e * lines); };
+  int best = epb;
+  for (int e = epb - 1; 2 * e > epb; e--)
+    if (idle(e) < idle(best)) best = e;
+  return best;
+}
+
 void set_smem_limits() {
   static bool done[64] = {false};
   int dev = 0;
@@ -119,7 +135,7 @@ template <>
 void launch_e3<kN>(const SolveDev& s, const RKStage& rk, const Launch& L, cudaStream_t st, int c0, int c1) {
   const int update = (rk.cQ != 0.0 || rk.cR != 0.0 || rk.nsrc > 0) ? 1 : 0;
   if (c1 < 0) c1 = s.NC;
-  const int epb = spread(c1 - c0, L.epb);
+  const int epb = e3_cells(c1 - c0, L);
   if (c1 > c0)
     launch_pdl(e3_pre(rk, update) ? k_e3<kN, true> : k_e3<kN, false>, grid_cells(c1 - c0, epb), L.threads,
                e3_smem(kN, epb), st, s, rk, epb, update, e3_visc(s, rk.write_resid), c0, c1);

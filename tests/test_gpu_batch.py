@@ -66,7 +66,8 @@ def test_batch_membership_changes_between_steps(case_root):
     assert np.abs(s1.state() - ref1).max() <= 1e-14 * np.abs(ref1).max()
 
 
-@pytest.mark.parametrize("N,nx,ny", [(2, 1, 1), (3, 19, 32), (3, 21, 29), (4, 42, 29), (5, 16, 38), (6, 29, 21), (8, 13, 47)])
+@pytest.mark.parametrize("N,nx,ny", [(2, 1, 1), (3, 19, 32), (3, 21, 29), (4, 42, 29), (5, 16, 38), (6, 29, 21), (8, 13, 47),
+                                     (2, 152, 191), (2, 152, 192), (3, 121, 120), (6, 76, 72), (6, 72, 77)])
 def test_small_meshes_equal_their_batched_form(case_root, N, nx, ny):
     """Alone, a mesh too small to fill the device takes fewer cells per CTA than in a batch: the
     same values to the last bit (cells do not depend on their grouping)."""
