@@ -158,7 +158,7 @@ FIX_HD int64_t ix_sqrt(int64_t v, int e, int& es) {
 FIX_HD int64_t ix_shift(int64_t v, int d) { return d >= 0 ? ix_shr(v, d) : ix_shl(v, -d); }
 
 // leading zeros of |v| among the upper 32 bits, less `keep`: a left shift by that many bits
-// (at least 0) leaves |v| < 2^(63 - keep)
+// (at least 0) leaves |v| <= 2^(64 - keep)
 FIX_HD int ix_room(int64_t v, int keep) {
   const int hi = (int)(v >> 32);
   const uint32_t a = (uint32_t)(hi ^ (hi >> 31));
@@ -168,6 +168,62 @@ FIX_HD int ix_room(int64_t v, int keep) {
   return ix_max((a ? __builtin_clz(a) : 32) - keep, 0);
 #endif
 }
+
+// ---------------------------------------------------------------------------
+// Values with an exponent of their own.  Every variable of a state, every component of a normal
+// and every product carries one, so that a small component beside a large one keeps all its bits
+// as it does in FP64 (with one exponent for the components of the plane a transverse flux of
+// 10^-8 of the main one was left with 29 bits); only the terms of a sum are aligned, to the
+// largest of them.  [b] in the comments means a magnitude of at most 2^b.
+// ---------------------------------------------------------------------------
+struct IxF {  // an operand: m 2^e, [61]
+  Limbs m;
+  int e;
+};
+struct IxV {  // a product or a sum: v 2^e
+  int64_t v;
+  int e;
+};
+
+constexpr uint32_t kIxLow = 823u << 20, kIxHigh = 1223u << 20;  // 2^-200 .. 2^200
+constexpr uint32_t kIxZero = 66u << 20;  // magnitude words below: a zero
+
+// x without rounding, 2^60 <= |m| < 2^61; both limbs carry the sign.  A zero gets the exponent of
+// kIxZero, which no sum aligns to
+FIX_HD IxF ix_load(double x) {
+  const uint64_t u = fix_bits(x);
+  const uint32_t hi = (uint32_t)(u >> 32), lo = (uint32_t)u, a = hi & 0x7fffffffu;
+  const int s = a < kIxZero ? 0 : (int)hi < 0 ? -1 : 1;
+  const int h = (int)((((hi << 9) | (lo >> 23)) & 0x3fffffffu) | 0x20000000u), l = (int)((lo << 8) & 0x7fffffffu);
+  return IxF{Limbs{h * s, l * s}, (int)(ix_max(a, kIxZero) >> 20) - 1083};
+}
+// 1/x of a positive normal x
+FIX_HD IxF ix_inverse(double x) {
+  const uint64_t u = fix_bits(x);
+  return IxF{ix_limbs(ix_rcp((int64_t)(((u << 11) | 0x8000000000000000ull) >> 2))), 962 - (int)(u >> 52)};
+}
+FIX_HD IxV ix_whole(IxF a) { return IxV{(int64_t)a.m.h * ((int64_t)1 << 31) + a.m.l, a.e}; }
+FIX_HD IxF ix_split(IxV a) { return IxF{ix_limbs(a.v), a.e}; }          // of [61.6] at most
+FIX_HD IxV ix_times(IxF a, IxF b) { return IxV{ix_mul(a.m, b.m), a.e + b.e + 62}; }  // [60], off by two units
+FIX_HD IxV ix_square(IxF a) {                                          // [60]
+  return IxV{fix_mad(a.m.h, a.m.h, fix_mad(a.m.h, a.m.l, 0) >> 30), 2 * a.e + 62};
+}
+FIX_HD int64_t ix_at(IxV a, int K) { return ix_shr(a.v, K - a.e); }  // a in units of 2^K, K >= a.e
+FIX_HD IxV ix_plus(IxV a, IxV b) {
+  const int K = ix_max(a.e, b.e);
+  return IxV{ix_at(a, K) + ix_at(b, K), K};
+}
+FIX_HD IxV ix_minus(IxV a, IxV b) {
+  const int K = ix_max(a.e, b.e);
+  return IxV{ix_at(a, K) - ix_at(b, K), K};
+}
+FIX_HD IxV ix_halved(IxV a) { return IxV{a.v >> 1, a.e + 1}; }  // the same value in one bit less
+// an operand of full length (up to 29 leading zeros are shifted out)
+FIX_HD IxF ix_up(IxV a) {
+  const int n = ix_room(a.v, 3);
+  return IxF{ix_limbs(ix_shl(a.v, n)), a.e - n};
+}
+FIX_HD double ix_double(IxV a) { return ix_double(a.v, a.e); }
 
 // limbs of v shifted up to [60] where it is below that, with its exponent; and of a pair
 FIX_HD Limbs ix_up(int64_t v, int& e) {
@@ -206,7 +262,6 @@ FIX_HD IxGas ix_gas(double gamma) {
   return c;
 }
 
-constexpr uint32_t kIxLow = 823u << 20, kIxHigh = 1223u << 20;  // 2^-200 .. 2^200
 
 // a product as an increment of a sum: (a b) >> 61
 FIX_HD int64_t ix_prod(Limbs a, Limbs b) {
@@ -217,92 +272,53 @@ FIX_HD int64_t ix_prod(Limbs a, Limbs b) {
 
 // Contravariant ideal-MHD flux F sx + G sy (iflux_contra); q(k) reads variable k, out(j, a, b)
 // takes components 2 j and 2 j + 1.  Returns false, without output, where the integer form does
-// not apply.  [b] in the comments means a magnitude below 2^b.
+// not apply.  Every term of a component's sum is off by less than 2^-54 of itself (three products
+// of operands of full length in a row).
 template <class Q, class Out>
 FIX_HD bool iflux_int(Q&& q, double sx, double sy, const IxGas& gas, Out&& out) {
-  const uint32_t zero = 66u << 20;  // a group of zeros: zeros are shifted out at this exponent
   const uint32_t r = (uint32_t)(fix_bits(q(0)) >> 32), me = ix_abs_word(q(4));  // r: huge if the sign is set
-  const uint32_t mm = ix_max(zero, ix_max(ix_abs_word(q(1)), ix_abs_word(q(2)))), mz = ix_max(zero, ix_abs_word(q(3)));
-  const uint32_t mb = ix_max(zero, ix_max(ix_abs_word(q(5)), ix_abs_word(q(6)))), mw = ix_max(zero, ix_abs_word(q(7)));
+  const uint32_t mz = ix_max(ix_abs_word(q(3)), ix_abs_word(q(7)));
+  const uint32_t mp = ix_max(ix_max(ix_abs_word(q(1)), ix_abs_word(q(2))), ix_max(ix_abs_word(q(5)), ix_abs_word(q(6))));
   const uint32_t ms = ix_max(ix_abs_word(sx), ix_abs_word(sy));
-  const uint32_t top = ix_max(ix_max(ix_max(r, me), ix_max(mm, mz)), ix_max(ix_max(mb, mw), ms));
-  if (top >= kIxHigh || r < kIxLow || me < kIxLow || ms < kIxLow) return false;
-  const int em = ix_exp<4>(mm), emz = ix_exp<4>(mz), eB = ix_exp<4>(mb), eBz = ix_exp<4>(mw), eE = ix_exp<3>(me);
-  const int eS = ix_exp<4>(ms), e_ri = -122 - ix_exp<2>(r);
-  const bool hasz = ix_max(mz, mw) != zero;
-  const Limbs nx = ix_limbs(ix_align<4>(sx, ms)), ny = ix_limbs(ix_align<4>(sy, ms));         // [60]
-  const Limbs mx = ix_limbs(ix_align<4>(q(1), mm)), my = ix_limbs(ix_align<4>(q(2), mm));     // [60]
-  const int64_t vby = ix_align<4>(q(6), mb);
-  const Limbs bx = ix_limbs(ix_align<4>(q(5), mb)), by = ix_limbs(vby);
-  const Limbs ri = ix_limbs(ix_rcp(ix_align<2>(q(0), r)));  // [61]
-  // mass flux, normal velocity
-  IxSum f;
-  f.add(mx, nx); f.add(my, ny);
-  const int64_t f0 = f.value4();  // [60.5]
-  const int eF0 = em + eS + 60;
-  const double F0 = ix_double(f0, eF0);
-  int64_t v = ix_mul(f0, ri);
-  const int nV = ix_room(v, 3), eV = eF0 + e_ri + 62 - nV;  // (slow flows keep their bits)
-  const Limbs V = ix_limbs(ix_shl(v, nV));                  // [60]
-  // v Bx - u By
-  IxSum w;
-  w.add(my, bx); w.add(mx, ix_limbs(-vby));
-  const Limbs W = ix_limbs(ix_mul(w.value4(), ri));
-  const int eW = em + eB + 60 + e_ri + 62;
-  // normal field, also over rho
-  IxSum b;
-  b.add(bx, nx); b.add(by, ny);
-  const int64_t bn = b.value4();  // [60.5]
-  const Limbs Bn = ix_limbs(bn), bnl = ix_limbs(ix_mul(bn, ri));
-  const int eBn = eB + eS + 60, ebn = eBn + e_ri + 62;
-  IxSum k2, b2, mB;
-  k2.square(mx); k2.square(my);
-  b2.square(bx); b2.square(by);
-  mB.add(mx, bx); mB.add(my, by);
-  int64_t kv = k2.value4_squares(), bv = b2.value4_squares(), mBv = mB.value4();  // [61]
-  int ek = 2 * em + 60, eB2 = 2 * eB + 60, emB = em + eB + 60;
+  if (ix_max(ix_max(ix_max(r, me), ix_max(mp, mz)), ms) >= kIxHigh || r < kIxLow || me < kIxLow || ms < kIxLow) return false;
+  const bool hasz = mz >= kIxZero;
+  const IxF nx = ix_load(sx), ny = ix_load(sy), mx = ix_load(q(1)), my = ix_load(q(2));
+  const IxF bx = ix_load(q(5)), by = ix_load(q(6)), ri = ix_inverse(q(0));
+  // mass flux, normal velocity (normal field the same), v Bx - u By
+  const IxV f0 = ix_plus(ix_times(mx, nx), ix_times(my, ny));  // [61]
+  const double F0 = ix_double(f0);
+  const IxF V = ix_up(ix_times(ix_split(f0), ri));
+  const IxF Bn = ix_up(ix_plus(ix_times(bx, nx), ix_times(by, ny))), bnl = ix_split(ix_times(Bn, ri));
+  const IxF W = ix_up(ix_times(ix_split(ix_minus(ix_times(my, bx), ix_times(mx, by))), ri));
+  IxV k2 = ix_plus(ix_square(mx), ix_square(my)), b2 = ix_plus(ix_square(bx), ix_square(by));  // [61]
+  IxV mB = ix_plus(ix_times(mx, bx), ix_times(my, by));
   double F3 = 0.0, F7 = 0.0;
-  if (hasz) {  // the z squares and products align with those of the plane
-    const int km = ix_max(em, emz), kb = ix_max(eB, eBz), kc = ix_max(em + eB, emz + eBz);
-    const Limbs mzl = ix_limbs(ix_align<4>(q(3), mz)), bzl = ix_limbs(ix_align<4>(q(7), mw));
-    IxSum kz, bz, mbz;
-    kz.square(mzl); bz.square(bzl); mbz.add(mzl, bzl);
-    kv = ix_shr(kv, 2 * (km - em)) + ix_shr(kz.value4_squares(), 2 * (km - emz));  // [61.6]
-    bv = ix_shr(bv, 2 * (kb - eB)) + ix_shr(bz.value4_squares(), 2 * (kb - eBz));
-    mBv = ix_shr(mBv, kc - em - eB) + ix_shr(mbz.value4(), kc - emz - eBz);
-    ek = 2 * km + 60;
-    eB2 = 2 * kb + 60;
-    emB = kc + 60;
-    const int ea = emz + eV + 61, eb = eBz + eBn + 61, K3 = ix_max(ea, eb);
-    F3 = ix_double(ix_shr(ix_prod(mzl, V), K3 - ea) - ix_shr(ix_prod(bzl, Bn), K3 - eb), K3);
-    const int ec = eBz + eV + 61, ed = emz + ebn + 61, K7 = ix_max(ec, ed);
-    F7 = ix_double(ix_shr(ix_prod(bzl, V), K7 - ec) - ix_shr(ix_prod(mzl, bnl), K7 - ed), K7);
+  if (hasz) {
+    const IxF w = ix_load(q(3)), bz = ix_load(q(7));
+    k2 = ix_plus(k2, ix_square(w));  // [61.6]
+    b2 = ix_plus(b2, ix_square(bz));
+    mB = ix_plus(mB, ix_times(w, bz));
+    F3 = ix_double(ix_minus(ix_times(w, V), ix_times(bz, Bn)));
+    F7 = ix_double(ix_minus(ix_times(bz, V), ix_times(w, bnl)));
   }
-  // pressure and total pressure
-  ek += e_ri + 62;
-  const int KS = ix_max(ix_max(eE + 1, ek), eB2);
-  const int ep = KS + gas.eg + 62, ept = ix_max(ep, eB2 - 1);
-  const int64_t E = ix_align<3>(q(4), me);  // [61]
-  const int64_t S = ix_shr(E, KS - eE - 1) - ix_shr(ix_mul(kv, ri), KS - ek) - ix_shr(bv, KS - eB2);
+  // 2 p / (gamma - 1) = 2 E - m^2/rho - B^2, the total pressure, E + pt
+  const IxF E = ix_load(q(4));
+  const IxV kr = ix_times(ix_split(k2), ri);
+  const int KS = ix_max(ix_max(E.e + 1, kr.e), b2.e);
+  const int64_t S = ix_shr(ix_whole(E).v, KS - E.e - 1) - ix_at(kr, KS) - ix_at(b2, KS);
   if (S < 0) return false;
-  const int64_t pt = ix_shr(ix_mul(S, gas.g), ept - ep) + ix_shr(bv, ept - eB2 + 1);  // [62.3]
-  {
-    const int64_t ps = pt >> 1;
-    const int np = ix_room(ps, 2), epn = ept + 1 - np + eS + 61;
-    const Limbs P = ix_limbs(ix_shl(ps, np));  // [61.3]
-    const int ea = em + eV + 61, eb = eB + eBn + 61, K = ix_max(ix_max(ea, eb), epn) + 1;
-    const double F1 = ix_double(ix_shr(ix_prod(mx, V), K - ea) - ix_shr(ix_prod(bx, Bn), K - eb) + ix_shr(ix_prod(P, nx), K - epn), K);
-    out(0, F0, F1);
-    const double F2 = ix_double(ix_shr(ix_prod(my, V), K - ea) - ix_shr(ix_prod(by, Bn), K - eb) + ix_shr(ix_prod(P, ny), K - epn), K);
-    out(1, F2, F3);
-  }
-  {
-    const int eEp = eE + gas.eh, ea = eEp + eV + 61, eb = emB + ebn + 61, K = ix_max(ea, eb);
-    const Limbs Ep = ix_limbs(ix_shr(E, gas.eh) + ix_shift(pt, eEp - ept));  // [61.7]
-    const double F4 = ix_double(ix_shr(ix_prod(Ep, V), K - ea) - ix_shr(ix_prod(ix_limbs(mBv), bnl), K - eb), K);
-    out(2, F4, ix_double(ix_prod(W, ny), eW + eS + 61));
-    out(3, ix_double(-ix_prod(W, nx), eW + eS + 61), F7);
-  }
+  const IxF P = ix_up(ix_halved(ix_plus(ix_times(IxF{ix_limbs(S), KS}, IxF{gas.g, gas.eg}), IxV{b2.v, b2.e - 1})));
+  const IxF Ep = ix_split(ix_halved(ix_plus(ix_whole(E), ix_whole(P))));
+  auto component = [&](IxF m, IxF b, IxF n) {  // m V - b Bn + pt n
+    const IxV a = ix_times(m, V), c = ix_times(b, Bn), d = ix_times(P, n);
+    const int K = ix_max(ix_max(a.e, c.e), d.e);
+    return ix_double(ix_at(a, K) - ix_at(c, K) + ix_at(d, K), K);
+  };
+  out(0, F0, component(mx, bx, nx));
+  out(1, component(my, by, ny), F3);
+  out(2, ix_double(ix_minus(ix_times(Ep, V), ix_times(ix_up(ix_halved(mB)), bnl))), ix_double(ix_times(W, ny)));
+  const IxV f6 = ix_times(W, nx);
+  out(3, ix_double(-f6.v, f6.e), F7);
   return true;
 }
 
