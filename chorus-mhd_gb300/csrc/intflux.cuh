@@ -487,217 +487,127 @@ FIX_HD bool vflux_int(Q&& q, G&& g, double mut, double eta, double sx, double sy
 // Rusanov flux along the unit normal (ux, uy) times `scale` (rusanov_core): Fh = scale
 // (Fl + Fr - eigv (qr - ql)).  q(side, k) reads variable k of the left (0) or right (1)
 // state, out(j, a, b) takes components 2 j and 2 j + 1.  Returns false, without output, where
-// the integer form does not apply.
+// the integer form does not apply (a density ratio above 8 among them).
 //
-// The two sides stream through sums (of the momentum flux, of the magnetic tension, ...) that
-// align when both are in, so that no component of the states lives longer than its side.
-// Bounds, in the comments: [b] means a magnitude below 2^b.
+// The two sides stream through sums (of the flux components without the pressure, of the
+// pressures, of the field), so that no component of the states lives longer than its side; each
+// term keeps its own exponent until its sum is formed, whichever side it comes from.
 template <class Q, class Out>
 FIX_HD bool rusanov_int(Q&& q, double ux, double uy, const IxGas& gas, double scale, double& eigv, Out&& out) {
-  // ---- exponents of the groups, range of the state
+  // ---- range of the states
   auto word = [&](int k) { return ix_max(ix_abs_word(q(0, k)), ix_abs_word(q(1, k))); };
-  const uint32_t zero = 66u << 20;  // a group of zeros: zeros are shifted out at this exponent
-  const uint32_t me = word(4), mr = word(0), ms = ix_abs_word(scale);
-  const uint32_t mm = ix_max(zero, ix_max(word(1), word(2))), mz = ix_max(zero, word(3));
-  const uint32_t mb = ix_max(zero, ix_max(word(5), word(6))), mw = ix_max(zero, word(7));
+  const uint32_t mr = word(0), ms = ix_abs_word(scale), el = ix_abs_word(q(0, 4)), er = ix_abs_word(q(1, 4));
+  const uint32_t mz = ix_max(word(3), word(7)), mp = ix_max(ix_max(word(1), word(2)), ix_max(word(5), word(6)));
   const uint32_t rl = (uint32_t)(fix_bits(q(0, 0)) >> 32), rr = (uint32_t)(fix_bits(q(1, 0)) >> 32);  // sign set: huge
   const uint32_t rmin = rl < rr ? rl : rr, rmax = rl < rr ? rr : rl;
-  if (ix_max(ix_max(ix_max(rmax, me), ix_max(mm, mz)), ix_max(ix_max(mb, mw), ms)) >= kIxHigh || rmin < kIxLow ||
-      me < kIxLow || ms < kIxLow || rmax - rmin >= (3u << 20))
+  if (ix_max(ix_max(ix_max(rmax, ix_max(el, er)), ix_max(mp, mz)), ms) >= kIxHigh || rmin < kIxLow ||
+      ix_max(el, er) < kIxLow || ms < kIxLow || rmax - rmin >= (3u << 20))
     return false;
-  const int em = ix_exp<4>(mm), emz = ix_exp<4>(mz), eB = ix_exp<4>(mb), eBz = ix_exp<4>(mw), eE = ix_exp<3>(me);
-  const bool hasz = ix_max(mz, mw) != zero;
-  const Limbs nx = ix_limbs(ix_align<3>(ux, 1023u << 20)), ny = ix_limbs(ix_align<3>(uy, 1023u << 20));  // [60], 2^-60
-  // ---- densities, mass fluxes, normal velocities
-  Limbs ri[2], V[2], mx[2], my[2];
-  const int e_ri = -122 - ix_exp<2>(rmin);  // of both reciprocals
-  int64_t Vv[2], F0 = 0;
-#pragma unroll
-  for (int s = 0; s < 2; s++) {
-    const double rho = q(s, 0);
-    const uint32_t r = ix_abs_word(rho);
-    ri[s] = ix_limbs(ix_rcp(ix_align<2>(rho, r)) >> ((r >> 20) - (rmin >> 20)));  // [61]
-    mx[s] = ix_limbs(ix_align<4>(q(s, 1), mm));  // [60]
-    my[s] = ix_limbs(ix_align<4>(q(s, 2), mm));
-    IxSum f;
-    f.add(mx[s], nx); f.add(my[s], ny);
-    const int64_t f0 = f.value4();  // [60.5], em
-    F0 += f0;
-    Vv[s] = ix_mul(f0, ri[s]);
-  }
-  const int nV = ix_room((Vv[0] ^ (Vv[0] >> 63)) | (Vv[1] ^ (Vv[1] >> 63)), 3), eV = em + e_ri + 62 - nV;
-  Vv[0] = ix_shl(Vv[0], nV);  // [60]: slow flows keep their bits
-  Vv[1] = ix_shl(Vv[1], nV);
-  V[0] = ix_limbs(Vv[0]);
-  V[1] = ix_limbs(Vv[1]);
-  // ---- the sums over the sides.  z squares and products align with those of the plane.
-  int dkx = 0, dkz = 0, dbx = 0, dbz = 0, dcx = 0, dcz = 0;
-  if (hasz) {
-    const int km = ix_max(em, emz), kb = ix_max(eB, eBz), kc = ix_max(em + eB, emz + eBz);
-    dkx = 2 * (km - em); dkz = 2 * (km - emz);
-    dbx = 2 * (kb - eB); dbz = 2 * (kb - eBz);
-    dcx = kc - em - eB; dcz = kc - emz - eBz;
-  }
-  const int ek = 2 * em + dkx + 60 + e_ri + 62, eB2 = 2 * eB + dbx + 60, emB = em + eB + dcx + 60;
-  const int KS = ix_max(ix_max(eE + 1, ek), eB2);
-  const int ep = KS + gas.eg + 62, ept = ix_max(ep, eB2 - 1), eEp = eE + gas.eh;
-  const int ebn = eB + e_ri + 62;
-  int64_t aVx = 0, aVy = 0, aBx = 0, aBy = 0, aVz = 0, aBz = 0, cVz = 0, cnz = 0, bE = 0;
-  int64_t W = 0, aE = 0, ps = 0, P = 0, bns = 0, sbX = 0, sbY = 0, sbZ = 0;
+  const bool hasz = mz >= kIxZero;
+  const IxF nx = ix_load(ux), ny = ix_load(uy);
+  // ---- the sums over the sides
+  IxV F0, W, Gx, Gy, Gz{0, 0}, G7{0, 0}, GE, va, P, ps, sx, sy, sz{0, 0};
   bool ok = true;
 #pragma unroll
   for (int s = 0; s < 2; s++) {
-    const int64_t vbx = ix_align<4>(q(s, 5), mb), vby = ix_align<4>(q(s, 6), mb);
-    sbX += vbx;
-    sbY += vby;
-    const Limbs bx = ix_limbs(vbx), by = ix_limbs(vby);
-    aVx += ix_prod(mx[s], V[s]);
-    aVy += ix_prod(my[s], V[s]);
-    IxSum b, k2, b2, mB, w;
-    b.add(bx, nx); b.add(by, ny);
-    const int64_t bn = b.value4();  // [60.5], eB
-    bns += bn;
-    const Limbs Bn = ix_limbs(bn), bnl = ix_limbs(ix_mul(bn, ri[s]));  // bnl [59.5], ebn
-    aBx += ix_prod(bx, Bn);
-    aBy += ix_prod(by, Bn);
-    k2.square(mx[s]); k2.square(my[s]);
-    b2.square(bx); b2.square(by);
-    mB.add(mx[s], bx); mB.add(my[s], by);
-    int64_t kv = k2.value4_squares(), bv = b2.value4_squares(), mBv = mB.value4();  // [61]
-    w.add(my[s], bx); w.add(mx[s], ix_limbs(-vby));
-    W += ix_mul(w.value4(), ri[s]);  // v Bx - u By, [60] a side
+    const IxF ri = ix_inverse(q(s, 0)), mx = ix_load(q(s, 1)), my = ix_load(q(s, 2));
+    const IxF bx = ix_load(q(s, 5)), by = ix_load(q(s, 6));
+    const IxV f = ix_plus(ix_times(mx, nx), ix_times(my, ny));  // [61]
+    const IxF V = ix_up(ix_times(ix_split(f), ri));
+    const IxF Bn = ix_up(ix_plus(ix_times(bx, nx), ix_times(by, ny))), bnl = ix_split(ix_times(Bn, ri));
+    const IxV w = ix_times(ix_split(ix_minus(ix_times(my, bx), ix_times(mx, by))), ri);  // v Bx - u By: [60]
+    const IxV gx = ix_minus(ix_times(mx, V), ix_times(bx, Bn)), gy = ix_minus(ix_times(my, V), ix_times(by, Bn));  // [61]
+    IxV k2 = ix_plus(ix_square(mx), ix_square(my)), b2 = ix_plus(ix_square(bx), ix_square(by));
+    IxV mB = ix_plus(ix_times(mx, bx), ix_times(my, by));
     if (hasz) {
-      const int64_t vz = ix_align<4>(q(s, 3), mz), vw = ix_align<4>(q(s, 7), mw);
-      sbZ += vw;
-      const Limbs mzl = ix_limbs(vz), bzl = ix_limbs(vw);
-      IxSum kz, bz, mbz;
-      kz.square(mzl); bz.square(bzl); mbz.add(mzl, bzl);
-      kv = ix_shr(kv, dkx) + ix_shr(kz.value4_squares(), dkz);  // [61.6]
-      bv = ix_shr(bv, dbx) + ix_shr(bz.value4_squares(), dbz);
-      mBv = ix_shr(mBv, dcx) + ix_shr(mbz.value4(), dcz);
-      aVz += ix_prod(mzl, V[s]);
-      aBz += ix_prod(bzl, Bn);
-      cVz += ix_prod(bzl, V[s]);
-      cnz += ix_prod(mzl, bnl);
+      const IxF mw = ix_load(q(s, 3)), bz = ix_load(q(s, 7));
+      k2 = ix_plus(k2, ix_square(mw));  // [61.6]
+      b2 = ix_plus(b2, ix_square(bz));
+      mB = ix_plus(mB, ix_times(mw, bz));
+      const IxV gz = ix_minus(ix_times(mw, V), ix_times(bz, Bn)), g7 = ix_minus(ix_times(bz, V), ix_times(mw, bnl));
+      Gz = s ? ix_plus(Gz, gz) : gz;  // [62]
+      G7 = s ? ix_plus(G7, g7) : g7;
+      sz = s ? ix_plus(sz, ix_whole(bz)) : ix_whole(bz);
     }
-    bE += ix_prod(ix_limbs(mBv), bnl);
-    const int64_t E = ix_align<3>(q(s, 4), me);  // [61]
-    const int64_t S = ix_shr(E, KS - eE - 1) - ix_shr(ix_mul(kv, ri[s]), KS - ek) - ix_shr(bv, KS - eB2);
-    ok = ok && S >= 0;  // 2 p / (gamma - 1); then [61]
-    const int64_t p = ix_mul(S, gas.g);
-    P += p;
-    const int64_t pt = ix_shr(p, ept - ep) + ix_shr(bv, ept - eB2 + 1);  // [62]
-    ps += pt >> 2;
-    aE += ix_prod(ix_limbs(ix_shr(E, gas.eh) + ix_shift(pt, eEp - ept)), V[s]);  // [61.7] [60]
+    // 2 p / (gamma - 1) = 2 E - m^2/rho - B^2, the total pressure, E + pt
+    const IxF E = ix_load(q(s, 4));
+    const IxV kr = ix_times(ix_split(k2), ri);
+    const int KS = ix_max(ix_max(E.e + 1, kr.e), b2.e);
+    const int64_t S = ix_shr(ix_whole(E).v, KS - E.e - 1) - ix_at(kr, KS) - ix_at(b2, KS);
+    ok = ok && S >= 0;
+    const IxV p = ix_times(IxF{ix_limbs(S & ~(S >> 63)), KS}, IxF{gas.g, gas.eg});  // [60]
+    const IxF pt = ix_up(ix_halved(ix_plus(p, IxV{b2.v, b2.e - 1})));
+    const IxF Ep = ix_split(ix_halved(ix_plus(ix_whole(E), ix_whole(pt))));
+    const IxV ge = ix_minus(ix_times(Ep, V), ix_times(ix_up(ix_halved(mB)), bnl));  // [61]
+    F0 = s ? ix_plus(F0, f) : f;  // [62]
+    W = s ? ix_plus(W, w) : w;    // [61]
+    Gx = s ? ix_plus(Gx, gx) : gx;
+    Gy = s ? ix_plus(Gy, gy) : gy;
+    GE = s ? ix_plus(GE, ge) : ge;
+    va = s ? ix_plus(va, ix_whole(V)) : ix_whole(V);  // [62]
+    P = s ? ix_plus(P, p) : p;  // [61]
+    ps = s ? ix_plus(ps, ix_whole(pt)) : ix_whole(pt);  // [62]
+    sx = s ? ix_plus(sx, ix_whole(bx)) : ix_whole(bx);
+    sy = s ? ix_plus(sy, ix_whole(by)) : ix_whole(by);
   }
-  // ---- wave speed: with P = gamma (pl + pr), T = P + 2 |B|^2, N = 2 bn^2 (B averaged) and
-  // rs = rho_l + rho_r, cf^2 = (T + sqrt(T^2 - 4 P N)) / (2 rs)
-  P = ix_mul(P, gas.gam);
-  if (!ok || P <= 0) return false;
-  int64_t eign;  // -eigv
-  int ee;
+  // ---- wave speed: with P = gamma (pl + pr), B twice the averaged field, T = P + |B|^2 / 2 and
+  // rs = rho_l + rho_r, cf^2 = (T + sqrt(T^2 - 2 P bn^2)) / (2 rs).  Operands are shifted up to full
+  // length before they are multiplied on: a field that reverses across the face leaves B far below
+  // either side's (with its leading zeros the speed lost up to 2^-26 of itself at a beta of 1e-8)
+  P = ix_times(ix_split(P), IxF{gas.gam, gas.egam});
+  if (!ok || P.v <= 0) return false;
+  IxF eig;  // -eigv
   {
-    const int nP = ix_room(P, 3);  // (a pressure far below the energy has few bits)
-    P = ix_shl(P, nP);
-    const int eP = ep + gas.egam + 62 - nP;
-    IxSum b2;
-    b2.square(ix_limbs(sbX >> 1));
-    b2.square(ix_limbs(sbY >> 1));
-    int64_t D = b2.value4_squares();
-    if (hasz) {
-      IxSum z;
-      z.square(ix_limbs(sbZ >> 1));
-      D = ix_shr(D, dbx) + ix_shr(z.value4_squares(), dbz);
-    }
-    const Limbs bn = ix_limbs(bns);  // twice the average
-    const int K = ix_max(eP, eB2 + 1) + 1;
-    const int64_t Pk = ix_shr(P, K - eP), Nk = ix_shr(ix_mul(bn, bn), K - (2 * eB + 61));
-    const int64_t T = Pk + ix_shr(D, K - eB2 - 1);  // [61.5]
-    const Limbs Tl = ix_limbs(T);
-    const int64_t disc = ix_mul(Tl, Tl) - ix_mul(ix_shl(Pk, 1), ix_limbs(ix_shl(Nk, 1)));
-    if (disc < 0) return false;
-    int64_t U = T >> 1;  // K + 1
-    if (disc > 0) {
-      int es;
-      const int64_t sq = ix_sqrt(disc, 2 * K + 62, es);
-      U += ix_shr(sq, K + 1 - es);
+    const IxF Pl = ix_up(P), Bx = ix_up(ix_halved(sx)), By = ix_up(ix_halved(sy));
+    IxV D = ix_plus(ix_square(Bx), ix_square(By));
+    if (hasz) D = ix_plus(D, ix_square(ix_up(ix_halved(sz))));  // [61.6]
+    const IxF bn = ix_up(ix_plus(ix_times(Bx, nx), ix_times(By, ny)));
+    const IxF T = ix_up(ix_halved(ix_plus(ix_whole(Pl), IxV{D.v, D.e - 1})));
+    IxV N = ix_times(Pl, ix_up(ix_square(bn)));
+    N.e++;
+    const IxV disc = ix_minus(ix_square(T), N);
+    if (disc.v < 0) return false;
+    IxV U = ix_halved(ix_whole(T));  // [60]
+    if (disc.v > 0) {
+      IxV sq;
+      sq.v = ix_sqrt(disc.v, disc.e, sq.e);  // at most T
+      U.v += ix_shr(sq.v, U.e - sq.e);       // [61]
     }
     const int64_t rs = ix_align<3>(q(0, 0), mr) + ix_align<3>(q(1, 0), mr);  // 2^60 < rs < 2^62
     const int up = rs < ((int64_t)1 << 61) ? 1 : 0;
-    const int64_t irs = ix_rcp(ix_shl(rs, up));
-    int ec;
-    const int64_t cf = ix_sqrt(ix_mul(U, ix_limbs(irs)), K - 122 - ix_exp<3>(mr) + up + 62, ec);
-    const int64_t va = Vv[0] + Vv[1];
-    ee = ix_max(eV, ec) + 1;
-    eign = -(ix_shr(va < 0 ? -va : va, ee - eV + 1) + ix_shr(cf, ee - ec));  // [60.6]
-    eigv = ix_double(-eign, ee);
+    const IxF irs{ix_limbs(ix_rcp(ix_shl(rs, up))), up - 122 - ix_exp<3>(mr)};
+    const IxV cf2 = ix_times(ix_split(U), irs);
+    IxV cf;
+    cf.v = ix_sqrt(cf2.v, cf2.e - 1, cf.e);  // [61]
+    va.v = va.v < 0 ? -va.v : va.v;
+    const int K = ix_max(va.e - 1, cf.e) + 1;
+    const int64_t ev = ix_shr(va.v, K - va.e + 1) + ix_at(cf, K);  // [61.6]
+    eig = IxF{ix_limbs(-ev), K};
+    eigv = ix_double(ev, K);
   }
-  const Limbs eig = ix_limbs(eign), sc = ix_limbs(ix_align<3>(scale, ms));
-  const int esc = ix_exp<3>(ms) + 62;
-  auto scaled = [&](int64_t v, int e) { return ix_double(ix_mul(v, sc), e + esc); };
+  const IxF sc = ix_load(scale);
   // - eigv (qr - ql) of variable k: one FP64 subtraction (the pipe has room), so that small
-  // differences keep their bits; [60.6] at exponent ed
-  auto jump = [&](int k, int& ed) {
-    const double d = q(1, k) - q(0, k);
-    const uint32_t m = ix_max(zero, ix_abs_word(d));
-    ed = ix_exp<3>(m) + ee + 61;
-    return ix_prod(ix_limbs(ix_align<3>(d, m)), eig);
-  };
-  int ed;
-  double f0, f1;
-  // ---- mass
+  // differences keep their bits
+  auto jump = [&](int k) { return ix_times(ix_load(q(1, k) - q(0, k)), eig); };  // [60.6]
+  auto scaled = [&](IxV a, IxV b) { return ix_double(ix_times(ix_up(ix_halved(ix_plus(a, b))), sc)); };  // a + b: [62.6]
+  double f0 = scaled(F0, jump(0)), f1;
   {
-    const int64_t d = jump(0, ed);
-    const int K = ix_max(em, ed) + 1;
-    f0 = scaled(ix_shr(F0, K - em) + ix_shr(d, K - ed), K);
-  }
-  // ---- momentum
-  {
-    const int np = ix_room(ps, 2), epts = ept + 2 - np;
-    const Limbs pt = ix_limbs(ix_shl(ps, np));  // [61]
-    const int ea = em + eV + 61, eb = 2 * eB + 61;
-    auto component = [&](int k, int64_t aV, int64_t aB, Limbs nn) {
-      IxSum p;
-      p.add(pt, nn);
-      const int64_t d = jump(k, ed);
-      const int K = ix_max(ix_max(ea, eb), ix_max(epts, ed)) + 1;
-      return scaled(ix_shr(aV, K - ea) - ix_shr(aB, K - eb) + ix_shr(p.value4(), K - epts) + ix_shr(d, K - ed), K);
-    };
-    f1 = component(1, aVx, aBx, nx);
+    const IxF pt = ix_up(ix_halved(ps));
+    f1 = scaled(ix_plus(Gx, ix_times(pt, nx)), jump(1));
     out(0, f0, f1);
-    f0 = component(2, aVy, aBy, ny);
+    f0 = scaled(ix_plus(Gy, ix_times(pt, ny)), jump(2));
   }
-  f1 = 0.0;
-  if (hasz) {
-    const int64_t d = jump(3, ed);
-    const int ea = emz + eV + 61, eb = eBz + eB + 61, K = ix_max(ix_max(ea, eb), ed) + 1;
-    f1 = scaled(ix_shr(aVz, K - ea) - ix_shr(aBz, K - eb) + ix_shr(d, K - ed), K);
-  }
-  out(1, f0, f1);
-  // ---- energy
-  {
-    const int64_t d = jump(4, ed);
-    const int ea = eEp + eV + 61, eb = emB + ebn + 61, K = ix_max(ix_max(ea, eb), ed) + 1;
-    f0 = scaled(ix_shr(aE, K - ea) - ix_shr(bE, K - eb) + ix_shr(d, K - ed), K);
-  }
-  // ---- induction: (v Bx - u By) (uy, -ux) in the plane
-  {
-    const int eW = em + eB + 60 + e_ri + 62 + 1;  // of W n >> 61
-    int64_t d = jump(5, ed);
-    int K = ix_max(eW, ed) + 1;
-    f1 = scaled(ix_shr(ix_prod(ix_limbs(W), ny), K - eW) + ix_shr(d, K - ed), K);
+  out(1, f0, hasz ? scaled(Gz, jump(3)) : 0.0);
+  f0 = scaled(GE, jump(4));
+  {  // induction: (v Bx - u By) (uy, -ux) in the plane
+    const IxF w = ix_up(W);
+    f1 = scaled(ix_times(w, ny), jump(5));
     out(2, f0, f1);
-    d = jump(6, ed);
-    K = ix_max(eW, ed) + 1;
-    f0 = scaled(ix_shr(ix_prod(ix_limbs(-W), nx), K - eW) + ix_shr(d, K - ed), K);
+    IxV d = ix_times(w, nx);
+    d.v = -d.v;
+    f0 = scaled(d, jump(6));
   }
-  f1 = 0.0;
-  if (hasz) {
-    const int64_t d = jump(7, ed);
-    const int ea = eBz + eV + 61, eb = emz + ebn + 61, K = ix_max(ix_max(ea, eb), ed) + 1;
-    f1 = scaled(ix_shr(cVz, K - ea) - ix_shr(cnz, K - eb) + ix_shr(d, K - ed), K);
-  }
-  out(3, f0, f1);
+  out(3, f0, hasz ? scaled(G7, jump(7)) : 0.0);
   return true;
 }
 

@@ -96,3 +96,62 @@ def test_interior_flux(driver, tmp_path, kind, normal, gam):  # noqa: F811
     Q, N, g = q.astype(LD), S.astype(LD), LD(gam)
     F = exact_flux(Q, N, g)[0]
     assert np.all(abs(out[:, 1:] - F) <= EPS * terms(Q, N, g)[0])
+
+
+SIDES = ["alike", "independent", "contrast"]
+
+
+def right_states(rng, kind, n, ql, gam):
+    """The right sides of faces: a little off the left one; any other state; the same but with the
+    momentum large where the left's is small and the field the other way round."""
+    if kind == "alike":
+        return ql * (1 + np.exp(rng.uniform(-20, -3, n))[:, None] * rng.uniform(-0.2, 0.2, ql.shape))
+    rho = ql[:, 0] * 2.0 ** rng.uniform(-2.4, 2.4, n)
+    if kind == "independent":
+        q = mixed(rng, "mixed", n, gam)
+        q[:, 4] = np.maximum(q[:, 4], 0.6 * (q[:, 1:4] ** 2).sum(1) / rho + 0.6 * (q[:, 5:8] ** 2).sum(1) + 1e-3)
+    else:
+        c = 10.0 ** rng.uniform(1, 6, n)[:, None]
+        q = ql.copy()
+        q[:, 1:4], q[:, 5:8] = q[:, 1:4] * c, q[:, 5:8] / c
+        q[:, 4] = 0.6 * (q[:, 1:4] ** 2).sum(1) / rho + 0.6 * (q[:, 5:8] ** 2).sum(1) + ql[:, 4]
+    q[:, 0] = rho
+    return q
+
+
+@pytest.mark.parametrize("gam", GAMMAS)
+@pytest.mark.parametrize("normal", ["axis", "near axis", "any"])
+@pytest.mark.parametrize("sides", SIDES)
+@pytest.mark.parametrize("kind", STATES)
+def test_face_flux(driver, tmp_path, kind, sides, normal, gam):  # noqa: F811
+    """The wave speed enters every component with its own error: the roundings of the normal
+    velocities and, through the square roots, that of the pressures."""
+    rng = np.random.default_rng(3000 + 10 * STATES.index(kind) + 100 * SIDES.index(sides) + len(normal) + int(100 * gam))
+    n = 2000
+    ql = mixed(rng, kind, n, gam)
+    qr = right_states(rng, sides, n, ql, gam)
+    ratio = np.maximum(ql[:, 0] / qr[:, 0], qr[:, 0] / ql[:, 0])
+    N = normals(rng, normal, n)
+    N = N / np.sqrt((N * N).sum(1))[:, None]
+    sc = rng.choice([-1, 1], n) * np.exp(rng.uniform(-8, 8, n))
+    out = evaluate(driver, tmp_path, 0, np.concatenate([ql, qr, N, sc[:, None], np.full((n, 1), gam)], 1))
+    took = out[:, 0] == 1
+    L, R, M, S, g = ql.astype(LD), qr.astype(LD), N.astype(LD), sc.astype(LD), LD(gam)
+    (Fl, pl, vl), (Fr, pr, vr) = exact_flux(L, M, g), exact_flux(R, M, g)
+    # (left to the FP64 form: a density ratio above 8, a negative pressure)
+    assert np.all(took[(ratio < 7.9) & (pl > 0) & (pr > 0)])
+    (tl, el, al), (tr, er, ar) = terms(L, M, g), terms(R, M, g)
+    B = (L[:, 5:] + R[:, 5:]) / 2
+    P, D, bn2 = g * (pl + pr), 2 * (B * B).sum(1), 2 * (B[:, :2] * M).sum(1) ** 2
+    T, rs = P + D, L[:, 0] + R[:, 0]
+    disc = np.maximum(T * T - 4 * P * bn2, 0)
+    cf = np.sqrt((T + np.sqrt(disc)) / (2 * rs))
+    eig = abs(vl + vr) / 2 + cf
+    dT = EPS * (g * (el + er) + D)
+    dsq = np.minimum(T * dT / np.maximum(np.sqrt(disc), LD(1e-300)), np.sqrt(T * dT))
+    deig = EPS * (al + ar + eig) + (dT + dsq) / (4 * rs * cf)
+    assert np.all(abs(out[:, 9] - eig)[took] <= deig[took])
+    J = R - L
+    F = S[:, None] * (Fl + Fr - eig[:, None] * J)
+    bound = abs(S[:, None]) * (EPS * (tl + tr + eig[:, None] * abs(J)) + deig[:, None] * abs(J))
+    assert np.all(abs(out[:, 1:9] - F)[took] <= bound[took])
