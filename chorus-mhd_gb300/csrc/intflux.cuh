@@ -2,26 +2,27 @@
 //
 // GB300 executes FP64 at 2 lane-operations per clock per SM (a warp instruction occupies
 // its scheduler's FP64 unit for 64 clocks), the integer pipes take 64 each.  The nonlinear
-// fluxes are products and sums of few variables, so they are evaluated as block fixed-point
-// numbers: a value is v 2^e with a 64-bit integer v and an exponent e that a group of
-// quantities shares, products keep the upper part of the 128-bit product of two such
-// integers, sums align to the larger exponent, and each result is rounded once into a
-// double.
+// fluxes are products and sums of few variables, so they are evaluated in integers: a value is
+// v 2^e with a 64-bit integer v and an exponent e of its own, products keep the upper part of the
+// 128-bit product of two such integers, sums align to the largest of their terms, and each
+// result is rounded once into a double.
 //
-//   * Groups: the x and y components of the momentum (of both sides of a face), their z
-//     components, the same for B, the energies, the densities.  The z components have
-//     exponents of their own because they can be small and decoupled from the plane.
-//   * A product takes the operands as limbs v = h 2^31 + l (0 <= l < 2^31):
+//   * A product takes the operands as limbs v = h 2^31 + l (|l| < 2^31):
 //     (a b) >> 62 = ha hb + ((ha lb + la hb) >> 31) in three 32x32->64 multiply-adds; the
 //     product of the low limbs is below one unit and left out.
-//   * Values keep 57 to 61 significant bits relative to the largest term of their sum, so
-//     the errors before the final rounding stay below those of the FP64 chain, which
-//     rounds every intermediate to 53 bits.
+//   * A product of two operands of full length (2^60 .. 2^61) is off by two units of at least 2^58;
+//     operands that have lost length, to a cancellation or over several products, are shifted up
+//     again (ix_up).  Each term of a component is then off by less than 2^-54 of itself, and the
+//     component, with its rounding, by less than 2^-52 of the sum of its terms' magnitudes (the
+//     viscous flux 2^-51).  Over states with components of all sizes the rms error is at or below
+//     that of the FP64 forms, component by component, typically half of it.
 //
-// The integer form takes finite states with a normal positive density and exponents within
-// a wide window (2^-200 .. 2^200; zero and smaller values of momentum and B as well); everything else (infinities, NaNs, zero or negative
-// density, a density ratio above 8 across a face, a negative discriminant) is left to the
-// FP64 form, whose results on such states the caller keeps.
+// The integer form takes finite states with a normal positive density and magnitudes within
+// a wide window (2^-200 .. 2^200; zero and smaller values of all but the density, energy and
+// metric as well);
+// everything else (infinities, NaNs, zero or negative density, a negative pressure, a density ratio
+// above 8 across a face, a negative discriminant) is left to the FP64 form, whose results on
+// such states the caller keeps.
 #pragma once
 #include <cstdint>
 
@@ -53,24 +54,6 @@ FIX_HD int64_t ix_mul(Limbs a, Limbs b) {
   return fix_mad(a.h, b.h, t >> 31);
 }
 FIX_HD int64_t ix_mul(int64_t a, Limbs b) { return ix_mul(ix_limbs(a), b); }
-
-// a sum of products, >> 62 at the end
-struct IxSum {
-  int64_t A = 0, T = 0;
-  FIX_HD void add(Limbs a, Limbs b) {
-    T = fix_mad(a.h, b.l, T);
-    T = fix_mad(a.l, b.h, T);
-    A = fix_mad(a.h, b.h, A);
-  }
-  FIX_HD void square(Limbs a) {  // half of the cross terms: value() with shift 30
-    T = fix_mad(a.h, a.l, T);
-    A = fix_mad(a.h, a.h, A);
-  }
-  FIX_HD int64_t value() const { return A + (T >> 31); }
-  FIX_HD int64_t value2() const { return ix_shl(A, 1) + (T >> 30); }  // >> 61
-  FIX_HD int64_t value4() const { return ix_shl(A, 2) + (T >> 29); }  // >> 60
-  FIX_HD int64_t value4_squares() const { return ix_shl(A, 2) + (T >> 28); }
-};
 
 FIX_HD uint32_t ix_abs_word(double x) { return (uint32_t)(fix_bits(x) >> 32) & 0x7fffffffu; }
 FIX_HD uint32_t ix_max(uint32_t a, uint32_t b) { return a > b ? a : b; }
@@ -154,9 +137,6 @@ FIX_HD int64_t ix_sqrt(int64_t v, int e, int& es) {
   return a + a + (fix_mad(La.h, c1, (fix_mad(La.l, c1, 0) >> 31) + (fix_mad(La.h, c0, 0) >> 7)) >> 19);
 }
 
-// v >> d, or v << -d (where the caller knows that it fits)
-FIX_HD int64_t ix_shift(int64_t v, int d) { return d >= 0 ? ix_shr(v, d) : ix_shl(v, -d); }
-
 // leading zeros of |v| among the upper 32 bits, less `keep`: a left shift by that many bits
 // (at least 0) leaves |v| <= 2^(64 - keep)
 FIX_HD int ix_room(int64_t v, int keep) {
@@ -225,50 +205,11 @@ FIX_HD IxF ix_up(IxV a) {
 }
 FIX_HD double ix_double(IxV a) { return ix_double(a.v, a.e); }
 
-// limbs of v shifted up to [60] where it is below that, with its exponent; and of a pair
-FIX_HD Limbs ix_up(int64_t v, int& e) {
-  const int n = ix_room(v, 3);
-  e -= n;
-  return ix_limbs(ix_shl(v, n));
-}
-FIX_HD void ix_up2(int64_t a, int64_t b, int& e, Limbs& la, Limbs& lb) {
-  const int n = ix_room((a ^ (a >> 63)) | (b ^ (b >> 63)), 3);
-  e -= n;
-  la = ix_limbs(ix_shl(a, n));
-  lb = ix_limbs(ix_shl(b, n));
-}
-
-// constants of a solve, prepared once (host or device): half of gamma - 1, gamma, as limbs
-// of normalised integers in [2^60, 2^61) with their exponents
+// constants of a solve, prepared once (host or device): half of gamma - 1, gamma, gamma / Pr
 struct IxGas {
-  Limbs g, gam;
-  int eg, egam;
-  Limbs kap;  // gamma / Pr
-  int ekap;
-  int eh;  // E + p + B^2/2 <= (1 + gamma) E, as p >= 0 and B^2/2 <= E: below 2^(eh + 0.7) E
+  IxF g, gam, kap;
 };
-FIX_HD IxGas ix_gas(double gamma) {
-  IxGas c;
-  const double gm = 0.5 * (gamma - 1.0);
-  c.g = ix_limbs(ix_align<3>(gm, ix_abs_word(gm)));
-  c.eg = ix_exp<3>(ix_abs_word(gm));
-  c.gam = ix_limbs(ix_align<3>(gamma, ix_abs_word(gamma)));
-  c.egam = ix_exp<3>(ix_abs_word(gamma));
-  const double kp = gamma / 0.72;
-  c.kap = ix_limbs(ix_align<3>(kp, ix_abs_word(kp)));
-  c.ekap = ix_exp<3>(ix_abs_word(kp));
-  for (c.eh = 1; c.eh < 60 && 1.0 + gamma > 1.62 * (double)(1LL << c.eh); c.eh++) {
-  }
-  return c;
-}
-
-
-// a product as an increment of a sum: (a b) >> 61
-FIX_HD int64_t ix_prod(Limbs a, Limbs b) {
-  IxSum p;
-  p.add(a, b);
-  return p.value2();
-}
+FIX_HD IxGas ix_gas(double gamma) { return IxGas{ix_load(0.5 * (gamma - 1.0)), ix_load(gamma), ix_load(gamma / 0.72)}; }
 
 // Contravariant ideal-MHD flux F sx + G sy (iflux_contra); q(k) reads variable k, out(j, a, b)
 // takes components 2 j and 2 j + 1.  Returns false, without output, where the integer form does
@@ -307,7 +248,7 @@ FIX_HD bool iflux_int(Q&& q, double sx, double sy, const IxGas& gas, Out&& out) 
   const int KS = ix_max(ix_max(E.e + 1, kr.e), b2.e);
   const int64_t S = ix_shr(ix_whole(E).v, KS - E.e - 1) - ix_at(kr, KS) - ix_at(b2, KS);
   if (S < 0) return false;
-  const IxF P = ix_up(ix_halved(ix_plus(ix_times(IxF{ix_limbs(S), KS}, IxF{gas.g, gas.eg}), IxV{b2.v, b2.e - 1})));
+  const IxF P = ix_up(ix_halved(ix_plus(ix_times(IxF{ix_limbs(S), KS}, gas.g), IxV{b2.v, b2.e - 1})));
   const IxF Ep = ix_split(ix_halved(ix_plus(ix_whole(E), ix_whole(P))));
   auto component = [&](IxF m, IxF b, IxF n) {  // m V - b Bn + pt n
     const IxV a = ix_times(m, V), c = ix_times(b, Bn), d = ix_times(P, n);
@@ -326,158 +267,91 @@ FIX_HD bool iflux_int(Q&& q, double sx, double sy, const IxGas& gas, Out&& out) 
 // these are): q(k) the state, g(d, k) its gradient, mut and eta the viscosity and resistivity.
 // out(k, value) takes components 1..7; false, without output, where the integer form does not
 // apply.  The first output comes after the last use of q, which may therefore lie in the outputs'
-// place.  [b] in the comments means a magnitude below 2^b.
+// place.
 template <class Q, class G, class Out>
 FIX_HD bool vflux_int(Q&& q, G&& g, double mut, double eta, double sx, double sy, const IxGas& gas, Out&& out) {
-  const uint32_t zero = 66u << 20;  // a group of zeros: zeros are shifted out at this exponent
-  auto w1 = [&](int k) { return ix_max(zero, ix_abs_word(q(k))); };
-  auto w2 = [&](int k) { return ix_max(zero, ix_max(ix_abs_word(g(0, k)), ix_abs_word(g(1, k)))); };
+  auto w1 = [&](int k) { return ix_abs_word(q(k)); };
+  auto w2 = [&](int k) { return ix_max(ix_abs_word(g(0, k)), ix_abs_word(g(1, k))); };
   const uint32_t r = (uint32_t)(fix_bits(q(0)) >> 32);  // huge if the sign is set
-  const uint32_t mm = ix_max(w1(1), w1(2)), mz = w1(3), me = w1(4), mb = ix_max(w1(5), w1(6)), mw = w1(7);
-  const uint32_t gr = w2(0), gm = ix_max(w2(1), w2(2)), gz = w2(3), ge = w2(4), gb = ix_max(w2(5), w2(6)), gw = w2(7);
-  const uint32_t ms = ix_max(ix_abs_word(sx), ix_abs_word(sy));
-  const uint32_t mu = ix_max(zero, ix_abs_word(mut)), mt = ix_max(zero, ix_abs_word(eta));
-  const uint32_t top = ix_max(ix_max(ix_max(ix_max(r, mm), ix_max(mz, me)), ix_max(ix_max(mb, mw), ix_max(ms, mu))),
-                              ix_max(ix_max(ix_max(gr, gm), ix_max(gz, ge)), ix_max(ix_max(gb, gw), mt)));
-  if (top >= kIxHigh || r < kIxLow || ms < kIxLow) return false;
-  const bool hasz = ix_max(ix_max(mz, mw), ix_max(gz, gw)) != zero;
-  const int em = ix_exp<4>(mm), eB = ix_exp<4>(mb), eS = ix_exp<4>(ms), e_ri = -122 - ix_exp<2>(r);
-  const int egr = ix_exp<4>(gr), egm = ix_exp<4>(gm), egB = ix_exp<4>(gb);
-  const Limbs nx = ix_limbs(ix_align<4>(sx, ms)), ny = ix_limbs(ix_align<4>(sy, ms));  // [60]
-  const Limbs ri = ix_limbs(ix_rcp(ix_align<2>(q(0), r)));                             // [61]
-  int eM = ix_exp<3>(mu) + e_ri + 62;
-  const Limbs M = ix_up(ix_mul(ix_align<3>(mut, mu), ri), eM);                         // [60] mu / rho
-  auto contracted = [&](Limbs a, Limbs b) {  // a sx + b sy: [60.5], exponent of a + eS + 60
-    IxSum t;
-    t.add(a, nx); t.add(b, ny);
-    return t.value4();
-  };
-  // velocities, m^2 + ... of the internal energy: X = |u|^2 + B^2/(2 rho) - E/rho
-  const Limbs mx = ix_limbs(ix_align<4>(q(1), mm)), my = ix_limbs(ix_align<4>(q(2), mm));  // [60]
-  int eu = em + e_ri + 61;
-  Limbs u, v;  // [60]
-  ix_up2(ix_prod(mx, ri), ix_prod(my, ri), eu, u, v);
-  const Limbs bx = ix_limbs(ix_align<4>(q(5), mb)), by = ix_limbs(ix_align<4>(q(6), mb));
-  IxSum k2, b2;
-  k2.square(mx); k2.square(my);
-  b2.square(bx); b2.square(by);
-  int64_t kv = k2.value4_squares(), bv = b2.value4_squares();  // [61]
-  int ek = 2 * em + 60, eB2 = 2 * eB + 60;
-  Limbs w{0, 0}, bz{0, 0};
-  int ew = 0, eBz = 0;
-  if (hasz) {
-    const int emz = ix_exp<4>(mz);
-    eBz = ix_exp<4>(mw);
-    const int km = ix_max(em, emz), kb = ix_max(eB, eBz);
-    const Limbs mzl = ix_limbs(ix_align<4>(q(3), mz));
-    bz = ix_limbs(ix_align<4>(q(7), mw));
-    IxSum a, b;
-    a.square(mzl); b.square(bz);
-    kv = ix_shr(kv, 2 * (km - em)) + ix_shr(a.value4_squares(), 2 * (km - emz));  // [61.6]
-    bv = ix_shr(bv, 2 * (kb - eB)) + ix_shr(b.value4_squares(), 2 * (kb - eBz));
-    ek = 2 * km + 60;
-    eB2 = 2 * kb + 60;
-    ew = emz + e_ri + 61;
-    w = ix_up(ix_prod(mzl, ri), ew);
-  }
-  ek += e_ri + 62;
-  const int eE = ix_exp<3>(me), KY = ix_max(ix_max(ek, eB2 - 1), eE) + 1;
-  int eX = KY + e_ri + 62;
-  const Limbs X = ix_up(ix_mul(ix_shr(ix_mul(kv, ri), KY - ek) + ix_shr(bv, KY - eB2 + 1) - ix_shr(ix_align<3>(q(4), me), KY - eE), ri), eX);  // [60]
-  // gradients of the density, and rho times those of the plane's velocity
-  const Limbs rx = ix_limbs(ix_align<4>(g(0, 0), gr)), ry = ix_limbs(ix_align<4>(g(1, 0), gr));
-  int erS = egr + eS + 60;
-  const Limbs rS = ix_up(contracted(rx, ry), erS);  // [60]
-  const int ep = egr + eu + 61, Kw = ix_max(egm, ep) + 1;
-  Limbs c1, c2;
-  int64_t t2;  // u.(grad m . S) of the plane
-  int ec = Kw + eS + 61, e2 = egm + eS + 60;
+  const uint32_t mz = ix_max(ix_max(w1(3), w1(7)), ix_max(w2(3), w2(7)));
+  const uint32_t mq = ix_max(ix_max(ix_max(w1(1), w1(2)), ix_max(w1(5), w1(6))), ix_max(w1(4), r));
+  const uint32_t mg = ix_max(ix_max(ix_max(w2(0), w2(1)), ix_max(w2(2), w2(4))), ix_max(w2(5), w2(6)));
+  const uint32_t ms = ix_max(ix_abs_word(sx), ix_abs_word(sy)), mc = ix_max(ix_abs_word(mut), ix_abs_word(eta));
+  if (ix_max(ix_max(ix_max(mq, mg), ix_max(mz, ms)), mc) >= kIxHigh || r < kIxLow || ms < kIxLow) return false;
+  const bool hasz = mz >= kIxZero;
+  const IxF nx = ix_load(sx), ny = ix_load(sy), ri = ix_inverse(q(0));
+  const IxF M = ix_up(ix_times(ix_load(mut), ri));  // mu / rho
+  auto along = [&](IxF a, IxF b) { return ix_plus(ix_times(a, nx), ix_times(b, ny)); };  // a sx + b sy: [61]
+  // velocities; X = |u|^2 + B^2/(2 rho) - E/rho
+  const IxF mx = ix_load(q(1)), my = ix_load(q(2)), bx = ix_load(q(5)), by = ix_load(q(6));
+  const IxF u = ix_up(ix_times(mx, ri)), v = ix_up(ix_times(my, ri));
+  IxF w{Limbs{0, 0}, 0}, bz{Limbs{0, 0}, 0};
+  IxF X;
   {
-    const int64_t ax = ix_align<4>(g(0, 1), gm), ay = ix_align<4>(g(1, 1), gm);
-    const int64_t bx_ = ix_align<4>(g(0, 2), gm), by_ = ix_align<4>(g(1, 2), gm);
-    Limbs mxS, myS;
-    ix_up2(contracted(ix_limbs(ax), ix_limbs(ay)), contracted(ix_limbs(bx_), ix_limbs(by_)), e2, mxS, myS);
-    t2 = ix_prod(mxS, u) + ix_prod(myS, v);  // [60]
-    e2 += eu + 61;
-    auto rel = [&](int64_t a, Limbs r_, Limbs u_) { return ix_shr(a, Kw - egm) - ix_shr(ix_prod(r_, u_), Kw - ep); };  // [60]
-    const int64_t ux = rel(ax, rx, u), uy = rel(ay, ry, u), vx = rel(bx_, rx, v), vy = rel(by_, ry, v);
-    const Limbs two3{(int)(1537228672809129301LL >> 31), (int)(1537228672809129301LL & 0x7fffffff)};  // 2^62 / 3
-    const int64_t ld = ix_prod(ix_limbs(ux + vy), two3);  // 2/3 of the divergence: [60.5]
-    const Limbs a = ix_limbs(ux + ux - ld), b = ix_limbs(uy + vx), d = ix_limbs(vy + vy - ld);  // [61.7]
-    ix_up2(ix_prod(a, nx) + ix_prod(b, ny), ix_prod(b, nx) + ix_prod(d, ny), ec, c1, c2);  // [61.4], [60] if shifted
+    IxV k2 = ix_plus(ix_square(mx), ix_square(my)), b2 = ix_plus(ix_square(bx), ix_square(by));  // [61]
+    if (hasz) {
+      const IxF mw = ix_load(q(3));
+      bz = ix_load(q(7));
+      w = ix_up(ix_times(mw, ri));
+      k2 = ix_plus(k2, ix_square(mw));  // [61.6]
+      b2 = ix_plus(b2, ix_square(bz));
+    }
+    const IxV kr = ix_times(ix_split(k2), ri), E = ix_whole(ix_load(q(4)));
+    const int K = ix_max(ix_max(kr.e, b2.e - 1), E.e) + 1;
+    X = ix_up(ix_times(ix_split(IxV{ix_at(kr, K) + ix_shr(b2.v, K - b2.e + 1) - ix_at(E, K), K}), ri));
   }
-  out(1, ix_double(ix_mul(c1, M), ec + eM + 62));
-  out(2, ix_double(ix_mul(c2, M), ec + eM + 62));
+  const IxF rx = ix_load(g(0, 0)), ry = ix_load(g(1, 0)), rS = ix_up(along(rx, ry));
+  // rho times the velocity gradients of the plane; with a third of the divergence D, the rows
+  // c1 = 2 (ux - D) sx + (uy + vx) sy, c2 = (uy + vx) sx + 2 (vy - D) sy of the stress
+  IxF c1, c2;
+  IxV t2;  // u.(grad m . S) of the plane
+  {
+    const IxF ax = ix_load(g(0, 1)), ay = ix_load(g(1, 1)), cx = ix_load(g(0, 2)), cy = ix_load(g(1, 2));
+    t2 = ix_plus(ix_times(ix_up(along(ax, ay)), u), ix_times(ix_up(along(cx, cy)), v));  // [61]
+    auto rel = [&](IxF a, IxF r_, IxF u_) { return ix_minus(ix_halved(ix_whole(a)), ix_times(r_, u_)); };  // [61]
+    const IxV ux = rel(ax, rx, u), uy = rel(ay, ry, u), vx = rel(cx, rx, v), vy = rel(cy, ry, v);
+    const IxF third{ix_limbs(1537228672809129301LL), -62};  // 2^62 / 3
+    const IxV D = ix_times(ix_split(ix_halved(ix_plus(ux, vy))), third);
+    const IxF a = ix_up(ix_halved(ix_minus(ux, D))), b = ix_up(ix_halved(ix_plus(uy, vx))), d = ix_up(ix_halved(ix_minus(vy, D)));
+    auto twice = [](IxV t) { return IxV{t.v, t.e + 1}; };
+    c1 = ix_up(ix_plus(twice(ix_times(a, nx)), ix_times(b, ny)));
+    c2 = ix_up(ix_plus(ix_times(b, nx), twice(ix_times(d, ny))));
+  }
+  out(1, ix_double(ix_times(c1, M)));
+  out(2, ix_double(ix_times(c2, M)));
   // energy: M (u.c + gamma/Pr H), H = grad E.S - u.(grad m.S) - B.(grad B.S) + X grad rho.S
-  const uint32_t gE = ge;
-  const int e1 = ix_exp<4>(gE) + eS + 60, e4 = eX + erS + 61;
-  int e3 = egB + eS + 60;
-  const int64_t t1 = contracted(ix_limbs(ix_align<4>(g(0, 4), gE)), ix_limbs(ix_align<4>(g(1, 4), gE)));
-  const int64_t yx = ix_align<4>(g(0, 6), gb), xy = ix_align<4>(g(1, 5), gb);
-  Limbs bxS, byS;
-  ix_up2(contracted(ix_limbs(ix_align<4>(g(0, 5), gb)), ix_limbs(xy)), contracted(ix_limbs(yx), ix_limbs(ix_align<4>(g(1, 6), gb))), e3,
-         bxS, byS);
-  const int64_t t3 = ix_prod(bxS, bx) + ix_prod(byS, by);
-  e3 += eB + 61;
-  const int64_t t4 = ix_prod(X, rS);
-  int KH = ix_max(ix_max(e1, e2), ix_max(e3, e4)) + 2;
-  int64_t H, uc = ix_prod(c1, u) + ix_prod(c2, v);  // [61.4]
-  int euc = ec + eu + 61;
+  const IxF yx = ix_load(g(0, 6)), xy = ix_load(g(1, 5));
+  IxV H = ix_minus(ix_plus(along(ix_load(g(0, 4)), ix_load(g(1, 4))), ix_times(X, rS)), t2);  // [62.6]
+  H = ix_minus(H, ix_plus(ix_times(ix_up(along(ix_load(g(0, 5)), xy)), bx), ix_times(ix_up(along(yx, ix_load(g(1, 6)))), by)));  // [63 - ]
+  IxV uc = ix_plus(ix_times(c1, u), ix_times(c2, v));  // [61]
   double F3 = 0.0;
-  int64_t bzS = 0;
-  int ebz = 0;
+  IxF bzS{Limbs{0, 0}, 0};
   if (hasz) {
-    const int egz = ix_exp<4>(gz), ez = egz + eS + 60;
-    ebz = ix_exp<4>(gw) + eS + 60;
-    const int64_t mzS = contracted(ix_limbs(ix_align<4>(g(0, 3), gz)), ix_limbs(ix_align<4>(g(1, 3), gz)));
-    bzS = contracted(ix_limbs(ix_align<4>(g(0, 7), gw)), ix_limbs(ix_align<4>(g(1, 7), gw)));
-    const int er = erS + ew + 61, K3 = ix_max(ez, er) + 1;
-    const int64_t c3 = ix_shr(mzS, K3 - ez) - ix_shr(ix_prod(rS, w), K3 - er);  // [60.5]
-    F3 = ix_double(ix_mul(c3, M), K3 + eM + 62);
-    const int e5 = ez + ew + 61, e6 = ebz + eBz + 61;
-    KH = ix_max(KH, ix_max(e5, e6) + 2);
-    H = -ix_shr(ix_prod(ix_limbs(mzS), w), KH - e5) - ix_shr(ix_prod(ix_limbs(bzS), bz), KH - e6);
-    const int e7 = K3 + ew + 61, K = ix_max(euc, e7) + 1;
-    uc = ix_shr(uc, K - euc) + ix_shr(ix_prod(ix_limbs(c3), w), K - e7);
-    euc = K;
-  } else {
-    H = 0;
+    const IxF mzS = ix_up(along(ix_load(g(0, 3)), ix_load(g(1, 3))));
+    bzS = ix_up(along(ix_load(g(0, 7)), ix_load(g(1, 7))));
+    const IxF c3 = ix_up(ix_minus(ix_halved(ix_whole(mzS)), ix_times(rS, w)));
+    F3 = ix_double(ix_times(c3, M));
+    H = ix_minus(ix_halved(H), ix_plus(ix_times(mzS, w), ix_times(bzS, bz)));
+    uc = ix_plus(uc, ix_times(c3, w));  // [61.6]
   }
   out(3, F3);
-  H += ix_shr(t1, KH - e1) - ix_shr(t2, KH - e2) - ix_shr(t3, KH - e3) + ix_shr(t4, KH - e4);  // [61.1]
-  const Limbs Hl = ix_up(H, KH);
-  const int eH = KH + gas.ekap + 61, K4 = ix_max(euc, eH) + 1;
-  int64_t F4 = ix_mul(ix_shr(uc, K4 - euc) + ix_shr(ix_prod(Hl, gas.kap), K4 - eH), M);  // [60]
-  int eF4 = K4 + eM + 62;
+  IxV F4 = ix_times(ix_up(ix_halved(ix_plus(uc, ix_times(ix_up(ix_halved(H)), gas.kap)))), M);  // [60]
   double F5 = 0.0, F6 = 0.0, F7 = 0.0;
   if (eta != 0.0) {  // resistive terms: F_B = eta (-Jz sy, Jz sx, grad Bz.S), the energy takes B.F_B
-    const Limbs et = ix_limbs(ix_align<3>(eta, mt));
-    const int eet = ix_exp<3>(mt);
-    int eJ = egB + eet + 62, eR = eB + eS + 60;
-    const int64_t j = ix_mul(yx - xy, et);  // [60]
-    Limbs jl, jn;
-    ix_up2(j, -j, eJ, jl, jn);
-    F5 = ix_double(ix_prod(jn, ny), eJ + eS + 61);
-    F6 = ix_double(ix_prod(jl, nx), eJ + eS + 61);
-    IxSum t;  // By sx - Bx sy
-    t.add(by, nx);
-    IxSum t_;
-    t_.add(bx, ny);
-    const Limbs Rl = ix_up(t.value4() - t_.value4(), eR);
-    int64_t R = ix_prod(jl, Rl);  // [60.5]
-    eR += eJ + 61;
+    const IxF et = ix_load(eta);
+    const IxF J = ix_up(ix_times(ix_up(ix_halved(ix_minus(ix_whole(yx), ix_whole(xy)))), et));
+    const IxV jy = ix_times(J, ny);
+    F5 = ix_double(-jy.v, jy.e);
+    F6 = ix_double(ix_times(J, nx));
+    IxV R = ix_times(J, ix_up(ix_minus(ix_times(by, nx), ix_times(bx, ny))));
     if (hasz) {
-      const int64_t f7 = ix_mul(bzS, et);  // [59.5]
-      const int e7 = ebz + eet + 62, e8 = e7 + eBz + 61, K = ix_max(eR, e8) + 1;
-      F7 = ix_double(f7, e7);
-      R = ix_shr(R, K - eR) + ix_shr(ix_prod(ix_limbs(f7), bz), K - e8);
-      eR = K;
+      const IxF f7 = ix_up(ix_times(bzS, et));
+      F7 = ix_double(ix_whole(f7));
+      R = ix_plus(R, ix_times(f7, bz));
     }
-    const int K = ix_max(eF4, eR) + 1;
-    F4 = ix_shr(F4, K - eF4) + ix_shr(R, K - eR);
-    eF4 = K;
+    F4 = ix_plus(F4, R);
   }
-  out(4, ix_double(F4, eF4));
+  out(4, ix_double(F4));
   out(5, F5);
   out(6, F6);
   out(7, F7);
@@ -535,7 +409,7 @@ FIX_HD bool rusanov_int(Q&& q, double ux, double uy, const IxGas& gas, double sc
     const int KS = ix_max(ix_max(E.e + 1, kr.e), b2.e);
     const int64_t S = ix_shr(ix_whole(E).v, KS - E.e - 1) - ix_at(kr, KS) - ix_at(b2, KS);
     ok = ok && S >= 0;
-    const IxV p = ix_times(IxF{ix_limbs(S & ~(S >> 63)), KS}, IxF{gas.g, gas.eg});  // [60]
+    const IxV p = ix_times(IxF{ix_limbs(S & ~(S >> 63)), KS}, gas.g);  // [60]
     const IxF pt = ix_up(ix_halved(ix_plus(p, IxV{b2.v, b2.e - 1})));
     const IxF Ep = ix_split(ix_halved(ix_plus(ix_whole(E), ix_whole(pt))));
     const IxV ge = ix_minus(ix_times(Ep, V), ix_times(ix_up(ix_halved(mB)), bnl));  // [61]
@@ -554,7 +428,7 @@ FIX_HD bool rusanov_int(Q&& q, double ux, double uy, const IxGas& gas, double sc
   // rs = rho_l + rho_r, cf^2 = (T + sqrt(T^2 - 2 P bn^2)) / (2 rs).  Operands are shifted up to full
   // length before they are multiplied on: a field that reverses across the face leaves B far below
   // either side's (with its leading zeros the speed lost up to 2^-26 of itself at a beta of 1e-8)
-  P = ix_times(ix_split(P), IxF{gas.gam, gas.egam});
+  P = ix_times(ix_split(P), gas.gam);
   if (!ok || P.v <= 0) return false;
   IxF eig;  // -eigv
   {

@@ -155,3 +155,47 @@ def test_face_flux(driver, tmp_path, kind, sides, normal, gam):  # noqa: F811
     F = S[:, None] * (Fl + Fr - eig[:, None] * J)
     bound = abs(S[:, None]) * (EPS * (tl + tr + eig[:, None] * abs(J)) + deig[:, None] * abs(J))
     assert np.all(abs(out[:, 1:9] - F)[took] <= bound[took])
+
+
+@pytest.mark.parametrize("coef", ["both", "viscous", "resistive"])
+@pytest.mark.parametrize("normal", ["axis", "near axis", "any"])
+@pytest.mark.parametrize("kind", STATES)
+def test_viscous_flux(driver, tmp_path, kind, normal, coef):  # noqa: F811
+    """Up to twelve products and sums of 2^-55 lie one behind the other: 2^-51 of the terms."""
+    rng = np.random.default_rng(5000 + 10 * STATES.index(kind) + len(normal) + 100 * len(coef))
+    n, gam, Pr = 3000, 5.0 / 3, 0.72
+    q = mixed(rng, kind, n, gam)
+    G = np.stack([spread(rng, 16 * n, -12 if kind == "transverse" else -18)]).reshape(n, 2, 8)
+    if kind == "transverse":
+        i = np.where(abs(q[:, 1]) > abs(q[:, 2]), 1, 0)  # the transverse variables of the plane
+        for k in (1, 5):
+            G[np.arange(n), :, k + i] *= (10.0 ** rng.uniform(-18, 0, n))[:, None]
+    if "mixed" != kind:
+        G[:, :, [3, 7]] = 0.0
+    S = normals(rng, normal, n) * np.exp(rng.uniform(-8, 8, (n, 1)))
+    mu = 1e-3 * np.exp(rng.uniform(-2, 2, (n, 1))) * (coef != "resistive")
+    eta = 1e-3 * np.exp(rng.uniform(-2, 2, (n, 1))) * (coef != "viscous")
+    out = evaluate(driver, tmp_path, 2, np.concatenate([q, G.reshape(n, 16), mu, eta, S, np.full((n, 1), gam)], 1))
+    assert np.all(out[:, 0] == 1)
+
+    def flux(q, G, N, M, H, s):
+        """The flux (s = -1: differences as they are) or the sums of its terms' magnitudes (s = 1, all inputs >= 0)."""
+        rho, E, B = q[:, 0], q[:, 4], q[:, 5:8]
+        u = q[:, 1:4] / rho[:, None]
+        dot = lambda a, b: (a * b).sum(-1)  # noqa: E731
+        rel = G[:, :, 1:4] + s * G[:, :, :1] * u[:, None]  # rho grad u
+        D = (rel[:, 0, 0] + rel[:, 1, 1]) / 3
+        sh = rel[:, 0, 1] + rel[:, 1, 0]
+        c = np.stack([2 * (rel[:, 0, 0] + s * D) * N[:, 0] + sh * N[:, 1], sh * N[:, 0] + 2 * (rel[:, 1, 1] + s * D) * N[:, 1],
+                      dot(rel[:, :, 2], N)], 1)
+        X = dot(u, u) + dot(B, B) / (2 * rho) + s * E / rho
+        GS = (G * N[:, :, None]).sum(1)
+        heat = GS[:, 4] + s * dot(u, GS[:, 1:4]) + s * dot(B, GS[:, 5:8]) + X * GS[:, 0]
+        J = H * (G[:, 0, 6] + s * G[:, 1, 5])
+        F7 = H * GS[:, 7]
+        energy = M / rho * (dot(u, c) + LD(gam) / LD(Pr) * heat) + J * (B[:, 1] * N[:, 0] + s * B[:, 0] * N[:, 1]) + F7 * B[:, 2]
+        return np.stack([0 * rho, *(M / rho * c.T), energy, s * J * N[:, 1], J * N[:, 0], F7], 1)
+
+    a = [x.astype(LD) for x in (q, G, S, mu[:, 0], eta[:, 0])]
+    F, scale = flux(*a, -1), flux(*[abs(x) for x in a], 1)
+    assert np.all(abs(out[:, 1:9] - F) <= 2 * EPS * scale)
