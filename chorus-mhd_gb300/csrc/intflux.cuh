@@ -205,6 +205,25 @@ FIX_HD IxF ix_up(IxV a) {
 }
 FIX_HD double ix_double(IxV a) { return ix_double(a.v, a.e); }
 
+// the products q(r) s(r) of a line as integers X_r, |X_r| < 2^58, aligned to the largest of them;
+// returns their exponent, or a number above kIxNoLine / 2 where an operand has the exponent
+// kIxNoLine (a value that the integer form leaves out)
+constexpr int kIxNoLine = 1 << 24;
+template <int NI, class Q, class S>
+FIX_HD int ix_line_products(Q&& q, S&& s, int64_t (&X)[NI]) {
+  int e[NI], K = -kIxNoLine;
+#pragma unroll
+  for (int r = 0; r < NI; r++) {
+    const IxV p = ix_times(q(r), s(r));
+    X[r] = p.v;
+    e[r] = p.e;
+    K = ix_max(K, p.e);
+  }
+#pragma unroll
+  for (int r = 0; r < NI; r++) X[r] = ix_shr(X[r], K - e[r] + 2);
+  return K + 2;
+}
+
 // constants of a solve, prepared once (host or device): half of gamma - 1, gamma, gamma / Pr
 struct IxGas {
   IxF g, gam, kap;

@@ -742,7 +742,7 @@ static __device__ __noinline__ double e3_fp64(int64_t V0, int k0, int64_t V1, in
 
 // shared memory of the pass for epb cells (e2_cells)
 constexpr size_t e2_smem(int N, int epb) {
-  return (size_t)epb * ((size_t)2 * (N + 1) * N * (72 + 16) + (size_t)N * N * (128 + 8 + 4) + (size_t)N * 8 * 4 + 2 * N * 4) + 64;
+  return (size_t)epb * ((size_t)2 * (N + 1) * N * (72 + 16 + 8) + (size_t)N * N * (128 + 8 + 4) + (size_t)N * 16 * 4) + 64;
 }
 
 template <int N, class O>
@@ -752,18 +752,17 @@ __device__ __forceinline__ void e2_cells(const SolveDev& s, const int* cells, in
   // form: grad_x Q = (1/J) [d/dxi (S1(1,1) Q) + d/deta (S2(2,1) Q)], grad_y the same with
   // the second metric entries, i.e. the divergence of the products of the face-averaged
   // flux-point states with the metric terms, differentiated along the lines on the integer
-  // pipes as in E3.  The products are integers too: a line's states aligned once serve both
-  // metric entries.  (128x128 cells, N = 5, every cell: 0.173 ms a stage with the products, the
-  // family sums and 1/J in FP64, 0.125 ms like this.)  An
-  // operand is cut at 2^-58 of its line's largest, a product at 2^-61.
+  // pipes as in E3.  The products are integers too (ix_line_products), each from operands with
+  // their own exponents and aligned to the line's largest product, so that a metric entry that is
+  // small beside the other one (flat cells) or along a part of the line keeps its bits.
   constexpr int NS = D<N>::NS, NF1 = D<N>::NF1, NFP = D<N>::NFP;
   double* sQ = sm;                                              // [n][NFP][9] Q
-  Limbs* sS = reinterpret_cast<Limbs*>(sQ + n * NFP * 9);       // [n][NFP][2] metric entries, aligned per line
+  Limbs* sS = reinterpret_cast<Limbs*>(sQ + n * NFP * 9);       // [n][NFP][2] metric entries (ix_load)
   double* sG = reinterpret_cast<double*>(sS + n * NFP * 2);     // [n][NS][16] grad Q (d*8 + k)
   int64_t* sJ = reinterpret_cast<int64_t*>(sG + n * NS * 16);   // [n][NS] 1/J as an integer
   int* sE = reinterpret_cast<int*>(sJ + n * NS);                // [n][NS] and its exponent
-  int* sK = sE + n * NS;                                        // [n][N][8] exponents of the xi-line sums
-  int* sM = sK + n * N * 8;                                     // [n][2N] exponents of the lines' metric entries
+  int* sK = sE + n * NS;                                        // [n][N][8][2] exponents of the xi-line sums
+  int* sX = sK + n * N * 16;                                    // [n][NFP][2] exponents of the metric entries
   for (int le = 0; le < n; le++)
     block_copy_async(sQ + le * NFP * 9, s.Qvf + (size_t)cells[le] * NFP * 9, NFP * 9);
   cp_async_commit();
@@ -774,24 +773,12 @@ __device__ __forceinline__ void e2_cells(const SolveDev& s, const int* cells, in
     sJ[i] = ix_align<2>(j, m);
     sE[i] = m >= kIxLow && m < kIxHigh ? ix_exp<2>(m) : kE3Fp64;
   }
-  // flux point r of line l of a cell: the xi lines, then the eta lines
-  auto line_point = [](int l, int r) { return l < N ? l * (N + 1) + r : NF1 + r * N + (l - N); };
-  for (int i = threadIdx.x; i < n * 2 * N; i += blockDim.x) {
-    const int le = i / (2 * N), l = i - le * 2 * N;
-    const double2* met = reinterpret_cast<const double2*>(s.met) + (size_t)cells[le] * NFP;
-    double2 a[N + 1];
-    uint32_t m = 0;
-#pragma unroll
-    for (int r = 0; r <= N; r++) a[r] = met[line_point(l, r)];
-#pragma unroll
-    for (int r = 0; r <= N; r++) m = ix_max(m, ix_max(ix_abs_word(a[r].x), ix_abs_word(a[r].y)));
-    sM[i] = m >= kIxLow && m < kIxHigh ? ix_exp<4>(m) : kE3Fp64;
-#pragma unroll
-    for (int r = 0; r <= N; r++) {
-      Limbs* o = sS + (le * NFP + line_point(l, r)) * 2;
-      o[0] = ix_limbs(ix_align<4>(a[r].x, m));
-      o[1] = ix_limbs(ix_align<4>(a[r].y, m));
-    }
+  for (int i = threadIdx.x; i < n * NFP * 2; i += blockDim.x) {
+    const int le = i / (NFP * 2);
+    const double m = s.met[(size_t)cells[le] * NFP * 2 + i - le * NFP * 2];
+    const IxF a = ix_load(m);
+    sS[i] = a.m;
+    sX[i] = ix_abs_word(m) < kIxHigh ? a.e : kIxNoLine;
   }
   cp_async_wait();
   __syncthreads();
@@ -810,25 +797,25 @@ __device__ __forceinline__ void e2_cells(const SolveDev& s, const int* cells, in
   for (int fam = 0; fam < 2; fam++) {
     for (int t = threadIdx.x; t < n * N * 8; t += blockDim.x) {
       const int k = t & 7, el = t >> 3, le = el / N, ln = el - le * N;
-      const int fp0 = le * NFP + (fam ? NF1 + ln : ln * (N + 1)), fps = fam ? N : 1, eS = sM[le * 2 * N + fam * N + ln];
-      uint32_t m = 66u << 20;
+      const int fp0 = le * NFP + (fam ? NF1 + ln : ln * (N + 1)), fps = fam ? N : 1;
+      uint32_t m = 0;
 #pragma unroll
       for (int r = 0; r <= N; r++) m = ix_max(m, ix_abs_word(sQ[(fp0 + r * fps) * 9 + k]));
-      const bool ok = m < kIxHigh && eS != kE3Fp64;
-      const int kv = ok ? ix_exp<4>(m) + eS + 62 + 58 - O::ops().MS : kE3Fp64;
-      Limbs q[N + 1];
-#pragma unroll
-      for (int r = 0; r <= N; r++) q[r] = ix_limbs(ix_align<4>(sQ[(fp0 + r * fps) * 9 + k], m));
-      if (!fam) sK[t] = kv;
 #pragma unroll 1
       for (int d = 0; d < 2; d++) {
         double* g = sG + le * NS * 16 + d * 8 + k;
+        int64_t X[N + 1];
+        const int eX = ix_line_products<N + 1>([&](int r) { return ix_load(sQ[(fp0 + r * fps) * 9 + k]); },
+                                               [&](int r) { const int i = (fp0 + r * fps) * 2 + d; return IxF{sS[i], sX[i]}; }, X);
+        const bool ok = m < kIxHigh && eX < kIxNoLine / 2;
+        const int kv = ok ? eX + 58 - O::ops().MS : kE3Fp64;
+        if (!fam) sK[2 * t + d] = kv;
         auto finish = [&](int i, int64_t V) {
           if (!fam) {
             g[(ln * N + i) * 16] = __longlong_as_double(V);
             return;
           }
-          const int p = i * N + ln, ps = le * NS + p, eJ = sE[ps], k0 = sK[(le * N + i) * 8 + k];
+          const int p = i * N + ln, ps = le * NS + p, eJ = sE[ps], k0 = sK[((le * N + i) * 8 + k) * 2 + d];
           const int64_t V0 = __double_as_longlong(g[p * 16]);
           double a;
           if (ok && k0 != kE3Fp64 && eJ != kE3Fp64) {
@@ -843,9 +830,6 @@ __device__ __forceinline__ void e2_cells(const SolveDev& s, const int* cells, in
           if (keep) s.nQs[((size_t)cells[le] * NS + p) * 18 + 9 * d + k] = a;
         };
         if (ok) {
-          int64_t X[N + 1];
-#pragma unroll
-          for (int r = 0; r <= N; r++) X[r] = ix_mul(q[r], sS[(fp0 + r * fps) * 2 + d]);
           fix_mirror_core<N, N + 1, -1>(X, O::ops().MH, O::ops().ML, finish);
         } else {
           const double* met = s.met + (size_t)cells[le] * NFP * 2 + d;
