@@ -233,20 +233,20 @@ FIX_HD double fix_round_v(int64_t V, int k) {
 }
 
 // the same through the conversion instruction (nearest, ties to even), which takes the FP64
-// unit of its scheduler for 64 clocks but saves some 20 instructions
+// unit of its scheduler for 64 clocks but saves some 20 instructions.  The exponent is added to the
+// bits, here as there, so a result past the largest double would come out as some other number:
+// the callers' windows keep |V 2^k'| below 2^1023.
 template <bool CHECK>
 FIX_HD double fix_cvt_v(int64_t V, int k) {
 #ifdef __CUDA_ARCH__
-  const double d = __ll2double_rn(V);
-  const int hi = __double2hiint(d);
-  int h = hi + (int)((uint32_t)(k - 1) << 20);
-  if (hi == 0) h = 0;
-  if (CHECK && ((hi >> 20) & 0x7ff) + k - 1 < 1) return 0.0;
-  return __hiloint2double(h, __double2loint(d));
+  const uint64_t d = (uint64_t)__double_as_longlong(__ll2double_rn(V));
 #else
-  const double d = __builtin_ldexp((double)V, k - 1);
-  return CHECK && __builtin_fabs(d) < 0x1p-1022 ? 0.0 : d;
+  const uint64_t d = fix_bits((double)V);
 #endif
+  const uint32_t hi = (uint32_t)(d >> 32);
+  if (CHECK && (int)((hi >> 20) & 0x7ff) + k - 1 < 1) return 0.0;
+  const uint32_t h = hi == 0 ? 0 : hi + ((uint32_t)(k - 1) << 20);
+  return fix_double(((uint64_t)h << 32) | (uint32_t)d);
 }
 // y = C v for C (NO x NI) in mirror form (fix_mirror_coefs: per row r < (NO+1)/2 the
 // coefficients [P(0..NI/2) | Q(0..NI/2) | R]), scaled by 2^k as fix_dot.  With

@@ -18,8 +18,8 @@
 //     that of the FP64 forms, component by component, typically half of it.
 //
 // The integer form takes finite states with a normal positive density and magnitudes within
-// a wide window (2^-200 .. 2^200; zero and smaller values of all but the density, energy and
-// metric as well);
+// a wide window (2^-200 .. 2^200, the viscous flux 2^-120 .. 2^120; zero and smaller values of all but
+// the density, energy and metric as well), so that no result leaves the range of a double;
 // everything else (infinities, NaNs, zero or negative density, a negative pressure, a density ratio
 // above 8 across a face, a negative discriminant) is left to the FP64 form, whose results on
 // such states the caller keeps.
@@ -166,6 +166,7 @@ struct IxV {  // a product or a sum: v 2^e
 };
 
 constexpr uint32_t kIxLow = 823u << 20, kIxHigh = 1223u << 20;  // 2^-200 .. 2^200
+constexpr uint32_t kIxVLow = 903u << 20, kIxVHigh = 1143u << 20;  // 2^-120 .. 2^120: the viscous flux
 constexpr uint32_t kIxZero = 66u << 20;  // magnitude words below: a zero
 
 // x without rounding, 2^60 <= |m| < 2^61; both limbs carry the sign.  A zero gets the exponent of
@@ -286,7 +287,8 @@ FIX_HD bool iflux_int(Q&& q, double sx, double sy, const IxGas& gas, Out&& out) 
 // these are): q(k) the state, g(d, k) its gradient, mut and eta the viscosity and resistivity.
 // out(k, value) takes components 1..7; false, without output, where the integer form does not
 // apply.  The first output comes after the last use of q, which may therefore lie in the outputs'
-// place.
+// place.  Magnitudes of up to 2^120 (and a density down to 2^-120) are taken: the largest product,
+// the viscosity times the squared velocity times the velocity gradient, stays below 2^1000.
 template <class Q, class G, class Out>
 FIX_HD bool vflux_int(Q&& q, G&& g, double mut, double eta, double sx, double sy, const IxGas& gas, Out&& out) {
   auto w1 = [&](int k) { return ix_abs_word(q(k)); };
@@ -296,7 +298,7 @@ FIX_HD bool vflux_int(Q&& q, G&& g, double mut, double eta, double sx, double sy
   const uint32_t mq = ix_max(ix_max(ix_max(w1(1), w1(2)), ix_max(w1(5), w1(6))), ix_max(w1(4), r));
   const uint32_t mg = ix_max(ix_max(ix_max(w2(0), w2(1)), ix_max(w2(2), w2(4))), ix_max(w2(5), w2(6)));
   const uint32_t ms = ix_max(ix_abs_word(sx), ix_abs_word(sy)), mc = ix_max(ix_abs_word(mut), ix_abs_word(eta));
-  if (ix_max(ix_max(ix_max(mq, mg), ix_max(mz, ms)), mc) >= kIxHigh || r < kIxLow || ms < kIxLow) return false;
+  if (ix_max(ix_max(ix_max(mq, mg), ix_max(mz, ms)), mc) >= kIxVHigh || r < kIxVLow || ms < kIxVLow) return false;
   const bool hasz = mz >= kIxZero;
   const IxF nx = ix_load(sx), ny = ix_load(sy), ri = ix_inverse(q(0));
   const IxF M = ix_up(ix_times(ix_load(mut), ri));  // mu / rho
