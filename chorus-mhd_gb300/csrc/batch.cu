@@ -386,7 +386,7 @@ static int batch_rebuild(ChorusBatch* b) {
       for (int k = 0; k < n; k++) grp[gidx(pass, sl.N)].push_back(make_int4(i, k, n, 0));
     };
     walk(PE2, o.epb[1]);
-    if (v_pass(sl.sd) && (sl.sd.artiv || !sl.sd.skip)) walk(PV, o.pass[PV].epb);
+    if (v_pass(sl.sd) && viscous(sl.sd)) walk(PV, o.pass[PV].epb);
     cut(PE3, sl.NC, o.epb[2]);
     cut(PCT, sl.NC, o.epb[3]);
     cut(PCTF, sl.nfp_two, kFaceTile);

@@ -1117,9 +1117,12 @@ constexpr long long kVPassPoints = 49152;
 // work that is exactly zero must not change a result.)
 __host__ __device__ inline bool v_pass(const SolveDev& s) { return (long long)s.NC * s.N * s.N >= kVPassPoints; }
 
+// Can a solve have a viscous flux at all?
+__host__ __device__ inline bool viscous(const SolveDev& s) { return s.artiv || s.mu != 0.0 || s.eta0 != 0.0; }
+
 // what E3 does about the viscous flux (e3_body): keep = the inviscid flux stays downloadable
 __host__ __device__ inline int e3_visc(const SolveDev& s, bool keep) {
-  return !s.artiv && s.skip ? 0 : !v_pass(s) ? 1 : keep ? 2 : 0;
+  return !viscous(s) ? 0 : !v_pass(s) ? 1 : keep ? 2 : 0;
 }
 
 // does a stage only need its increment cR * resid, so that cR is folded into 1/J?

@@ -116,7 +116,7 @@ void launch_e2<kN>(const SolveDev& s, const Launch& L, cudaStream_t st, bool kee
   const int nsm = sm_count();
   const int all2 = grid_cells(s.NC, L.epb);
   launch_pdl(k_e2<kN>, s.skip ? std::min(all2, 8 * nsm) : all2, L.threads, e2_smem(kN, L.epb), st, s, L.epb, (int)keep);
-  if (v_pass(s) && (s.artiv || !s.skip)) {
+  if (v_pass(s) && viscous(s)) {
     const int allv = grid_cells(s.NC, v_epb(kN));
     launch_pdl(k_v<kN>, s.skip ? std::min(allv, 8 * nsm) : allv, v_threads(kN), v_smem(kN), st, s, keep ? s.Ft : s.Fc);
   }

@@ -94,7 +94,8 @@ int chorus_gpu_bind(const ChorusDims* dims, const int32_t* IF2C, const int32_t* 
                     const double* Mmat, const double* S1, const double* S2, const double* Jac,
                     const ChorusParams* params, int32_t device, ChorusCtx** ctx);
 int chorus_gpu_free(ChorusCtx* ctx);
-/* Change dt / mu / eta0 / ARTIV of a bound context (setup2d.f90:72,77,81). */
+/* Change dt / mu / eta0 / ARTIV of a bound context (setup2d.f90:72,77,81).  A context that comes
+ * to need viscous work allocates for it here: CHORUS_ENOMEM leaves the parameters as they were. */
 int chorus_gpu_set_params(ChorusCtx* ctx, const ChorusParams* params);
 
 /* Resident state Q(9,N,N,NCELL) (setup2d.f90:54). */
