@@ -80,7 +80,8 @@ FIX_HD int fix_clz64(uint64_t u) {
 FIX_HD int64_t fix_mad(int a, int b, int64_t acc) {
 #ifdef __CUDA_ARCH__
   uint32_t lo = (uint32_t)acc, hi = (uint32_t)((uint64_t)acc >> 32);
-  asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.s32 %1, %2, %3, %1;" : "+r"(lo), "+r"(hi) : "r"(a), "r"(b));
+  // (the low word is written before the factors are read again: early clobber)
+  asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.s32 %1, %2, %3, %1;" : "+&r"(lo), "+r"(hi) : "r"(a), "r"(b));
   return (int64_t)(((uint64_t)hi << 32) | lo);
 #else
   return acc + (int64_t)a * b;
