@@ -203,10 +203,10 @@ FIX_HD bool fix_line_ok(uint32_t a) {
   return a == 0 || a - ((uint32_t)kFixEmaxMin << 20) < ((uint32_t)(kFixEmaxFast + 1 - kFixEmaxMin) << 20);
 }
 
-// V 2^k' (|V| < 2^63) rounded to nearest (ties up in magnitude), k' = k - 1 with k as in
-// fix_round; CHECK: results below the normal range are flushed to zero (otherwise the
-// caller knows that there are none)
-template <bool CHECK>
+// V 2^k' (|V| < 2^63) rounded to nearest, k' = k - 1 with k as in fix_round; CHECK: results
+// below the normal range are flushed to zero (otherwise the caller knows that there are
+// none); ties up in magnitude, or (EVEN) to even as the conversion instruction rounds them
+template <bool CHECK, bool EVEN = false>
 FIX_HD double fix_round_v(int64_t V, int k) {
   const int64_t s = V >> 63;
   const uint64_t u = (uint64_t)((V ^ s) - s);
@@ -222,8 +222,8 @@ FIX_HD double fix_round_v(int64_t V, int k) {
 #else
   const int lz = uh ? __builtin_clz(uh) : 32;
 #endif
-  const uint64_t top = ((((uint64_t)uh << 32) | ul) << (lz - 1)) + 0x200;  // leading bit 62 (lz >= 1)
-  const uint64_t mant = top >> 10;                                         // 2^52 .. 2^53
+  const uint64_t top = (((uint64_t)uh << 32) | ul) << (lz - 1);                      // leading bit 62 (lz >= 1)
+  const uint64_t mant = (top + (EVEN ? 0x1ff + ((top >> 10) & 1) : 0x200)) >> 10;  // 2^52 .. 2^53
   const int E = e - lz;
   uint32_t h = (uint32_t)(mant >> 32) + ((uint32_t)E << 20);
   uint32_t l = (uint32_t)mant;
@@ -282,11 +282,17 @@ FIX_HD void fix_mirror_core(const int64_t (&X)[NI], const int* ch, const int* cl
     h = (int)(x >> kFixSplit);
     l = (int)(x & ((1 << kFixSplit) - 1)) - (1 << (kFixSplit - 1));
   };
+  // limbs of -x are those of x negated (half a limb is rounded away from zero), so that the products
+  // left out are too: a mirrored line, whose O change sign, has the mirrored sums to the bit
+  auto split_odd = [](int64_t x, int& h, int& l) {
+    h = (int)((x + kHalfL + (x >> 63)) >> kFixSplit);
+    l = (int)((uint32_t)x - ((uint32_t)h << kFixSplit));
+  };
   int eh[NP > 0 ? NP : 1], el[NP > 0 ? NP : 1], oh[NP > 0 ? NP : 1], ol[NP > 0 ? NP : 1];
 #pragma unroll
   for (int j = 0; j < NP; j++) {
     split(X[j] + X[NI - 1 - j] + kHalfL, eh[j], el[j]);
-    split(X[j] - X[NI - 1 - j] + kHalfL, oh[j], ol[j]);
+    split_odd(X[j] - X[NI - 1 - j], oh[j], ol[j]);
   }
   int mh = 0, ml = 0;
   if (NI & 1) split(X[NP] + kHalfL, mh, ml);
@@ -343,7 +349,7 @@ FIX_HD void fix_mirror_sums(const double (&v)[NI], int emax, const int* ch, cons
 
 template <int NO, int NI, int SIGMA, bool CHECK>
 FIX_HD void fix_mirror_line(const double (&v)[NI], int emax, const int* ch, const int* cl, int k, double (&y)[NO]) {
-  fix_mirror_sums<NO, NI, SIGMA>(v, emax, ch, cl, [&](int r, int64_t V) { y[r] = r < NO / 2 ? fix_cvt_v<CHECK>(V, k) : fix_round_v<CHECK>(V, k); });
+  fix_mirror_sums<NO, NI, SIGMA>(v, emax, ch, cl, [&](int r, int64_t V) { y[r] = r < NO / 2 ? fix_cvt_v<CHECK>(V, k) : fix_round_v<CHECK, true>(V, k); });
 }
 
 // the same for any finite line with emax <= kFixEmaxFast: lines below kFixEmaxMin are scaled
