@@ -499,11 +499,12 @@ __device__ __forceinline__ int active_cells(const SolveDev& s, int e0, int cnt, 
 // ---------------------------------------------------------------------------
 // F1: Rusanov flux on every face point (interfaceflux / CYCLOCFLUX / BCFLUX)
 // ---------------------------------------------------------------------------
-// the FP64 form of a face point's flux, for the states that the integer form leaves out:
-// a call, so that it takes no registers from the points that do not need it
+// the FP64 form of a face point's flux, for the states that the integer form leaves out, and the
+// left side's normal velocity: a call, so that it takes no registers from the points that do not
+// need it
 static __device__ __noinline__ double rusanov_fp64(const double* pl, const double* pr, const FaceNorm* fn, double gam,
-                                            double* Fh) {
-  double ql[9], qr[9], vnl, ev;
+                                            double* Fh, double& vnl) {
+  double ql[9], qr[9], ev;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     ql[k] = pl[k];
@@ -614,17 +615,17 @@ __device__ __forceinline__ unsigned long long f1_points(const SolveDev& s, int f
         F[2 * j] = a;
         F[2 * j + 1] = b;
       };
-      double ev;
+      double ev, vn = fma(ql[1], nrm.x, ql[2] * nrm.y);  // m.n, of the sign of u.n
       if (!rusanov_int([&](int side, int k) { return side ? qr[k] : ql[k]; }, nrm.x, nrm.y, s.gas, w.fn[buf][lane][1].x, ev, put)) {
         double Fd[8];
-        ev = rusanov_fp64(w.q[buf][0] + 9 * lane, w.q[buf][1] + 9 * lane, normal(t), s.gam, Fd);
+        ev = rusanov_fp64(w.q[buf][0] + 9 * lane, w.q[buf][1] + 9 * lane, normal(t), s.gam, Fd, vn);  // (a negative density among them)
 #pragma unroll
         for (int j = 0; j < 4; j++) put(j, Fd[2 * j], Fd[2 * j + 1]);
       }
       const unsigned long long e = ev_bits(ev, s.err);
       evb = e > evb ? e : evb;
-      // A_z from the upwind side (getrusanov.f90:99-103); the sign of u.n is that of m.n
-      const double az = fma(ql[1], nrm.x, ql[2] * nrm.y) > 0.0 ? ql[8] : qr[8];
+      // A_z from the upwind side (getrusanov.f90:99-103)
+      const double az = vn > 0.0 ? ql[8] : qr[8];
       s.Azf[gl] = az;
       if (gr >= 0) {
         s.Azf[gr] = az;
