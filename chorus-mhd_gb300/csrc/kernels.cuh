@@ -984,6 +984,12 @@ __device__ __forceinline__ void v_cells(const SolveDev& s, const int* cells, int
     const double mut = point_mu<N, O>(s, smu[le], fp);
     volatile double* q = sQ + 9 * t;
     const volatile double* gr = sG + 18 * t;
+    if (((__double_as_longlong(mut) | __double_as_longlong(s.eta0)) << 1) == 0) {
+      // no flux, whatever the gradient is: 0 times an infinity of a neighbour is not let in
+#pragma unroll
+      for (int k = 1; k < 8; k++) q[k] = 0.0;
+      continue;
+    }
     // (the flux takes the place of the point's state, which vflux_int has read by its first output)
     if (!vflux_int([&](int k) { return q[k]; }, [&](int d, int k) { return gr[9 * d + k]; }, mut, s.eta0, m.x, m.y, s.gas,
                    [&](int k, double f) { q[k] = f; }))
