@@ -221,7 +221,9 @@ struct ChorusCtx {
   int nface2 = 0, nface1 = 0;
   cudaStream_t st = nullptr;
   void* arena = nullptr;
-  size_t arena_bytes = 0, ft_bytes = 0;
+  size_t arena_bytes = 0;
+  void* ft = nullptr;  // SolveDev::Ft of a context that came to need it after its binding
+  size_t ft_bytes = 0;
   SolveDev sd{};
   double* red = nullptr;       // [4]: diag sums, eig as double
   double* h_pinned = nullptr;  // pinned staging for diag records
@@ -294,25 +296,6 @@ struct ArenaPlan {
   }
 };
 
-// bytes of one solve's device arena (the same allocation sequence as chorus_gpu_bind)
-static size_t arena_plan_bytes(int N, int NC, int nface2, int nface1, int k_stage) {
-  const int NS = N * N, NFP = 2 * (N + 1) * N;
-  const size_t nq = (size_t)NC * NS * 9, nfp = (size_t)NC * NFP;
-  ArenaPlan P;
-  P.take<double>(nq); P.take<double>(nq); P.take<double>(nq);
-  if (k_stage == 5) { P.take<double>(nq); P.take<double>(nq); P.take<double>(nq); }
-  P.take<double>(nq); P.take<double>(nfp * 9); P.take<double>(nfp * 8); P.take<double>(nfp);
-  P.take<double>((size_t)NC * NS * 18); P.take<double>(nfp * 18); P.take<double>((size_t)NC * NS * 2);
-  P.take<double>(nfp * 2); P.take<double>((size_t)NC * NS);
-  P.take<double>((size_t)NC * 2); P.take<double>((size_t)NC * 4); P.take<double>((size_t)NC * 2);
-  P.take<int4>(nface2 + 1); P.take<int2>(nface1 + 1); P.take<FaceNorm>((size_t)nface2 * N + 1);
-  P.take<FaceNorm>((size_t)nface1 * N + 1); P.take<unsigned long long>(4); P.take<unsigned int>(4);
-  P.take<double>(8); P.take<int>(NC); P.take<int>(NC); P.take<int4>(NC); P.take<int4>(NC);
-  P.take<double>((size_t)NC * NS * 2); P.take<double>(NC);
-  P.take<int>(NC); P.take<int>(NC);
-  return P.off;
-}
-
 // bytes of the total fluxes (SolveDev::Ft), which only pass V of a step's last stage writes: none
 // for a solve below the pass's size or without viscosity
 static size_t total_flux_bytes(int N, int NC, const ChorusParams& p) {
@@ -325,9 +308,28 @@ static size_t total_flux_bytes(int N, int NC, const ChorusParams& p) {
   return v_pass(s) && viscous(s) ? (size_t)NC * 2 * (N + 1) * N * 8 * sizeof(double) : 0;
 }
 
+// bytes of one solve's device arena (the same allocation sequence as chorus_gpu_bind)
+static size_t arena_plan_bytes(int N, int NC, int nface2, int nface1, const ChorusParams& p) {
+  const int NS = N * N, NFP = 2 * (N + 1) * N;
+  const size_t nq = (size_t)NC * NS * 9, nfp = (size_t)NC * NFP;
+  ArenaPlan P;
+  P.take<double>(nq); P.take<double>(nq); P.take<double>(nq);
+  if (p.k_stage == 5) { P.take<double>(nq); P.take<double>(nq); P.take<double>(nq); }
+  P.take<double>(nq); P.take<double>(nfp * 9); P.take<double>(nfp * 8); P.take<double>(nfp);
+  P.take<double>((size_t)NC * NS * 18); P.take<double>(nfp * 18); P.take<double>((size_t)NC * NS * 2);
+  P.take<double>(nfp * 2); P.take<double>((size_t)NC * NS);
+  P.take<double>((size_t)NC * 2); P.take<double>((size_t)NC * 4); P.take<double>((size_t)NC * 2);
+  P.take<int4>(nface2 + 1); P.take<int2>(nface1 + 1); P.take<FaceNorm>((size_t)nface2 * N + 1);
+  P.take<FaceNorm>((size_t)nface1 * N + 1); P.take<unsigned long long>(4); P.take<unsigned int>(4);
+  P.take<double>(8); P.take<int>(NC); P.take<int>(NC); P.take<int4>(NC); P.take<int4>(NC);
+  P.take<double>((size_t)NC * NS * 2); P.take<double>(NC);
+  P.take<int>(NC); P.take<int>(NC); P.take<char>(total_flux_bytes(N, NC, p));
+  return P.off;
+}
+
 // the total fluxes of a solve that has come to need them
-static int ensure_total_flux(ChorusCtx* c, int N, int NC, const ChorusParams& p) {
-  const size_t bytes = total_flux_bytes(N, NC, p);
+static int ensure_total_flux(ChorusCtx* c, const ChorusParams& p) {
+  const size_t bytes = total_flux_bytes(c->dims.N, c->dims.NCELL, p);
   if (!bytes || c->sd.Ft) return CHORUS_OK;
   if (ctx_device(c)) return CHORUS_ECUDA;
   void* m = nullptr;
@@ -336,6 +338,7 @@ static int ensure_total_flux(ChorusCtx* c, int N, int NC, const ChorusParams& p)
     cudaGetLastError();  // (not left for the next launch check)
     return set_err(CHORUS_ENOMEM, "cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
   }
+  c->ft = m;
   c->sd.Ft = (double*)m;
   c->ft_bytes = bytes;
   return CHORUS_OK;
@@ -394,7 +397,6 @@ int chorus_gpu_bind(const ChorusDims* dims, const int32_t* IF2C, const int32_t* 
   for (int w = 0; w < 4; w++) c->L[w] = default_launch(N, w);
   auto fail = [&](int code) {
     if (c->arena) cudaFree(c->arena);
-    if (c->sd.Ft) cudaFree(c->sd.Ft);
     if (c->st) cudaStreamDestroy(c->st);
     if (c->cp) cudaStreamDestroy(c->cp);
     for (auto& ev : c->ev)
@@ -541,14 +543,13 @@ int chorus_gpu_bind(const ChorusDims* dims, const int32_t* IF2C, const int32_t* 
          ofn2 = P.take<FaceNorm>(fn2.size() + 1), ofn1 = P.take<FaceNorm>(fn1.size() + 1),
          oeig = P.take<unsigned long long>(4), oerr = P.take<unsigned int>(4), ored = P.take<double>(8),
          oact = P.take<int>(NC), onv = P.take<int>(NC), onbr = P.take<int4>(NC), onbrlf = P.take<int4>(NC),
-         onQs9 = P.take<double>((size_t)NC * NS * 2), oSw = P.take<double>(NC), ovl = P.take<int>(NC), ogr = P.take<int>(NC);
+         onQs9 = P.take<double>((size_t)NC * NS * 2), oSw = P.take<double>(NC), ovl = P.take<int>(NC), ogr = P.take<int>(NC), oFt = P.take<char>(total_flux_bytes(N, NC, *params));
   c->arena_bytes = P.off;
-  if (P.off != arena_plan_bytes(N, NC, c->nface2, c->nface1, params->k_stage))
+  if (P.off != arena_plan_bytes(N, NC, c->nface2, c->nface1, *params))
     return fail(set_err(CHORUS_EINVAL, "internal: arena plan mismatch"));
   cudaError_t e = cudaMalloc(&c->arena, P.off);
   if (e != cudaSuccess)
     return fail(set_err(CHORUS_ENOMEM, "cudaMalloc(%zu bytes) failed: %s", P.off, cudaGetErrorString(e)));
-  if (int rc = ensure_total_flux(c, N, NC, *params)) return fail(rc);
   char* A = (char*)c->arena;
   SolveDev& s = c->sd;
   s.N = N;
@@ -594,6 +595,7 @@ int chorus_gpu_bind(const ChorusDims* dims, const int32_t* IF2C, const int32_t* 
   s.Sw = (double*)(A + oSw);
   s.vlist = (int*)(A + ovl);
   s.gr = (int*)(A + ogr);
+  s.Ft = total_flux_bytes(N, NC, *params) ? (double*)(A + oFt) : nullptr;
   c->skip_option = 1;
   s.skip = (params->mu == 0.0 && params->eta0 == 0.0) ? 1 : 0;
   s.eig = (unsigned long long*)(A + oeig);
@@ -637,7 +639,7 @@ int chorus_gpu_free(ChorusCtx* c) {
   drop_host_graphs(c);
   if (c->st) cudaStreamSynchronize(c->st);
   if (c->arena) cudaFree(c->arena);
-  if (c->sd.Ft) cudaFree(c->sd.Ft);
+  if (c->ft) cudaFree(c->ft);
   if (c->h_pinned) cudaFreeHost(c->h_pinned);
   if (c->cp) cudaStreamSynchronize(c->cp);
   if (c->st) cudaStreamDestroy(c->st);
@@ -658,7 +660,7 @@ static void drop_graphs(ChorusCtx* c) {
 int chorus_gpu_set_params(ChorusCtx* c, const ChorusParams* p) {
   if (!c || !p) return set_err(CHORUS_EINVAL, "null argument");
   if (p->k_stage != c->p.k_stage) return set_err(CHORUS_EINVAL, "k_stage is fixed at bind time");
-  if (int rc = ensure_total_flux(c, c->dims.N, c->dims.NCELL, *p)) return rc;
+  if (int rc = ensure_total_flux(c, *p)) return rc;
   c->p.dt = p->dt;
   c->p.mu = p->mu;
   c->p.eta0 = p->eta0;
@@ -1631,7 +1633,7 @@ int64_t chorus_mesh_device_bytes(const ChorusMesh* mh) {
   if (!mh) return -1;
   const Mesh& m = mh->m;
   const int nface2 = (int)m.IBFINTER.size() + m.NPAIR, nface1 = (int)m.IBFREE.size();
-  return (int64_t)(arena_plan_bytes(m.N, m.NCELL, nface2, nface1, m.params.k_stage) + total_flux_bytes(m.N, m.NCELL, m.params));
+  return (int64_t)arena_plan_bytes(m.N, m.NCELL, nface2, nface1, m.params);
 }
 
 int chorus_mesh_host_chunks(const ChorusMesh* mh, int32_t chunks, int32_t* K, int32_t* cut, int32_t* f2cut,
