@@ -1258,6 +1258,12 @@ int chorus_gpu_profile_stage(ChorusCtx* c, int32_t reps, double* ms) {
   }
   for (auto& e : ev) cudaEventDestroy(e);
   for (int k = 0; k < 6; k++) ms[k] = acc[k] / reps;
+  // stages that do not end a step keep no arrays: evaluate the state they left, as compresid does
+  RKStage keep = rk_blank();
+  keep.write_resid = 1;
+  enqueue_stage(c, keep, true);
+  c->se6_valid = c->plot_sensor;
+  CK(cudaGetLastError());
   return check_err_flag(c);
 }
 

@@ -218,7 +218,8 @@ int getrusanovflux_noalloc_gpu(int32_t n, double gam, const double* Qfl, const d
 void* chorus_gpu_stream(ChorusCtx* ctx);
 /* Run `reps` RK stages (stage 1 of RK_S5P3, state updated) launching each stage
  * kernel with CUDA events around it; ms[0..4] = mean duration of E1, F1, E2, F2, E3
- * and ms[5] = mean duration of a whole stage. */
+ * and ms[5] = mean duration of a whole stage.  The work arrays are then those of an
+ * evaluation at the state it leaves (untimed). */
 int chorus_gpu_profile_stage(ChorusCtx* ctx, int32_t reps, double* ms);
 /* Runtime options of a context:
  *   "diagnostics" (default 1): compute the norms of every tenth step in iterations_gpu;
