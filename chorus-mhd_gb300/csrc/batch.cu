@@ -349,7 +349,8 @@ static void order_shape(ChorusBatch* b, const BatchSlot& sl) {
     o.epb[p] = std::max(1, std::min(ctx_epb(sl.ctx, p), 64));
     o.threads[p] = std::max(32, std::min(ctx_threads(sl.ctx, p), 512));
   }
-  // an E2 tile tests up to one cell per thread: a multiple of the group size
+  // E2: no more cells than threads, which keeps shapes of many cells and few threads within the
+  // shared memory
   o.epb[1] = std::min(o.epb[1], o.threads[1]);
 #define CALL(n) pass_shapes<n>(b->nsm, o.epb, o.threads, o.pass)
   CHORUS_BATCH_SWITCH(sl.N, CALL)
@@ -460,9 +461,8 @@ static int batch_rebuild(ChorusBatch* b) {
 // one step: for every order present, its own chain on its own stream -- five stages of
 // E1, F1, E2, E3, then the CT projection -- forked from and joined to the batch stream.
 // The orders' solves share nothing, so the chains run concurrently and the block
-// scheduler mixes their CTAs (FP64-bound flux passes of one order beside the integer
-// line operators of another); within a chain every launch is programmatic (scheduled
-// while its predecessor drains, waiting for it at entry).  Each launch has one CTA per
+// scheduler mixes their CTAs; within a chain every launch is programmatic (launch_pdl), waiting for
+// its predecessor at entry.  Each launch has one CTA per
 // tile of the composition it was captured for.
 static void batch_enqueue_step(ChorusBatch* b) {
   BatchDev a;

@@ -164,9 +164,11 @@ static const Dispatch* dispatch_for(int N) {
 
 // default launch shapes per N (cells per CTA, threads per CTA)
 Launch default_launch(int N, int which) {
-  // which: 0 = E1, 1 = E2, 2 = E3, 3 = CT; cells per CTA and threads per CTA as the
-  // autotuner's sweep picked them on GB300 (2 M solution points); the CT passes take about
-  // 128/(2N) cells so that their (cell, line) loop fills the 128 threads
+  // which: 0 = E1, 1 = E2, 2 = E3, 3 = CT; cells per CTA and threads per CTA, E1's and E3's as
+  // sweeps of the present passes had them fastest on GB300 (2 M solution points), E2's of sweeps of
+  // an earlier form of the pass, at N = 4 with two cells (64x64 cells with fronts: a step 0.51 -> 0.47 ms
+  // together with spread()); the CT passes take about 128/(2N) cells so that their (cell, line) loop
+  // fills the 128 threads
   static const int epb[kMaxN + 1][4] = {{0}, {0}, {16, 6, 16, 32}, {8, 4, 8, 21}, {4, 2, 6, 16},
                                         {4, 2, 5, 12}, {4, 2, 3, 10}, {2, 1, 3, 9}, {2, 1, 2, 8}};
   static const int thr[kMaxN + 1][4] = {{0}, {0}, {64, 96, 96, 128}, {96, 128, 96, 128}, {96, 128, 128, 128},

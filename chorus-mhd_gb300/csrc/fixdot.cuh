@@ -2,34 +2,38 @@
 // applied in integer arithmetic.
 //
 // GB300 executes FP64 at 2 operations per clock per SM, while its integer pipes take
-// 64 lane-operations per clock each and sit nearly idle in these FP64-bound passes.  A
+// 64 lane-operations per clock each and sat nearly idle while these passes were in FP64.  A
 // line operator y_k = sum_j C_kj x_j with fixed coefficients is therefore cheaper as an
 // integer dot product:
 //   * the inputs of one line are aligned to the largest exponent among them and held as
-//     57-bit signed integers X_j = x_j * 2^(1075 + G - emax) (G = 4 guard bits below the
-//     53-bit significand of the largest input; smaller inputs lose only bits below
-//     2^-58 of the largest, by rounding),
+//     58-bit signed integers (5 guard bits below the 53-bit significand of the largest input;
+//     smaller inputs lose only bits below 2^-58 of the largest, by truncation),
 //   * the coefficients as 59-bit signed integers c = round(C * 2^S), S per operator,
-//   * both split at bit 29 (X = h 2^29 + l, c = ch 2^29 + cl, 0 <= l, cl < 2^29), so the
-//     product sum is four 32x32->64 multiply-adds per term, exact in three 64-bit
-//     accumulators:  sum c X = 2^58 sum h ch + 2^29 sum (h cl + l ch) + sum l cl,
-//   * the sum, truncated to a multiple of 2^58 (at most 2^-55 of the largest term), is
-//     rounded once, to nearest-even, into a double.
+//   * both split into signed limbs h 2^29 + l, |l| <= 2^28; the products of two low limbs are left
+//     out, so a term is three 32x32->64 multiply-adds into two 64-bit accumulators,
+//   * the sum, rounded to a multiple of 2^58 in the units of the products, is rounded once, to
+//     nearest-even, into a double.
 // The error stays below one unit in the last place of the line's largest term, as with a
 // chain of FP64 fused multiply-adds, whose rounding errors are of that size too.
 //
-// The stage kernels apply the operators in mirror form (fix_mirror_line): the solution
-// and flux points are symmetric about the cell centre, so the operators satisfy
-// C(NO-1-k, NI-1-j) = sigma C(k, j) (sigma = +1 for the interpolation Lmat, -1 for the
-// derivative Mmat) up to the rounding of their construction (1e-16 to 2e-15 of the
-// largest coefficient for N = 2..8).  With E_j = X_j + X_{NI-1-j} and O_j = X_j - X_{NI-1-j}
-// (exact integers) each pair of mirror outputs k, NO-1-k shares one sum over the NI/2
-// input pairs, U + W and sigma (U - W), so a line takes half the multiply-adds.  The
+// The stage kernels apply the operators in this form through the mirror symmetry
+// (fix_mirror_line, fix_mirror_sums): the solution and flux points are symmetric about the cell
+// centre, so the operators satisfy C(NO-1-k, NI-1-j) = sigma C(k, j) (sigma = +1 for the
+// interpolation Lmat, -1 for the derivative Mmat) up to the rounding of their construction
+// (1e-16 to 2e-15 of the largest coefficient for N = 2..8).  With E_j = X_j + X_{NI-1-j} and
+// O_j = X_j - X_{NI-1-j} (exact integers) each pair of mirror outputs k, NO-1-k shares one sum over
+// the NI/2 input pairs, U + W and sigma (U - W), so a line takes half the multiply-adds.  The
 // coefficients are those of the operator averaged with its mirror image, each within one
 // unit of 2^-S of both rows, and the error bound above holds for that operator.  The
 // caller keeps the FP64 form for lines with NaN, infinite, huge (above 2^876) or tiny (below
 // 2^-957, not zero) inputs, so non-finite states propagate as before.  Zero results are +0;
 // results below the normal range are flushed to zero.
+//
+// fix_dot and what it calls (fix_align, fix_mac, fix_round, fix_split_coef) are the plain form for
+// any operator: 57-bit inputs rounded with kFixG = 4 guard bits, unsigned low limbs, four
+// multiply-adds a term, the sum truncated to a multiple of 2^58.  No kernel calls it, nor
+// fix_apply_mirror, the mirror form for lines of any finite size: they are what the host tests
+// compare with exact sums and hold the mirror form against.
 #pragma once
 #include <cstdint>
 
@@ -41,7 +45,7 @@
 
 namespace chorus {
 
-constexpr int kFixG = 4;       // guard bits of the aligned inputs
+constexpr int kFixG = 4;       // guard bits of the aligned inputs of the plain form (and of the scale k of all forms)
 constexpr int kFixSplit = 29;  // limb split of inputs and coefficients
 constexpr int kFixEmaxFast = 1900;  // largest biased input exponent of the integer form
 

@@ -20,8 +20,9 @@
 // Cell passes stage a block of `epb` cells in shared memory; face passes run one
 // thread per face point.  Values are IEEE doubles throughout; the fixed line operators
 // (Lmat interpolation, Mmat differentiation, which carry no data-dependent
-// coefficients) run as exact integer dot products on the integer pipes (fixdot.cuh), the
-// point fluxes in block fixed point there too (intflux.cuh), all other arithmetic is FP64.
+// coefficients) run as integer dot products on the integer pipes (fixdot.cuh), the
+// point fluxes in integers with an exponent per value there too (intflux.cuh), all other
+// arithmetic is FP64.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -40,10 +41,11 @@ constexpr int kHalfS = kMaxN / 2;      // mirrored pairs of solution points
 // memory; a no-op for a launch without the attribute
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Launch with programmatic stream serialization: the kernel may be scheduled while its
-// predecessor on the stream drains, and waits (griddepcontrol.wait, at its entry) for
-// the predecessor's completion and memory before touching any of its data.  Hides the
-// launch gap between dependent passes; the wait is hardware-managed.
+// Launch with programmatic stream serialization: the kernel waits (griddepcontrol.wait, at its
+// entry) for the predecessor's completion and memory before touching any of its data; the wait
+// is hardware-managed.  No pass releases its dependents before it ends, so what overlaps is the
+// scheduling of the next pass with the flush of the last one's memory after its last CTA has
+// exited: 0.430 -> 0.407 ms a step of 64x64 cells.
 template <typename... KArgs, typename... Args>
 inline void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t st, Args... args) {
   cudaLaunchConfig_t cfg = {};
@@ -338,7 +340,7 @@ __device__ __forceinline__ void e1_body(const SolveDev& s, int e0, int cnt, int 
   // contravariant inviscid flux at the interior flux points only (face points of Fc and
   // Azf belong to the face pass), one point per thread, in the place of the point's state
   // 512x512 cells, N = 5 (GB300): the pass took 1.14 ms a stage with 40 FP64 operations a point
-  // (84% of that pipe), 0.84 ms with some 700 integer instructions (issue slots 61% busy, the
+  // (84% of that pipe), 0.86 ms with integer instructions (issue slots 62% busy, the
   // FP64 pipe 45% with conversions and sensor).  A quarter of the points left in FP64 form beside them:
   // 0.92 ms (part-filled warps in two loops).  64 registers (32 warps per SM): 0.95 ms at 80,
   // 1.06 at 96 without the spill of 28 bytes.
@@ -537,14 +539,15 @@ __device__ __forceinline__ void mark_viscous(const SolveDev& s, int c) {
 // (t < nface2*N) then FREE face points.  Returns the bit pattern of the lane's largest wave
 // speed.
 //
-// A point is one lane's work, some 1900 integer instructions at about 150 registers, so ten
-// warps share an SM: too few to hide the two dependent loads (face record, traces) behind
+// A point is one lane's work, some 2500 instructions at 168 registers, so ten warps share an SM:
+// too few to hide the two dependent loads (face record, traces) behind
 // other warps.  The warp therefore copies the next 32 points' traces and the face records of
 // the 32 after them while it computes a round.  The 72-byte traces and 64-byte flux records
 // are moved by the warp together, consecutive lanes taking consecutive words of a record:
 // one lane per record would touch every 32-byte sector of the L2 four times.
 // 512x512 cells, N = 5 (GB300): 0.867 ms a stage in FP64 (80% of that pipe), 0.62 ms in integer
-// form with one thread's own loads and the averaged traces stored, 0.36 ms in this form, of
+// form with one thread's own loads and the averaged traces stored, 0.42 ms in this form (0.36 with
+// one exponent for several components, which cost small ones their bits), of
 // which the 5.1 kB per cell that it moves take 0.2 ms at the copy rate.  Ten warps at 168
 // registers: at 128 registers (16 warps) the spills go past an L1 that the traces fill, 0.73 ms.
 template <int N, class Map>
@@ -915,9 +918,9 @@ __global__ void __launch_bounds__(512, 2) k_e2(const __grid_constant__ SolveDev 
 // Fc's place or (where the inviscid flux stays downloadable) beside it (interfaceVISflux /
 // BCVISFLUX / CYCLOCVISFLUX, comp_viscous_flux).  One flux point per thread with the integer
 // form of the flux; the FP64 form inside E3 kept that pass at 0.37 ms over its inviscid time
-// (128x128 cells, N = 5, every cell viscous), V takes 0.148 ms.  Bound by latency with the integer
-// issue (49%), the FP64 pipe (54%: averages, conversions) and the loads of Q and grad Q (292 MB,
-// 2.0 TB/s) all about half used: 27 doubles of shared memory a point (the flux in the place of
+// (128x128 cells, N = 5, every cell viscous), V takes 0.153 ms.  Bound by latency with the integer
+// issue (51%), the FP64 pipe (52%: averages, conversions) and the loads of Q and grad Q (292 MB,
+// 1.9 TB/s) all about half used: 27 doubles of shared memory a point (the flux in the place of
 // the state) and 64 registers for eight CTAs per SM, against 0.171 ms with 36 and 72 for six.
 // ---------------------------------------------------------------------------
 // cells per group and threads per CTA: one flux point per thread
@@ -1122,6 +1125,12 @@ constexpr long long kVPassPoints = 49152;
 // small beside a stage; E3 then runs without the registers, the shared memory and the uneven
 // load that the flux needs.  (By the size alone: the two forms round differently, and skipping
 // work that is exactly zero must not change a result.)
+// A step without the pass -> with it (us; GB300), every cell viscous: 8,000 points 207 -> 237 at
+// N = 3, 229 -> 244 at N = 5; 16,000 256 -> 260, 286 -> 276; 32,000 362 -> 329, 376 -> 338; 49,000 516 -> 424,
+// 513 -> 418; 200,000 1641 -> 1400, 1574 -> 1235.  With AV in a few fronts: 16,000 332 -> 339, 383 -> 364; 49,000
+// 513 -> 434, 508 -> 466; 200,000 954 -> 874, 915 -> 848.  Without any active cell its launches
+// cost some 7 us a step.  So the pass pays from some 20,000 points on where it has work, and the
+// line keeps smaller solves, for which the launch counts most, free of it.
 __host__ __device__ inline bool v_pass(const SolveDev& s) { return (long long)s.NC * s.N * s.N >= kVPassPoints; }
 
 // Can a solve have a viscous flux at all?
@@ -1204,7 +1213,7 @@ __device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int 
   // xi sums are not rounded in between.
   // 512x512 cells, N = 5 (GB300), a stage without terms of earlier states: 1.15 ms with the two
   // operations in FP64, the state read from global memory where it is used and predicated FP64
-  // instructions (see PRE), 0.73 ms in this form; 9.2 kB per cell take 0.36 ms at the copy rate.
+  // instructions (see PRE), 0.72 ms in this form; 9.2 kB per cell take 0.36 ms at the copy rate.
   // (the stage update takes the state's place as the residual appears: what else reads the old
   // state does so here)
   if (update && rk.save_old) block_copy_out(rk.save_old + (size_t)e0 * NS * 9, sQ, cnt * NS * 9);
@@ -1370,7 +1379,9 @@ __device__ __forceinline__ void e3_body(const SolveDev& s, int e0, int cnt, int 
   }
 }
 
-// registers per thread of the pass: the line sums spill at 64, more cost resident CTAs
+// registers per thread of the pass: the line sums spill at 64, more cost resident CTAs.  A step of
+// 800,000 points at 72 -> 80 (us; GB300): N = 3 1679 -> 1702, N = 4 1549 -> 1581, N = 5 1666 -> 1575,
+// N = 6 1625 -> 1615, N = 7 1591 -> 1656, N = 8 1513 -> 1548.
 constexpr int e3_regs(int N) { return N == 5 ? 80 : 72; }
 
 template <int N, bool PRE>

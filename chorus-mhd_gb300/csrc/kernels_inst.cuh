@@ -103,7 +103,7 @@ void launch_f1<kN>(const SolveDev& s, cudaStream_t st, int a2, int b2, int a1, i
   if (b2 < 0) b2 = s.nface2;
   if (b1 < 0) b1 = s.nface1;
   const int n2 = (b2 - a2) * kN, n = n2 + (b1 - a1) * kN;
-  // two resident CTAs of 256 threads per SM walk the points; fewer points than that go one
+  // two resident CTAs of kF1Threads per SM walk the points; fewer points than that go one
   // to a thread, in CTAs of 64 so that they spread over every SM
   const int thr = n >= 2 * kF1Threads * sm_count() ? kF1Threads : 64;
   const int grid = std::min((n + thr - 1) / thr, thr == kF1Threads ? 2 * sm_count() : n);
